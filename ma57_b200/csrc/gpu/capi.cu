@@ -252,10 +252,60 @@ void build_maps(const std::vector<int>& cbRows, const std::unordered_map<int, in
   }
 }
 
+// The children (offsets) of a front with a row in each 32-column block, from
+// their extend-add maps; rel(t) is child t's map to the front's rows.
+template <typename Rel>
+void block_children(int m, int nchildren, Rel&& rel, std::vector<int>& ptr, std::vector<int>& child) {
+  const int nb = (m + 31) / 32;
+  std::vector<std::vector<int>> of(nb);
+  for (int t = 0; t < nchildren; ++t)
+    for (const int loc : rel(t))
+      if (of[loc / 32].empty() || of[loc / 32].back() != t) of[loc / 32].push_back(t);
+  ptr.assign(1, 0);
+  child.clear();
+  for (const auto& v : of) {
+    child.insert(child.end(), v.begin(), v.end());
+    ptr.push_back(static_cast<int>(child.size()));
+  }
+}
+
+// Assembly tasks of large front s: 32-column blocks cut into chunks of
+// kAsmRows rows (whole columns of the top fronts left too few CTAs in the
+// last wave), each with its block's children and its own A entries.
+void add_assembly_tasks(const symla_gpu_ctx* c, int s, LevelLists& L) {
+  const auto& f = c->fronts[s];
+  const auto& ptr = f.replanned ? f.dyn_blk_ptr : f.blk_ptr;
+  const auto& child = f.replanned ? f.dyn_blk_child : f.blk_child;
+  auto row_of = [&](int pos) { return pos < f.ncols ? pos : pos + f.nextra; };
+  for (int j0 = 0; j0 < f.m; j0 += 32) {
+    const int b = j0 / 32;
+    AsmTask t{};
+    t.front = s;
+    t.j0 = j0;
+    t.ch0 = static_cast<int>(L.touch.size());
+    t.nch = ptr[b + 1] - ptr[b];
+    L.touch.insert(L.touch.end(), child.begin() + ptr[b], child.begin() + ptr[b + 1]);
+    int e = 0, e1 = 0;
+    if (j0 < f.ncols) {
+      e = c->h_a_colptr[f.firstCol + j0];
+      e1 = c->h_a_colptr[f.firstCol + std::min(j0 + 32, f.ncols)];
+    }
+    for (int i0 = j0; i0 < f.m; i0 += kAsmRows) {
+      t.i0 = i0;
+      t.i1 = std::min(i0 + kAsmRows, f.m);
+      t.a0 = e;
+      while (e < e1 && row_of(c->h_a_pos[e]) < t.i1) ++e;
+      t.a1 = e;
+      L.tasks.push_back(t);
+    }
+  }
+}
+
 void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, LevelLists& L) {
   L.small.clear();
   L.large.clear();
   L.tasks.clear();
+  L.touch.clear();
   L.all = frontsOfLevel;
   L.small_max_m = L.large_max_m = 0;
   L.panels = 0;
@@ -293,12 +343,7 @@ void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, 
         const double mt = f.m - (ps + p);
         L.trailing_flops[it] += static_cast<double>(p) * mt * (mt + 1.0);
       }
-      for (int j0 = 0; j0 < f.m; j0 += 32) {
-        L.tasks.push_back(s);
-        L.tasks.push_back(j0);
-        L.tasks.push_back(j0);
-        L.tasks.push_back(-1);
-      }
+      add_assembly_tasks(c, s, L);
       double cbsum = 0.0;
       for (int ch : f.children) {
         const double cb = c->fronts[ch].m - c->fronts[ch].nelig;
@@ -309,21 +354,6 @@ void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, 
       const int nt = (mt + 127) / 128;
       tiles = std::max(tiles, nt * (nt + 1) / 2);
     }
-  }
-  if (!L.large.empty() && L.tasks.size() / 4 < 4 * 148) {
-    // too few (front, 32 columns) assembly tasks to fill the GPU: split
-    // their rows into chunks
-    std::vector<int> split;
-    for (size_t t = 0; t < L.tasks.size(); t += 4) {
-      const int s = L.tasks[t], j0 = L.tasks[t + 1], m = c->fronts[s].m;
-      for (int i0 = j0; i0 < m; i0 += kAsmRows) {
-        split.push_back(s);
-        split.push_back(j0);
-        split.push_back(i0);
-        split.push_back(i0 + kAsmRows >= m ? -1 : i0 + kAsmRows);
-      }
-    }
-    L.tasks.swap(split);
   }
   if (!L.large.empty()) {
     // one grid over the tiles of every front of the level, in 128 x 128
@@ -347,12 +377,14 @@ void free_level_device(LevelLists& L) {
   dfree(L.d_small);
   dfree(L.d_large);
   dfree(L.d_tasks);
+  dfree(L.d_touch);
   dfree(L.d_all);
   dfree(L.d_fwd_tasks);
   dfree(L.d_bwd_tasks);
   dfree(L.d_tcmaps);
   dfree(L.d_tcws);
-  L.d_small = L.d_large = L.d_tasks = L.d_all = nullptr;
+  L.d_small = L.d_large = L.d_touch = L.d_all = nullptr;
+  L.d_tasks = nullptr;
   L.d_fwd_tasks = L.d_bwd_tasks = nullptr;
   L.d_tcmaps = nullptr;
   L.d_tcws = nullptr;
@@ -447,6 +479,7 @@ void upload_level_lists(LevelLists& L, cudaStream_t s) {
   if (!L.large.empty() && !panel_fits_shared(L.large_max_m))
     L.d_panel_cols = dalloc<double>(2 * static_cast<size_t>(L.large_max_m) * L.large.size());
   L.d_tasks = dupload(L.tasks, s);
+  L.d_touch = dupload(L.touch, s);
   L.d_all = dupload(L.all, s);
 }
 
@@ -547,6 +580,15 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
       mapPool.insert(mapPool.end(), rel.begin(), rel.end());
       ltmp.push_back(lt);
     }
+    if (f.m > kSmallFrontMax)
+      block_children(
+          f.m, static_cast<int>(f.children.size()),
+          [&](int t) {
+            const LinkTmp& lt = ltmp[c->link_begin_static[s] + t];
+            rel.assign(mapPool.begin() + lt.rel, mapPool.begin() + lt.rel + lt.cb);
+            return rel;
+          },
+          c->fronts[s].blk_ptr, c->fronts[s].blk_child);
     c->link_end_static[s] = static_cast<int>(ltmp.size());
   }
   c->d_maps = dupload(mapPool, c->stream);
@@ -583,9 +625,13 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
       ents.push_back(AEnt{lo, static_cast<int>(it - rp.begin()), lo - c->fronts[s].firstCol, p});
     }
   }
+  // by front and 32-column block, then row: the range of a block's columns
+  // (or of the whole front) stays contiguous and the entries of a row of a
+  // block are consecutive (the assembly's order)
   std::sort(ents.begin(), ents.end(), [](const AEnt& a, const AEnt& b) {
-    if (a.col != b.col) return a.col < b.col;
-    return a.pos < b.pos;
+    const int ka = a.col - a.j % 32, kb = b.col - b.j % 32;
+    if (ka != kb) return ka < kb;
+    return a.pos != b.pos ? a.pos < b.pos : a.col < b.col;
   });
   std::vector<int> acolptr(n + 1, 0), aj(ents.size()), apos(ents.size()), aidx(ents.size());
   for (const auto& e : ents) acolptr[e.col + 1]++;
@@ -595,6 +641,8 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
     apos[t] = ents[t].pos;
     aidx[t] = ents[t].idx;
   }
+  c->h_a_colptr = acolptr;
+  c->h_a_pos = apos;
   c->d_a_colptr = dupload(acolptr, c->stream);
   c->d_a_j = dupload(aj, c->stream);
   c->d_a_pos = dupload(apos, c->stream);
@@ -874,7 +922,7 @@ void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, co
 // The level's kernels with `iters` panel iterations, no host synchronisation
 // (the part a graph launch captures).
 void launch_level_planned(symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko, int dynamic,
-                          const int* d_small, const int* d_large, const int* d_tasks, int iters) {
+                          const int* d_small, const int* d_large, int iters) {
   cudaStream_t st = c->stream;
   c->cur_level = level;
   if (!L.small.empty())
@@ -884,8 +932,8 @@ void launch_level_planned(symla_gpu_ctx* c, const LevelLists& L, int level, cons
     });
   if (!L.large.empty()) {
     timed(c, SYMLA_KERNEL_ASSEMBLE, 0.0, L.assemble_bytes, [&] {
-      launch_assemble(c->d_desc, c->d_links, c->d_state, d_tasks, static_cast<int>(L.tasks.size() / 4),
-                      c->d_a_colptr, ko, c->d_glob, level, dynamic, st);
+      launch_assemble(c->d_desc, c->d_links, c->d_state, L.d_tasks, static_cast<int>(L.tasks.size()), L.d_touch, ko,
+                      c->d_glob, level, dynamic, st);
     });
     for (int it = 0; it < iters; ++it) launch_panel_iteration(c, L, level, ko, dynamic, d_large);
   }
@@ -903,14 +951,14 @@ int level_plan_iters(const symla_gpu_ctx* c, const LevelLists& L, int level) {
 }
 
 void launch_level(symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko, int dynamic,
-                  const int* d_small, const int* d_large, const int* d_tasks) {
+                  const int* d_small, const int* d_large) {
   const int iters = level_plan_iters(c, L, level);
   FactorGlobals before{};
   if (c->profiling && !L.large.empty()) {
     CK(cudaMemcpyAsync(&before, c->d_glob, sizeof before, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
   }
-  launch_level_planned(c, L, level, ko, dynamic, d_small, d_large, d_tasks, iters);
+  launch_level_planned(c, L, level, ko, dynamic, d_small, d_large, iters);
   if (!L.large.empty()) complete_level(c, L, level, ko, dynamic, d_large, iters);
   if (c->profiling && !L.large.empty()) {
     FactorGlobals after{};
@@ -981,7 +1029,7 @@ void run_static_pass_graph(symla_gpu_ctx* c, const KernelOpts& ko) {
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     for (int l = 0; l < c->numLevels; ++l) {
       const LevelLists& L = c->levels[l];
-      launch_level_planned(c, L, l, ko, 0, L.d_small, L.d_large, L.d_tasks, iters[l]);
+      launch_level_planned(c, L, l, ko, 0, L.d_small, L.d_large, iters[l]);
       if (!L.large.empty())
         launch_mark_unfinished(c->d_state, L.d_large, static_cast<int>(L.large.size()), c->d_glob, l, st);
     }
@@ -1086,6 +1134,14 @@ void replan_front(symla_gpu_ctx* c, int s) {
     pool.insert(pool.end(), inv.begin(), inv.end());
     pool.insert(pool.end(), rel.begin(), rel.end());
   }
+  if (f.m > kSmallFrontMax)
+    block_children(
+        f.m, static_cast<int>(f.children.size()),
+        [&](int t) {
+          rel.assign(pool.begin() + offs[t].second, pool.begin() + offs[t].second + cbRowsOf[t].size());
+          return rel;
+        },
+        f.dyn_blk_ptr, f.dyn_blk_child);
   int* dmaps = dupload(pool, c->stream);
   c->dyn_allocs.push_back(dmaps);
   const int begin = static_cast<int>(c->hlinks.size());
@@ -1151,13 +1207,13 @@ void run_factorization(symla_gpu_ctx* c, const symla_factor_opts* o, symla_facto
       complete_level(c, c->levels[u], u, ko, 0, c->levels[u].d_large, c->graph_level_iters[u]);
       for (int l = u + 1; l < c->numLevels; ++l) {
         const LevelLists& L = c->levels[l];
-        launch_level(c, L, l, ko, 0, L.d_small, L.d_large, L.d_tasks);
+        launch_level(c, L, l, ko, 0, L.d_small, L.d_large);
       }
     }
   } else {
     for (int l = 0; l < c->numLevels; ++l) {
       const LevelLists& L = c->levels[l];
-      launch_level(c, L, l, ko, 0, L.d_small, L.d_large, L.d_tasks);
+      launch_level(c, L, l, ko, 0, L.d_small, L.d_large);
     }
   }
   FactorGlobals g;
@@ -1190,7 +1246,7 @@ void run_factorization(symla_gpu_ctx* c, const symla_factor_opts* o, symla_facto
         }
       }
       validate_tables(c, 0, ko, "after re-planning delayed pivots");
-      launch_level(c, L, l, ko, 1, L.d_small, L.d_large, L.d_tasks);
+      launch_level(c, L, l, ko, 1, L.d_small, L.d_large);
       read_states(c);
       free_level_device(L);
     }

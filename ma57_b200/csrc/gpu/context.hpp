@@ -9,6 +9,7 @@
 
 #include "../host/symbolic.hpp"
 #include "common.cuh"
+#include "factor_kernels.h"
 
 struct symla_symbolic {
   symla_host::SymbolicFactor sf;
@@ -24,6 +25,10 @@ struct HostFront {
   std::vector<int> children;
   const std::vector<int>* rowPattern = nullptr;
   bool replanned = false;
+  // large fronts: the children with a row in each 32-column block, as offsets
+  // into `children` (blk_child[blk_ptr[b] .. blk_ptr[b + 1])), for the
+  // symbolic structure and, after re-planning, for the current one
+  std::vector<int> blk_ptr, blk_child, dyn_blk_ptr, dyn_blk_child;
 };
 
 struct LevelLists {
@@ -38,7 +43,8 @@ struct LevelLists {
   int panel_width = 32;        // pivots per panel (narrower for fronts too tall for a full-width cluster panel)
   double* d_panel_cols = nullptr;  // single-CTA panel kernel, fronts too tall for shared memory: 2 m per front
   int trailing_grid = 0;
-  std::vector<int> tasks;      // assembly tasks (front, column block) for large fronts
+  std::vector<AsmTask> tasks;  // assembly tasks of the large fronts
+  std::vector<int> touch;      // and their children (AsmTask::ch0)
   std::vector<int> all;        // every front of the level (solve)
   // algorithmic work estimates (instrumentation)
   double small_flops = 0.0;
@@ -53,7 +59,8 @@ struct LevelLists {
   // device copies (static plan)
   int* d_small = nullptr;
   int* d_large = nullptr;
-  int* d_tasks = nullptr;
+  AsmTask* d_tasks = nullptr;
+  int* d_touch = nullptr;
   int* d_all = nullptr;
   // mixed-precision far update: per large front (list order) its TF32
   // workspace and the tensor map over it (built on first use)
@@ -111,6 +118,7 @@ struct symla_gpu_ctx {
   symla_gpu::FrontState* d_state = nullptr;
   symla_gpu::FactorGlobals* d_glob = nullptr;
   int* d_a_colptr = nullptr;
+  std::vector<int> h_a_colptr, h_a_pos;  // host copies: the assembly tasks' A entries
   int* d_a_j = nullptr;
   int* d_a_pos = nullptr;
   int* d_a_idx = nullptr;

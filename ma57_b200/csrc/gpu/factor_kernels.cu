@@ -67,40 +67,77 @@ __device__ __forceinline__ bool a_entry(const KernelOpts& o, const FrontDesc& f,
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Assembly of large fronts in global memory: one CTA per (front, 32-column
-// block, row range); levels with few large fronts split the rows into
-// chunks so that they still fill the GPU. Every parent entry is written exactly once (gather
-// form), so no separate zero fill and no atomics; then the A entries of the
-// block's own columns and rows are added. The children's map pointers, contribution-block
-// origins and their maps of the block's 32 columns are staged in shared
-// memory once; each thread then takes rows, reads a row's position in each
-// child once and issues the (independent) loads of 16 of the 32 columns,
-// summing over the children in their fixed order.
+// Assembly of large fronts in global memory: one CTA per task, a 32-column
+// block of a front over at most kAsmRows rows. Every parent entry is written
+// once per batch of children (gather form; no zero fill, no atomics), with the
+// block's A entries added and its max |entry| taken (dense_kernel.hpp:413) on
+// the way.
+//
+// A task carries the list of the children that have a row among its 32
+// columns, made on the host with the plan, and visits those alone, 16 at a
+// time (their maps of the block's columns and their column origins staged in
+// shared memory). A front near the root of a KKT tree has thousands of
+// children of which a block meets about twenty: looking up every child's map
+// for every entry took 315 ms on a front of 15568 rows with 2533 children,
+// visiting the block's own takes 1.2 ms
+// (of 335 and 4.8 ms for all levels of that KKT system).
+// What bounds it is the latency of the chain map -> contribution block ->
+// store, so a thread has the 16 loads of its half row in flight per child,
+// the first children's maps of its next row are loaded one row ahead, and the
+// A entries (sorted by row within a block, so that a task's are one range and
+// a row's are consecutive) go through registers instead of a second pass over
+// the block: the pass that added them to the front and the pass that read it
+// again for the maximum took the rest of a 64^3 stencil's 7.0 ms, now 4.2 ms
+// (2.4 TB/s of the entries read and written, of 6.5 TB/s for a plain copy).
 namespace {
-constexpr int kAsmMaxChildren = 16;
+constexpr int kAsmBatch = 16;   // children staged at a time
+constexpr int kAsmAhead = 2;    // children whose row maps are loaded one row ahead
 }
 
 __global__ void __launch_bounds__(256, 4) assemble_kernel(const FrontDesc* __restrict__ fronts,
                                                        const ChildLink* __restrict__ links,
-                                                       FrontState* st, const int* __restrict__ tasks,
-                                                       const int* __restrict__ a_colptr, KernelOpts o,
+                                                       FrontState* st, const AsmTask* __restrict__ tasks,
+                                                       const int* __restrict__ touch, KernelOpts o,
                                                        const FactorGlobals* __restrict__ g, int level, int dynamic) {
   if (level_aborted(g, level, dynamic)) return;
-  __shared__ const int* s_inv[kAsmMaxChildren];
-  __shared__ const double* s_cb[kAsmMaxChildren];
-  __shared__ int64_t s_ld[kAsmMaxChildren];
-  __shared__ int s_b[kAsmMaxChildren][32];
-  __shared__ int s_lim[kAsmMaxChildren];  // checked build: contribution-block rows of each child
-  const int4 task = reinterpret_cast<const int4*>(tasks)[blockIdx.x];
-  const int s = task.x, j0 = task.y, i0 = task.z;  // i0 >= j0
+  __shared__ const int* s_inv[kAsmBatch];
+  __shared__ const double* s_cb[kAsmBatch];
+  __shared__ int64_t s_ld[kAsmBatch];
+  __shared__ int s_b[kAsmBatch][32];
+  __shared__ unsigned s_mask[kAsmBatch];  // the block's columns the child has
+  __shared__ int s_lim[kAsmBatch];        // checked build: contribution-block rows of each child
+  __shared__ int s_e0[kAsmRows], s_e1[kAsmRows];  // the A entries of each row of the task
+  const AsmTask task = tasks[blockIdx.x];
+  const int s = task.front, j0 = task.j0, i0 = task.i0;  // i0 >= j0
   const FrontDesc f = fronts[s];
   const int j1 = min(j0 + 32, f.m), nj = j1 - j0;
-  const int iend = task.w < 0 ? f.m : min(task.w, f.m);
-  const int nch = f.ch_end - f.ch_begin;
+  const int iend = min(task.i1, f.m);
   if (i0 == j0 && threadIdx.x < nj) f.lperm[j0 + threadIdx.x] = j0 + threadIdx.x;
-  if (nch <= kAsmMaxChildren) {
+  for (int t = threadIdx.x; t < kAsmRows; t += 256) s_e0[t] = s_e1[t] = 0;
+  if (task.a0 < task.a1) {
+    __syncthreads();
+    for (int e = task.a0 + threadIdx.x; e < task.a1; e += 256) {
+      int j, i, idx;
+      if (!a_entry(o, f, e, j, i, idx)) continue;
+      if (!check(i >= i0 && i < iend, o.chk, kChkAEntry, e)) continue;
+      const int pos = o.a_pos[e];
+      if (e == task.a0 || o.a_pos[e - 1] != pos) s_e0[i - i0] = e;
+      if (e + 1 == task.a1 || o.a_pos[e + 1] != pos) s_e1[i - i0] = e + 1;
+    }
+  }
+  // warp w takes columns j0 + 16 (w & 1) .. + 16 of rows 32 (w >> 1) + lane
+  // + 128 t: half a row's loads per thread keeps the registers low enough
+  // for four CTAs per SM
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h0 = 16 * (warp & 1);
+  const int ifirst = i0 + 32 * (warp >> 1) + lane;
+  double tmax = 0.0;
+  for (int c0 = 0; c0 == 0 || c0 < task.nch; c0 += kAsmBatch) {
+    const int nch = min(kAsmBatch, task.nch - c0);
+    const bool last = c0 + kAsmBatch >= task.nch;
+    __syncthreads();  // (also: the row ranges of the A entries are set)
     if (threadIdx.x < nch) {
-      const ChildLink L = links[f.ch_begin + threadIdx.x];
+      const ChildLink L = links[f.ch_begin + touch[task.ch0 + c0 + threadIdx.x]];
       const FrontDesc& cf = fronts[L.child];
       const int np = st[L.child].npiv;
       s_inv[threadIdx.x] = L.invmap;
@@ -110,23 +147,31 @@ __global__ void __launch_bounds__(256, 4) assemble_kernel(const FrontDesc* __res
         s_lim[threadIdx.x] = check(np >= 0 && np <= cf.m, o.chk, kChkPivots, L.child) ? cf.m - np : 0;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < nch * 32; t += blockDim.x) {
-      const int c = t / 32, jj = t % 32;
-      s_b[c][jj] = (jj < nj) ? s_inv[c][j0 + jj] : -1;
+    for (int t = threadIdx.x; t < nch * 32; t += 256) {
+      const int c = t >> 5, jj = t & 31;
+      const int b = (jj < nj) ? s_inv[c][j0 + jj] : -1;
+      s_b[c][jj] = b;
+      const unsigned mask = __ballot_sync(0xffffffffu, b >= 0);
+      if (jj == 0) s_mask[c] = mask;
     }
     __syncthreads();
-    // warp w takes columns j0 + 16 (w & 1) .. + 16 of rows 32 (w >> 1) + lane
-    // + 128 t: half a row's loads per thread keeps the registers low enough
-    // for four CTAs per SM (the gather is load-latency-bound)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = 16 * (warp & 1);
-    for (int i = i0 + 32 * (warp >> 1) + lane; i < iend; i += 128) {
-      double acc[16];
+    int ahead[kAsmAhead];
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) acc[jj] = 0.0;
-      for (int c = 0; c < nch; ++c) {
-        const int a = s_inv[c][i];
-        if (a < 0) continue;
+    for (int c = 0; c < kAsmAhead; ++c) ahead[c] = (c < nch && ifirst < iend) ? s_inv[c][ifirst] : -1;
+    for (int i = ifirst; i < iend; i += 128) {
+      double acc[16];
+      double* out = f.F + static_cast<int64_t>(j0 + h0) * f.ld + i;
+#pragma unroll
+      for (int jj = 0; jj < 16; ++jj)
+        acc[jj] = (c0 > 0 && h0 + jj < nj && j0 + h0 + jj <= i) ? out[static_cast<int64_t>(jj) * f.ld] : 0.0;
+      int row[kAsmAhead];
+#pragma unroll
+      for (int c = 0; c < kAsmAhead; ++c) {
+        row[c] = ahead[c];
+        ahead[c] = (c < nch && i + 128 < iend) ? s_inv[c][i + 128] : -1;
+      }
+      auto add_child = [&](int c, int a) {
+        if (a < 0) return;
         const double* cb = s_cb[c];
         const int64_t cld = s_ld[c];
 #pragma unroll
@@ -137,48 +182,31 @@ __global__ void __launch_bounds__(256, 4) assemble_kernel(const FrontDesc* __res
             if (check(r < s_lim[c], o.chk, kChkGather, s)) acc[jj] += cb[static_cast<int64_t>(cc) * cld + r];
           }
         }
+      };
+#pragma unroll
+      for (int c = 0; c < kAsmAhead; ++c)
+        if (c < nch) add_child(c, row[c]);
+      for (int c = kAsmAhead; c < nch; ++c)
+        if ((s_mask[c] >> h0) & 0xffffu) add_child(c, s_inv[c][i]);
+      if (last) {
+        for (int e = s_e0[i - i0]; e < s_e1[i - i0]; ++e) {
+          const int j = o.a_j[e] - j0 - h0;
+          const double v = o.values[o.a_idx[e]];
+#pragma unroll
+          for (int jj = 0; jj < 16; ++jj)
+            if (jj == j) acc[jj] += v;
+        }
       }
 #pragma unroll
       for (int jj = 0; jj < 16; ++jj)
-        if (h0 + jj < nj && j0 + h0 + jj <= i) f.F[static_cast<int64_t>(j0 + h0 + jj) * f.ld + i] = acc[jj];
+        if (h0 + jj < nj && j0 + h0 + jj <= i) {
+          out[static_cast<int64_t>(jj) * f.ld] = acc[jj];
+          if (last) tmax = fmax(tmax, fabs(acc[jj]));
+        }
     }
-  } else {
-    for (int j = j0; j < j1; ++j) {
-      double* col = f.F + static_cast<int64_t>(j) * f.ld;
-      for (int i = max(j, i0) + threadIdx.x; i < iend; i += blockDim.x)
-        col[i] = gather_children(fronts, links, st, f.ch_begin, f.ch_end, i, j, o.chk);
-    }
-  }
-  __syncthreads();
-  if (j0 < f.ncols) {
-    const int jend = min(j1, f.ncols);
-    const int e0 = a_colptr[f.a_begin + j0], e1 = a_colptr[f.a_begin + jend];
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      int j, i, idx;
-      if (a_entry(o, f, e, j, i, idx) && i >= i0 && i < iend) f.F[static_cast<int64_t>(j) * f.ld + i] += o.values[idx];
-    }
-  }
-  // max |entry| of the assembled front (dense_kernel.hpp:413), folded here
-  // so the panel kernel does not rescan the front: a thread takes a row and
-  // reads its (up to) 32 entries of the task's columns with independent
-  // loads (consecutive rows across a warp), then the next row
-  __syncthreads();
-  double tmax = 0.0;
-  const double* blk = f.F + static_cast<int64_t>(j0) * f.ld;
-  for (int i = i0 + threadIdx.x; i < iend; i += blockDim.x) {
-    double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
-#pragma unroll
-    for (int jj = 0; jj < 32; jj += 4) {
-      const double* p = blk + static_cast<int64_t>(jj) * f.ld + i;
-      if (jj + 0 < nj && j0 + jj + 0 <= i) t0 = fmax(t0, fabs(p[0]));
-      if (jj + 1 < nj && j0 + jj + 1 <= i) t1 = fmax(t1, fabs(p[f.ld]));
-      if (jj + 2 < nj && j0 + jj + 2 <= i) t2 = fmax(t2, fabs(p[2 * static_cast<int64_t>(f.ld)]));
-      if (jj + 3 < nj && j0 + jj + 3 <= i) t3 = fmax(t3, fabs(p[3 * static_cast<int64_t>(f.ld)]));
-    }
-    tmax = fmax(tmax, fmax(fmax(t0, t1), fmax(t2, t3)));
   }
   tmax = warp_max(tmax);
-  if ((threadIdx.x & 31) == 0) atomic_max_nonneg(&st[s].orig_max, tmax);
+  if (lane == 0) atomic_max_nonneg(&st[s].orig_max, tmax);
 }
 
 // ---------------------------------------------------------------------------
@@ -1324,11 +1352,11 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
 // ---------------------------------------------------------------------------
 // Host launchers
 
-void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* tasks,
-                     int ntasks, const int* a_colptr, const KernelOpts& o, const FactorGlobals* g, int level,
-                     int dynamic, cudaStream_t stream) {
+void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const AsmTask* tasks,
+                     int ntasks, const int* touch, const KernelOpts& o, const FactorGlobals* g, int level, int dynamic,
+                     cudaStream_t stream) {
   if (ntasks <= 0) return;
-  assemble_kernel<<<ntasks, 256, 0, stream>>>(fronts, links, st, tasks, a_colptr, o, g, level, dynamic);
+  assemble_kernel<<<ntasks, 256, 0, stream>>>(fronts, links, st, tasks, touch, o, g, level, dynamic);
 }
 
 size_t small_front_smem(int m) {

@@ -12,17 +12,24 @@ namespace symla_gpu {
 constexpr int kSmallFrontMax = 128;
 // Panel width of the large-front path.
 constexpr int kPanelWidth = 32;
-// Rows of one assembly task when a level's (front, 32 columns) tasks are
-// too few to fill the GPU (they are then split into row chunks).
-constexpr int kAsmRows = 1024;
+// Most rows of one assembly task.
+constexpr int kAsmRows = 512;
+
+// An assembly task: columns [j0, j0 + 32) of a front over its rows [i0, i1)
+// (i0 >= j0), the nch children with a row among those columns (child offsets
+// within the front, in order, touch[ch0 ..]) and the A entries [a0, a1) of
+// those columns and rows.
+struct AsmTask {
+  int front, j0, i0, i1;
+  int ch0, nch, a0, a1;
+};
 
 cudaError_t configure_factor_kernels();
 size_t small_front_smem(int m);
 
-// tasks: (front, first column, first row, end row or -1 for the front's m)
-void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* tasks,
-                     int ntasks, const int* a_colptr, const KernelOpts& o, const FactorGlobals* g, int level,
-                     int dynamic, cudaStream_t stream);
+void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const AsmTask* tasks,
+                     int ntasks, const int* touch, const KernelOpts& o, const FactorGlobals* g, int level, int dynamic,
+                     cudaStream_t stream);
 void launch_factor_small(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* list, int count,
                          int max_m, const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
                          cudaStream_t stream, int threads = 0);  // threads: 32 (a warp per front, fronts of
