@@ -472,6 +472,28 @@ void ensure_tc_static(symla_gpu_ctx* c) {
   c->tc_static_ready = true;
 }
 
+// Packed operands of the FP64 Schur updates: per large front, L and -(L D) of
+// an outer block (packed_at). Levels run one after another and share one
+// buffer.
+size_t packed_doubles(const FrontDesc& d) {
+  return 2 * static_cast<size_t>(packed_chunks(d.nelig)) * ((d.m + 63) / 64) * kPkTile;
+}
+size_t packed_level_doubles(const symla_gpu_ctx* c, const LevelLists& L) {
+  size_t t = 0;
+  for (int s : L.large) t += packed_doubles(c->hdesc[s]);
+  return t;
+}
+void assign_packed_level(symla_gpu_ctx* c, const LevelLists& L, double* base) {
+  for (int s : L.large) {
+    FrontDesc& d = c->hdesc[s];
+    const size_t len = packed_doubles(d);
+    d.P = base;
+    d.pw = static_cast<int64_t>(len / 2);
+    d.prt = (d.m + 63) / 64;
+    base += len;
+  }
+}
+
 void upload_level_lists(LevelLists& L, cudaStream_t s) {
   free_level_device(L);
   L.d_small = dupload(L.small, s);
@@ -673,9 +695,10 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
     d.a_end = f.firstCol + f.ncols;
     d.level = f.level;
     d.wld = f.m;
+    d.P = nullptr;
+    d.pw = 0;
+    d.prt = 0;
   }
-  c->hdesc_static = c->hdesc;
-  c->d_desc = dupload(c->hdesc, c->stream);
   c->d_state = dalloc<FrontState>(numSN);
   c->d_glob = dalloc<FactorGlobals>(1);
 
@@ -688,7 +711,12 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   for (int l = 0; l < numLevels; ++l) {
     build_level_lists(c, byLevel[l], c->levels[l]);
     upload_level_lists(c->levels[l], c->stream);
+    c->packed_doubles = std::max(c->packed_doubles, packed_level_doubles(c, c->levels[l]));
   }
+  c->d_packed = dalloc<double>(c->packed_doubles);
+  for (const auto& L : c->levels) assign_packed_level(c, L, c->d_packed);
+  c->hdesc_static = c->hdesc;
+  c->d_desc = dupload(c->hdesc, c->stream);
 
   // residual: full symmetric CSR gathered from the stored lower triangle,
   // columns sorted per row; and the stored-entry rows for ||A||
@@ -1235,6 +1263,16 @@ void run_factorization(symla_gpu_ctx* c, const symla_factor_opts* o, symla_facto
       LevelLists L;
       build_level_lists(c, Ls.all, L);
       upload_level_lists(L, st);
+      if (!L.large.empty()) {
+        const size_t need = packed_level_doubles(c, L);
+        double* pk = c->d_packed;
+        if (need > c->packed_doubles) {
+          pk = dalloc<double>(need);
+          c->dyn_allocs.push_back(pk);
+        }
+        assign_packed_level(c, L, pk);
+        CK(cudaMemcpyAsync(c->d_desc, c->hdesc.data(), c->hdesc.size() * sizeof(FrontDesc), cudaMemcpyHostToDevice, st));
+      }
       if (mixed && !L.large.empty()) {
         float* ws = dalloc<float>(tc_level_floats(c, L));
         c->dyn_allocs.push_back(ws);
@@ -1651,7 +1689,7 @@ extern "C" void symla_gpu_destroy(symla_gpu_ctx* c) {
                   c->d_Bp, c->d_Z, c->d_Xf, c->d_B, c->d_X, c->d_R, c->d_dX, c->d_Xn, c->d_Rn, c->d_norms,
                   c->d_scratch_int, c->d_flag_base, c->d_flags, c->d_solve_err, c->d_counter,
                   c->d_tcws, c->d_tc_err, c->d_tc_guard, c->d_hflags, c->d_hscratch,
-                  c->d_gmres, c->d_zero, c->d_gpart, c->d_gcoef, c->d_check, c->d_ranges};
+                  c->d_gmres, c->d_zero, c->d_gpart, c->d_gcoef, c->d_check, c->d_ranges, c->d_packed};
   for (void* p : ptrs) dfree(p);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);

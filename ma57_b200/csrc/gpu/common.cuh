@@ -27,7 +27,24 @@ struct FrontDesc {
   int a_begin, a_end;    // original-A entries of the own columns
   int level;
   int wld;            // leading dimension of W (>= m)
+  // large fronts: the current outer block's pivot columns packed for the
+  // Schur updates (see packed_at): L at P, -(L D) at P + pw
+  double* P;
+  int64_t pw;
+  int prt;            // 64-row tiles of the front
 };
+
+// Packed operands of the Schur updates. Pivot q (counted from the outer
+// block's first) of row i sits in the 16-pivot x 64-row tile (q / 16, i / 64),
+// pivot-major with a stride of kPkRow doubles (conflict-free fragment loads),
+// a tile being kPkTile consecutive doubles and the row tiles of a pivot chunk
+// following one another: what an update tile needs of a chunk is one
+// contiguous range per operand.
+constexpr int kPkRow = 68;
+constexpr int kPkTile = 16 * kPkRow;
+__host__ __device__ inline int64_t packed_at(int prt, int q, int i) {
+  return (static_cast<int64_t>(q >> 4) * prt + (i >> 6)) * kPkTile + (q & 15) * kPkRow + (i & 63);
+}
 
 // Child -> parent extend-add maps.
 struct ChildLink {
@@ -59,6 +76,11 @@ enum : int { kFlagDone = 1, kFlagDelayed = 2, kFlagSingularRoot = 4, kFlagFlush 
 
 // Columns per outer block of the large-front factorization.
 constexpr int kOuterBlock = 256;
+// 16-pivot chunks of packed operands a front needs: an outer block, plus one
+// pivot when a 2x2 straddles its end, of the eligible columns.
+__host__ __device__ inline int packed_chunks(int nelig) {
+  return ((nelig < kOuterBlock + 1 ? nelig : kOuterBlock + 1) + 15) / 16;
+}
 // Pivots per far update the tensor-core workspace holds (>= kOuterBlock + 1,
 // a multiple of 32).
 constexpr int kTcKpad = 288;

@@ -102,6 +102,8 @@ struct symla_gpu_ctx {
   // device: static plan
   double* d_arena = nullptr;
   size_t arena_doubles = 0;
+  double* d_packed = nullptr;  // packed operands of the Schur updates (the largest level's)
+  size_t packed_doubles = 0;
   int* d_fidx = nullptr;       // per-front row index pool (static layout)
   int* d_lperm = nullptr;      // per-front local pivot permutation pool
   int* d_lpos = nullptr;       // and its inverse

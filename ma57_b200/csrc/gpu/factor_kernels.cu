@@ -635,8 +635,18 @@ __device__ void panel_current_column(const FrontDesc& f, int ps, int p, int k, i
 }
 
 // Symmetric swap of positions i < j in lower storage over the whole front
-// (global memory).
-__device__ void global_swap(const FrontDesc& f, int i, int j) {
+// (global memory), and of their rows in the packed pivots [ob, k).
+__device__ void global_swap(const FrontDesc& f, int i, int j, int ob, int k) {
+  for (int t = threadIdx.x; t < k - ob; t += blockDim.x) {
+    double* a = f.P + packed_at(f.prt, t, i);
+    double* b = f.P + packed_at(f.prt, t, j);
+    double x = a[0];
+    a[0] = b[0];
+    b[0] = x;
+    x = a[f.pw];
+    a[f.pw] = b[f.pw];
+    b[f.pw] = x;
+  }
   const int m = f.m;
   double* F = f.F;
   const int64_t ld = f.ld;
@@ -730,6 +740,13 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
   const int ps = k;
   const int pe = ps + min(nb, S.ob_end - ps);
   double thread_rmax = 0.0;
+  // L and -(L D) of pivot kk, row i, to the front and the packed operands
+  auto put = [&](int kk, int i, double l, double a) {
+    f.F[static_cast<int64_t>(kk) * f.ld + i] = l;
+    double* pk = f.P + packed_at(f.prt, kk - S.ob, i);
+    pk[0] = l;
+    pk[f.pw] = -a;
+  };
   bool stopped = false;
   bool flush = false;
   int n_pos = S.n_pos, n_neg = S.n_neg, n_zero = S.n_zero, nPert = S.num_perturbed;
@@ -769,7 +786,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
       for (int i = k + 1 + threadIdx.x; i < m; i += NT) {
         const double a = colk[i];
         thread_rmax = fmax(thread_rmax, fabs(a));
-        f.F[static_cast<int64_t>(k) * f.ld + i] = a / d;
+        put(k, i, a / d, a);
       }
       if (threadIdx.x == 0) {
         f.F[static_cast<int64_t>(k) * f.ld + k] = d;
@@ -820,7 +837,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
     if (dec == 0 || dec == 1) {
       double* col = colk;
       if (dec == 1) {
-        global_swap(f, k, r);
+        global_swap(f, k, r, S.ob, k);
         // new column k = old column r with rows k and r exchanged
         if (threadIdx.x == 0) {
           const double a = colr[k];
@@ -841,7 +858,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
       for (int i = k + 1 + threadIdx.x; i < m; i += NT) {
         const double a = col[i];
         thread_rmax = fmax(thread_rmax, fabs(a));
-        f.F[static_cast<int64_t>(k) * f.ld + i] = a / d;
+        put(k, i, a / d, a);
       }
       if (threadIdx.x == 0) {
         f.F[static_cast<int64_t>(k) * f.ld + k] = d;
@@ -855,7 +872,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
     }
     // 2x2: bring r to k+1
     if (r != k + 1) {
-      global_swap(f, k + 1, r);
+      global_swap(f, k + 1, r, S.ob, k);
       if (threadIdx.x == 0) {
         double a = colk[k + 1];
         colk[k + 1] = colk[r];
@@ -893,8 +910,8 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
     for (int i = k + 2 + threadIdx.x; i < m; i += NT) {
       const double a0 = colk[i], a1 = colr[i];
       thread_rmax = fmax(thread_rmax, fmax(fabs(a0), fabs(a1)));
-      f.F[static_cast<int64_t>(k) * f.ld + i] = a0 * inv11 + a1 * inv21;
-      f.F[static_cast<int64_t>(k + 1) * f.ld + i] = a0 * inv21 + a1 * inv22;
+      put(k, i, a0 * inv11 + a1 * inv21, a0);
+      put(k + 1, i, a0 * inv21 + a1 * inv22, a1);
     }
     if (threadIdx.x == 0) {
       f.F[static_cast<int64_t>(k) * f.ld + k] = d11;
@@ -978,11 +995,12 @@ __device__ __forceinline__ bool update_range(const FrontState& S, int m, bool fa
   return q1 > q0 && c1 > c0;
 }
 
-// Tiles of front s's update region: column tiles of width tj over [c0, c1),
-// each with tm-row tiles from its diagonal down to m.
-__device__ __forceinline__ int update_tiles(int m, int c0, int c1, int tj, int tm) {
+// Column tiles of an update region sit on the 64-row grid of the packed
+// operands: tile t covers columns [64 t, 64 t + 64) of [c0, c1) and its row
+// tiles of tm rows start at row 64 t.
+__device__ __forceinline__ int update_tiles(int m, int c0, int c1, int tm) {
   int n = 0;
-  for (int j = c0; j < c1; j += tj) n += (m - j + tm - 1) / tm;
+  for (int j = c0 & ~63; j < c1; j += 64) n += (m - j + tm - 1) / tm;
   return n;
 }
 
@@ -991,32 +1009,33 @@ __device__ __forceinline__ int update_tiles(int m, int c0, int c1, int tj, int t
 // (DMMA; the 5th-gen tcgen05 MMA has no FP64 kind). TM x 64 tiles: TM = 128,
 // 8 warps of 32 x 32 (2 x 4 MMA tiles, 4 accumulators each per lane), or
 // TM = 64 for small fronts, 8 warps of 32 x 16 (the autotuner picks per
-// level); two CTAs per SM, so that one CTA's C load and store overlap the
-// other's MMAs.
+// level); two CTAs per SM.
 //
-// A chunk of 16 pivots of the A rows (L(i, q)) and of the B rows (L(j, q),
-// with the 2 x 2 partner columns either side) is staged pivot-major, as the
-// front stores it, by bulk copies (cp.async.bulk, one per pivot column, no
-// multicast) that one thread issues and an mbarrier per stage counts, in a
-// ring of three stages (two chunks in flight). A column's copy starts at the
-// even row at or before the tile's first row (16-byte alignment; fronts have
-// an even leading dimension) and the tile is read at that parity offset.
-// W(j, q) = -(L D)(j, q) is formed once per chunk in shared memory (double
-// buffered, D read from global) and the L fragment accumulates onto the C
-// tile held in registers: one block barrier per chunk.
+// The operands come packed from the panel kernels (packed_at): L of the
+// tile's rows and W = -(L D) of its columns, so that a chunk of 16 pivots is
+// one bulk copy (cp.async.bulk, no multicast) per operand into a ring of four
+// stages, and C += L W^T is all that is left to do. A stage has a full
+// mbarrier (its copies' bytes) and an empty one (an arrival per warp); the
+// warps take turns issuing the chunk three ahead and meet at no block
+// barrier, so that a warp's C load, store or late start hides behind the
+// other fifteen warps' MMAs.
+//
+// What bounds it is the DMMA pipe (37.1 TF/s) while a launch has several
+// tiles per CTA. Forming W in the kernel from L and D, with one copy per
+// pivot column and a block barrier per chunk, kept the pipe half idle: the
+// updates of the 64^3 27-point stencil took 38.4 ms (11.7 TF/s, most launches
+// being near updates of at most 32 pivots) and take 29.7 ms (15.2 TF/s), those
+// of a KKT system with a 15568-row front 84.8 ms (15.5) and 68.0 ms (19.3).
 namespace {
 constexpr int kTJ = 64;   // column tile width
 constexpr int kKM = 16;   // K chunk
-constexpr int kBS = 68;   // pivot-major stride of the staged B rows and W
 constexpr int kMThreads = 256;  // 8 warps
-constexpr int kMStages = 3;  // staging ring depth (two chunks in flight)
-// pivot-major stride of the staged A rows (doubles): TM + 4 keeps the
-// fragment loads conflict-free and holds the parity offset
+constexpr int kMStages = 4;     // staging ring depth (three chunks in flight)
 template <int TM>
-constexpr int kAS = TM + 4;
+constexpr int kStageDoubles = (TM / 64 + 1) * kPkTile;
 template <int TM>
 constexpr size_t mma_smem() {
-  return static_cast<size_t>(kMStages * (kKM * kAS<TM> + (kKM + 2) * kBS) + 2 * kKM * kBS) * sizeof(double);
+  return static_cast<size_t>(kMStages) * kStageDoubles<TM> * sizeof(double);
 }
 
 // c (16 x 8) += a (16 x 8) * b (8 x 8); lane (g, t) = (lane >> 2, lane & 3):
@@ -1031,8 +1050,8 @@ __device__ __forceinline__ void dmma16x8x8(double* c, const double* a, const dou
 __device__ __forceinline__ uint32_t u_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 // Bounded wait for the mbarrier phase `parity`: at most kDefaultWaitNs / 8
 // probes (each a few ns or more, so at least about a second); false when
-// they run out.
-__device__ __forceinline__ bool u_mbar_wait(uint64_t* bar, uint32_t parity) {
+// they run out, or at once when another warp's wait ran out (*err).
+__device__ __forceinline__ bool u_mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* err) {
   constexpr uint32_t kMaxProbes = static_cast<uint32_t>(kDefaultWaitNs / 8);
   for (uint32_t it = 0; it < kMaxProbes; ++it) {
     uint32_t ok;
@@ -1044,6 +1063,7 @@ __device__ __forceinline__ bool u_mbar_wait(uint64_t* bar, uint32_t parity) {
         : "r"(u_smem(bar)), "r"(parity)
         : "memory");
     if (ok) return true;
+    if ((it & 1023) == 1023 && *err != 0) return false;
   }
   return false;
 }
@@ -1057,34 +1077,31 @@ __device__ __forceinline__ void u_copy(double* dst, const double* src, uint32_t 
       : "memory");
 }
 
-// Row ranges of the tile being staged (thread 0 sets them at the tile's
-// start; only warp 0 reads them): A rows [ra, ra + na) and B rows
-// [rb, rb + nb), both starting on an even row, with na, nb even.
-struct UpdateCopyRows {
-  int ra, na, rb, nb;
-};
-
-// Issue the copies of chunk kc (kn pivots) into one ring stage: A columns
-// kc .. kc + kn, B columns kc - 1 .. kc + kn (those inside [q0, q1)), rows
-// as in cr. Warp 0: lane 0 registers the bytes on the stage's mbarrier, then
-// every lane issues one or two of the (at most 34) column copies.
-template <int TM>
-__device__ __forceinline__ void u_issue(const double* F, int64_t ld, int q0, int q1, int kc, int kn,
-                                        const UpdateCopyRows& cr, double* As, double* Bs, uint64_t* bar, int lane) {
-  const int qa = max(kc - 1, q0), qb = min(kc + kn + 1, q1);
-  const uint32_t per_a = static_cast<uint32_t>(cr.na) * sizeof(double);
-  const uint32_t per_b = static_cast<uint32_t>(cr.nb) * sizeof(double);
-  if (lane == 0) {
-    const uint32_t total = per_a * kn + per_b * (qb - qa);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(u_smem(bar)), "r"(total) : "memory");
-  }
-  __syncwarp();
-  for (int t = lane; t < kn + (qb - qa); t += 32) {
-    if (t < kn)
-      u_copy(As + t * kAS<TM>, F + (kc + t) * ld + cr.ra, per_a, bar);
-    else
-      u_copy(Bs + (qa + t - kn - kc + 1) * kBS, F + (qa + t - kn) * ld + cr.rb, per_b, bar);
+// One 8-pivot step of a warp's 32 x 8 CT sub-tile; As and Ws point at the
+// step's first pivot (lane offsets included). Edge steps take only the
+// pivots [lo, hi) of the chunk: what the packed operands hold outside them is
+// stale and may be anything, so both sides are masked.
+template <int CT, bool Edge>
+__device__ __forceinline__ void mma_step(double (&acc)[2][CT][4], const double* As, const double* Ws, int k0, int lt,
+                                         int lo, int hi) {
+  double bq[CT][2];
+#pragma unroll
+  for (int ct = 0; ct < CT; ++ct)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const double w = Ws[4 * r * kPkRow + ct * 8];
+      bq[ct][r] = (!Edge || (k0 + lt + 4 * r >= lo && k0 + lt + 4 * r < hi)) ? w : 0.0;
+    }
+#pragma unroll
+  for (int rt = 0; rt < 2; ++rt) {
+    double a[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const double l = As[4 * (r >> 1) * kPkRow + rt * 16 + 8 * (r & 1)];
+      a[r] = (!Edge || (k0 + lt + 4 * (r >> 1) >= lo && k0 + lt + 4 * (r >> 1) < hi)) ? l : 0.0;
+    }
+#pragma unroll
+    for (int ct = 0; ct < CT; ++ct) dmma16x8x8(acc[rt][ct], a, bq[ct]);
   }
 }
 }  // namespace
@@ -1095,22 +1112,23 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
                                                                FactorGlobals* g, int level, int dynamic,
                                                                const double* __restrict__ tc_guard) {
   if (level_aborted(g, level, dynamic)) return;
-  constexpr int AS = kAS<TM>;
   constexpr int WROWS = TM / 32;       // warps along the tile's rows
   constexpr int WCOLS = 8 / WROWS;     // warps along its 64 columns
   constexpr int WN = kTJ / WCOLS;      // columns per warp (32 or 16)
   constexpr int CT = WN / 8;           // 8-column MMA tiles per warp
-  extern __shared__ __align__(16) double usm[];
-  // stage b of the ring: A rows at As_of(b), B rows at Bs_of(b); W double buffered
-  auto As_of = [&](int b) { return usm + b * kKM * AS; };
-  auto Bs_of = [&](int b) { return usm + kMStages * kKM * AS + b * (kKM + 2) * kBS; };
-  auto Ws_of = [&](int b) { return usm + kMStages * (kKM * AS + (kKM + 2) * kBS) + b * kKM * kBS; };
-  __shared__ __align__(8) uint64_t full[kMStages];
-  __shared__ UpdateCopyRows copy_rows;
+  constexpr int NB = TM / 64;          // packed row tiles of L per chunk
+  extern __shared__ __align__(128) double usm[];  // stage b at usm + b * kStageDoubles: L tiles, then W
+  __shared__ __align__(8) uint64_t full[kMStages], empty[kMStages];
+  __shared__ int s_err;
+  __shared__ unsigned s_issued[kMStages];  // copies issued into each stage so far
   __shared__ int tile_end[2 * kMaxUpdateFronts];
   if (threadIdx.x == 0) {
-    for (int b = 0; b < kMStages; ++b)
+    s_err = 0;
+    for (int b = 0; b < kMStages; ++b) {
+      s_issued[b] = 0;
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(u_smem(&full[b])) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(u_smem(&empty[b])), "r"(kMThreads / 32) : "memory");
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const int nent = (MODE == 2) ? 2 * count : count;
@@ -1123,7 +1141,7 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
     bool use = update_range(S, fronts[sf].m, far, c0, c1, q0, q1);
     if (far && use && tc_guard && tc_block_ok(q1 - q0, tc_guard[2 * t], tc_guard[2 * t + 1], g->amax))
       use = false;  // the tensor-core kernel applied this block
-    tile_end[t] = use ? update_tiles(fronts[sf].m, c0, c1, kTJ, TM) : 0;
+    tile_end[t] = use ? update_tiles(fronts[sf].m, c0, c1, TM) : 0;
     if (blockIdx.x == 0 && tile_end[t] > 0) {
       const double nc = c1 - c0, mm = fronts[sf].m;
       const double entries = nc * mm - (static_cast<double>(c0) + c1 - 1) * nc / 2.0;
@@ -1136,62 +1154,29 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wr = warp / WCOLS, wc = warp % WCOLS;   // warp's 32 x WN sub-tile
   const int lg = lane >> 2, lt = lane & 3;          // fragment coordinates
+  // the warp's fragments within a stage
+  const int a_off = (wr >> 1) * kPkTile + lt * kPkRow + (wr & 1) * 32 + lg;
+  const int w_off = NB * kPkTile + lt * kPkRow + wc * WN + lg;
   double tmax = 0.0;
   int cur = -1, s = -1;
-  const double* Fp = nullptr;
-  int m = 0, c0 = 0, c1 = 0, q0 = 0, q1 = 0, nchunks = 0;
+  double* Fp = nullptr;
+  const double* P = nullptr;
+  int64_t pw = 0;
+  int m = 0, c0 = 0, c1 = 0, q0 = 0, q1 = 0, prt = 0;
   int64_t ld = 0;
-  unsigned u = 0;  // chunks consumed by this CTA so far (ring stage u % 3, phase (u / 3) & 1)
+  unsigned u = 0;  // chunks of this CTA's earlier tiles (chunk v of the CTA: stage v % 4, use v / 4 of the stage)
+  bool failed = false;
+  // a wait ran out: the factorization fails with a timeout, and the CTA's
+  // warps stop waiting and leave
+  auto fail = [&] {
+    atomicCAS(&g->error, 0, kUpdateErrTimeout);
+    *const_cast<volatile int*>(&s_err) = 1;
+  };
   // the CTA's tiles increase, so the entry fi, its column tile tj and that
   // column tile's first tile (tj_first, counted within the entry) only move
   // forward: each is advanced from where the previous tile left it
   int fi = 0, tj = 0, tj_first = 0;
-  // rows of a tile's copies, from the even row at or before its first row,
-  // rounded up to whole 16-byte pairs (the extra row of an odd m is the
-  // padding row of the front's even leading dimension); warp 0
-  auto set_copy_rows = [&](int ti0, int tj0, int tm) {
-    if (lane == 0) {
-      copy_rows.ra = ti0 & ~1;
-      copy_rows.na = ((min(ti0 + TM, tm) + 1) & ~1) - copy_rows.ra;
-      copy_rows.rb = tj0 & ~1;
-      copy_rows.nb = ((min(tj0 + kTJ, tm) + 1) & ~1) - copy_rows.rb;
-    }
-    __syncwarp();
-  };
-  // the CTA's next tile nt: its first (up to two) chunks into stages
-  // (u + 1) % 3 and (u + 2) % 3, issued by warp 0 after the barrier of this
-  // tile's last chunk u (every warp is past the chunks that used those
-  // stages). The walk runs on copies: the tile loop repeats it at nt.
-  auto issue_next = [&](int nt) {
-    int nfi = fi, ntj = tj, ntjf = tj_first;
-    while (nt >= tile_end[nfi]) {
-      ++nfi;
-      ntj = 0;
-      ntjf = 0;
-    }
-    const int ns = front_list[nfi % count];
-    const int nm = fronts[ns].m;
-    int nc0, nc1, nq0, nq1;
-    update_range(st[ns], nm, entry_far(nfi), nc0, nc1, nq0, nq1);
-    const int nrel = nt - (nfi > 0 ? tile_end[nfi - 1] : 0);
-    for (;;) {
-      const int nr = (nm - (nc0 + ntj * kTJ) + TM - 1) / TM;
-      if (nrel < ntjf + nr) break;
-      ntjf += nr;
-      ++ntj;
-    }
-    const int nj0 = nc0 + ntj * kTJ, ni0 = nj0 + (nrel - ntjf) * TM;
-    set_copy_rows(ni0, nj0, nm);
-    const int nn = (nq1 - nq0 + kKM - 1) / kKM;
-    for (int cc = 0; cc < 2 && cc < nn; ++cc) {
-      const int kc = nq0 + cc * kKM;
-      const unsigned b = (u + 1 + cc) % kMStages;
-      u_issue<TM>(fronts[ns].F, fronts[ns].ld, nq0, nq1, kc, min(kKM, nq1 - kc), copy_rows, As_of(b), Bs_of(b),
-                  &full[b], lane);
-    }
-  };
-  bool ahead = false;  // warp 0 issued this tile's first chunks during the previous tile
-  for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+  for (int tile = blockIdx.x; tile < total && !failed; tile += gridDim.x) {
     while (tile >= tile_end[fi]) {
       ++fi;
       tj = 0;
@@ -1206,30 +1191,52 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
       cur = fi;
       s = front_list[fi % count];
       Fp = fronts[s].F;
+      P = fronts[s].P;
+      pw = fronts[s].pw;
+      prt = fronts[s].prt;
       m = fronts[s].m;
       ld = fronts[s].ld;
       update_range(st[s], m, entry_far(fi), c0, c1, q0, q1);
-      nchunks = (q1 - q0 + kKM - 1) / kKM;
+      // pivots relative to the outer block
+      q0 -= st[s].ob;
+      q1 -= st[s].ob;
     }
     const int rel = tile - (fi > 0 ? tile_end[fi - 1] : 0);
     for (;;) {
-      const int nr = (m - (c0 + tj * kTJ) + TM - 1) / TM;
+      const int nr = (m - ((c0 & ~63) + tj * kTJ) + TM - 1) / TM;
       if (rel < tj_first + nr) break;
       tj_first += nr;
       ++tj;
     }
-    const int j0 = c0 + tj * kTJ, i0 = j0 + (rel - tj_first) * TM;
-    const int sa = i0 & 1, sb = j0 & 1;  // parity offsets of the staged rows
-    __syncthreads();  // previous tile done with every stage and with W
-    if (warp == 0 && !ahead) {
-      set_copy_rows(i0, j0, m);
-      for (int c = 0; c < 2 && c < nchunks; ++c) {
-        const int kc = q0 + c * kKM;
-        const unsigned b = (u + c) % kMStages;
-        u_issue<TM>(Fp, ld, q0, q1, kc, min(kKM, q1 - kc), copy_rows, As_of(b), Bs_of(b), &full[b], lane);
+    const int j0 = (c0 & ~63) + tj * kTJ, i0 = j0 + (rel - tj_first) * TM;
+    const int kc0 = q0 >> 4, nchunks = ((q1 + 15) >> 4) - kc0;
+    // issue chunk c of this tile: wait until every warp is done with the
+    // stage's previous chunk, then one copy per operand
+    auto issue = [&](int c) {
+      bool ok = true;
+      if (lane == 0) {
+        const unsigned v = u + c, b = v % kMStages, use = v / kMStages;
+        if (use > 0 && !u_mbar_wait(&empty[b], (use - 1) & 1, &s_err)) {
+          ok = false;
+          fail();
+        } else {
+          s_issued[b] = use + 1;
+          const uint32_t ba = static_cast<uint32_t>(min(NB, prt - (i0 >> 6))) * kPkTile * sizeof(double);
+          constexpr uint32_t bw = kPkTile * sizeof(double);
+          double* dst = usm + b * kStageDoubles<TM>;
+          const double* src = P + static_cast<int64_t>(kc0 + c) * prt * kPkTile;
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(u_smem(&full[b])), "r"(ba + bw)
+                       : "memory");
+          u_copy(dst, src + static_cast<int64_t>(i0 >> 6) * kPkTile, ba, &full[b]);
+          u_copy(dst + NB * kPkTile, src + pw + static_cast<int64_t>(j0 >> 6) * kPkTile, bw, &full[b]);
+        }
       }
-    }
-    ahead = false;
+      failed = !__shfl_sync(0xffffffffu, ok, 0);
+    };
+    if (warp < kMStages - 1 && warp < nchunks) issue(warp);
+    // the warp's sub-tile has entries of the lower triangle
+    const bool busy = i0 + wr * 32 < m && j0 + wc * WN < c1 && j0 + wc * WN + WN > c0 && i0 + wr * 32 + 31 >= j0 + wc * WN;
     // C tile into the accumulators (lane holds rows gi0 + 16 rt + 8 v,
     // columns gj0 + 8 ct + h as acc[rt][ct][2 v + h])
     const int gi0 = i0 + wr * 32 + lg, gj0 = j0 + wc * WN + 2 * lt;
@@ -1239,104 +1246,57 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int gj = gj0 + ct * 8 + h;
-        const double* colp = Fp + static_cast<int64_t>(gj < c1 ? gj : 0) * ld;
+        const bool in = gj >= c0 && gj < c1;
+        const double* colp = Fp + static_cast<int64_t>(in ? gj : 0) * ld;
 #pragma unroll
         for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
           for (int v = 0; v < 2; ++v) {
             const int gi = gi0 + rt * 16 + 8 * v;
-            acc[rt][ct][2 * v + h] = (gj < c1 && gi < m && gi >= gj) ? colp[gi] : 0.0;
+            acc[rt][ct][2 * v + h] = (in && gi < m && gi >= gj) ? colp[gi] : 0.0;
           }
       }
-    // D of this thread's pivot of a chunk (pivot q = threadIdx.x / 16 of the
-    // chunk; W row q, columns (threadIdx.x % 16) + 16 j): loaded one chunk
-    // ahead into registers, so no global load waits between a chunk's
-    // staging and its barrier
-    const int wq = threadIdx.x >> 4, wr0 = threadIdx.x & 15;
-    int dk = 0;
-    double dd = 0.0, dn = 0.0, dp = 0.0;
-    auto load_d = [&](int kc, int kn) {
-      if (wq < kn) {
-        const FrontDesc& fd = fronts[s];
-        const int pq = kc + wq;
-        dk = fd.pk[pq];
-        dd = fd.Dd[pq];
-        dn = fd.Do[pq];
-        dp = pq > 0 ? fd.Do[pq - 1] : 0.0;
+    for (int c = 0; c < nchunks; ++c) {
+      // the chunk three ahead, by the warps in turn
+      if (warp == ((c + kMStages - 1) & 7) && c + kMStages - 1 < nchunks) issue(c + kMStages - 1);
+      if (failed) break;
+      const unsigned v = u + c, b = v % kMStages;
+      if (!__all_sync(0xffffffffu, u_mbar_wait(&full[b], (v / kMStages) & 1, &s_err))) {
+        fail();
+        failed = true;
+        break;
       }
-    };
-    load_d(q0, min(kKM, q1 - q0));
-    for (int c = 0; c < nchunks; ++c, ++u) {
-      const int kc = q0 + c * kKM, kn = min(kKM, q1 - kc);
-      const unsigned b = u % kMStages;
-      if (!u_mbar_wait(&full[b], (u / kMStages) & 1)) {
-        // a copy did not land within the wait limit: record it (the
-        // factorization then fails with a timeout) and wait once more,
-        // bounded, for this stage's copies before going on
-        atomicCAS(&g->error, 0, kUpdateErrTimeout);
-        u_mbar_wait(&full[b], (u / kMStages) & 1);
-      }
-      double* As = As_of(b);
-      const double* Bs = Bs_of(b) + sb;
-      double* Ws = Ws_of(c & 1);
-      // the MMAs run over 8-pivot steps: A columns past kn are zeroed (the
-      // stage's copies did not write them), W rows past kn are zero
-      const int kn8 = (kn + 7) & ~7;
-      for (int t = threadIdx.x; t < (kn8 - kn) * AS; t += kMThreads) As[kn * AS + t] = 0.0;
-      // W(j, q) = -(L D)(j, q)
-      if (wq < kn8) {
+      if (busy) {
+        const int lo = q0 - (kc0 + c) * kKM, hi = q1 - (kc0 + c) * kKM;  // the update's pivots of this chunk
+        const double* stage = usm + b * kStageDoubles<TM>;
+        if (lo <= 0 && hi >= kKM) {
 #pragma unroll
-        for (int j = 0; j < kTJ / 16; ++j) {
-          const int r = wr0 + 16 * j;
-          double w = 0.0;
-          if (wq < kn) {
-            const double* col = Bs + (wq + 1) * kBS + r;
-            w = dd * col[0];
-            if (dk == 1) w += dn * col[kBS];
-            if (dk == 2) w += dp * col[-kBS];
-          }
-          Ws[wq * kBS + r] = -w;
+          for (int k0 = 0; k0 < kKM; k0 += 8)
+            mma_step<CT, false>(acc, stage + a_off + k0 * kPkRow, stage + w_off + k0 * kPkRow, k0, lt, lo, hi);
+        } else {
+          for (int k0 = 0; k0 < kKM; k0 += 8)
+            if (k0 < hi && k0 + 8 > lo)
+              mma_step<CT, true>(acc, stage + a_off + k0 * kPkRow, stage + w_off + k0 * kPkRow, k0, lt, lo, hi);
         }
       }
-      __syncthreads();  // W and the zeroed columns ready; every thread is past chunk c - 1
-      if (c + 1 < nchunks) load_d(kc + kKM, min(kKM, q1 - kc - kKM));
-      if (warp == 0 && c + 2 < nchunks) {
-        const int kc2 = kc + 2 * kKM;
-        const unsigned b2 = (u + 2) % kMStages;
-        u_issue<TM>(Fp, ld, q0, q1, kc2, min(kKM, q1 - kc2), copy_rows, As_of(b2), Bs_of(b2), &full[b2], lane);
-      } else if (warp == 0 && c == nchunks - 1 && tile + static_cast<int>(gridDim.x) < total) {
-        issue_next(tile + static_cast<int>(gridDim.x));
-        ahead = true;
-      }
-      const double* Aq = As + sa;
-      for (int k0 = 0; k0 < kn8; k0 += 8) {
-        double bq[CT][2];
-#pragma unroll
-        for (int ct = 0; ct < CT; ++ct)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) bq[ct][r] = Ws[(k0 + lt + 4 * r) * kBS + wc * WN + ct * 8 + lg];
-#pragma unroll
-        for (int rt = 0; rt < 2; ++rt) {
-          double a[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) a[r] = Aq[(k0 + lt + 4 * (r >> 1)) * AS + wr * 32 + rt * 16 + lg + 8 * (r & 1)];
-#pragma unroll
-          for (int ct = 0; ct < CT; ++ct) dmma16x8x8(acc[rt][ct], a, bq[ct]);
-        }
-      }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(u_smem(&empty[b])) : "memory");
     }
+    u += nchunks;
+    if (failed) break;
 #pragma unroll
     for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int gj = gj0 + ct * 8 + h;
-        double* colp = const_cast<double*>(Fp) + static_cast<int64_t>(gj < c1 ? gj : 0) * ld;
+        const bool in = gj >= c0 && gj < c1;
+        double* colp = Fp + static_cast<int64_t>(in ? gj : 0) * ld;
 #pragma unroll
         for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
           for (int v = 0; v < 2; ++v) {
             const int gi = gi0 + rt * 16 + 8 * v;
-            if (gj < c1 && gi < m && gi >= gj) {
+            if (in && gi < m && gi >= gj) {
               colp[gi] = acc[rt][ct][2 * v + h];
               tmax = fmax(tmax, fabs(acc[rt][ct][2 * v + h]));
             }
@@ -1346,6 +1306,15 @@ __global__ void __launch_bounds__(kMThreads, 2) update_mma_kernel(const FrontDes
   if (cur >= 0) {
     tmax = warp_max(tmax);
     if (lane == 0) atomic_max_nonneg(&st[s].running_max, tmax);
+  }
+  if (failed && lane == 0) {
+    // the copies in flight must land before the CTA's shared memory goes
+    // (bounded; every warp of a failed CTA sees the error and comes here)
+    const int none = 0;
+    for (int b = 0; b < kMStages; ++b) {
+      const unsigned n = *const_cast<volatile unsigned*>(&s_issued[b]);
+      if (n > 0) u_mbar_wait(&full[b], (n - 1) & 1, &none);
+    }
   }
 }
 

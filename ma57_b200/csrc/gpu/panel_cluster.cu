@@ -185,6 +185,13 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   }
   __syncthreads();
 
+  // packed operands of the Schur updates (common.cuh): L and -(L D) of pivot
+  // kk, row i
+  auto put_packed = [&](int kk, int i, double l, double a) {
+    double* pk = f.P + packed_at(f.prt, kk - S.ob, i);
+    pk[0] = l;
+    pk[f.pw] = -a;
+  };
   auto owner = [&](int i) { return (i - ps) / Rr; };
   auto remote = [&](auto* p, int rank) { return cluster.map_shared_rank(p, rank); };
 
@@ -242,7 +249,18 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   };
   // symmetric interchange of positions a < b: global front, row indices and
   // the shared copies of both rows / current values
-  auto interchange = [&](int a, int b, bool swapVr) {
+  auto interchange = [&](int a, int b, int k, bool swapVr) {
+    // packed rows of the outer block's pivots so far
+    for (int t = q * kCT + threadIdx.x; t < k - S.ob; t += CS * kCT) {
+      double* pa = f.P + packed_at(f.prt, t, a);
+      double* pb = f.P + packed_at(f.prt, t, b);
+      double x = pa[0];
+      pa[0] = pb[0];
+      pb[0] = x;
+      x = pa[f.pw];
+      pa[f.pw] = pb[f.pw];
+      pb[f.pw] = x;
+    }
     // global front: split the m-1 index range over the cluster
     for (int t = q * kCT + threadIdx.x; t < m - 1; t += CS * kCT) {
       if (t < a) {
@@ -372,6 +390,7 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
       const double l = a * inv;
       Lr[p * R + li] = l;
       F[k * ld + i] = l;
+      put_packed(k, i, l, a);
     }
     if (threadIdx.x == 0) {
       sh.Dd[p] = d;
@@ -639,12 +658,19 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
         any_accept = true;
         for (int c = 0; c < kstar; ++c) {
           const double iv = sh.iv[c];
-          for (int i = r0 + threadIdx.x; i < rend; i += kCT)
-            F[static_cast<int64_t>(k0 + c) * ld + i] = Lr[(p0 + c) * R + (i - base)] * iv;
+          for (int i = r0 + threadIdx.x; i < rend; i += kCT) {
+            const double a = Lr[(p0 + c) * R + (i - base)];
+            F[static_cast<int64_t>(k0 + c) * ld + i] = a * iv;
+            put_packed(k0 + c, i, a * iv, a);
+          }
         }
         if (q == 0) {
           for (int c = 0; c < kstar; ++c)
-            for (int i = c + threadIdx.x; i < np; i += kCT) F[static_cast<int64_t>(k0 + c) * ld + k0 + i] = sh.db[i][c];
+            for (int i = c + threadIdx.x; i < np; i += kCT) {
+              F[static_cast<int64_t>(k0 + c) * ld + k0 + i] = sh.db[i][c];
+              // block rows past the accepted pivots are rows of the updates
+              if (i >= kstar) put_packed(k0 + c, k0 + i, sh.db[i][c], sh.wv[i][c]);
+            }
           for (int c = threadIdx.x; c < kstar; c += kCT) {
             f.Dd[k0 + c] = sh.dv[c];
             f.Do[k0 + c] = 0.0;
@@ -844,13 +870,13 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     }
     pf_col = -1;  // an interchange invalidates the prefetched column
     if (dec == 1) {
-      interchange(k, r, true);
+      interchange(k, r, k, true);
       finish_1x1(p, arr, vr);
       __syncthreads();
       k += 1;
     } else {
       // 2x2 at (k, r): bring r to k+1
-      if (r != k + 1) interchange(k + 1, r, true);
+      if (r != k + 1) interchange(k + 1, r, k, true);
       const double d11 = akk, d21 = vkr, d22 = arr;
       const double det = d11 * d22 - d21 * d21;
       // cluster-uniform value (the running max known at panel start), so
@@ -886,6 +912,8 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
         Lr[(p + 1) * R + li] = l1;
         F[k * ld + i] = l0;
         F[(k + 1) * ld + i] = l1;
+        put_packed(k, i, l0, a0);
+        put_packed(k + 1, i, l1, a1);
       }
       if (threadIdx.x == 0) {
         sh.Dd[p] = d11;
