@@ -253,19 +253,36 @@ void build_maps(const std::vector<int>& cbRows, const std::unordered_map<int, in
 }
 
 // The children (offsets) of a front with a row in each 32-column block, from
-// their extend-add maps; rel(t) is child t's map to the front's rows.
-template <typename Rel>
-void block_children(int m, int nchildren, Rel&& rel, std::vector<int>& ptr, std::vector<int>& child) {
+// their extend-add maps: rel(t) points at child t's map to the front's rows,
+// cb(t) entries.
+template <typename Rel, typename Cb>
+void block_children(int m, int nchildren, Rel&& rel, Cb&& cb, std::vector<int>& ptr, std::vector<int>& child) {
   const int nb = (m + 31) / 32;
-  std::vector<std::vector<int>> of(nb);
-  for (int t = 0; t < nchildren; ++t)
-    for (const int loc : rel(t))
-      if (of[loc / 32].empty() || of[loc / 32].back() != t) of[loc / 32].push_back(t);
-  ptr.assign(1, 0);
-  child.clear();
-  for (const auto& v : of) {
-    child.insert(child.end(), v.begin(), v.end());
-    ptr.push_back(static_cast<int>(child.size()));
+  std::vector<int> last(nb, -1);
+  ptr.assign(nb + 1, 0);
+  for (int t = 0; t < nchildren; ++t) {
+    const int* r = rel(t);
+    for (int i = 0, n = cb(t); i < n; ++i) {
+      const int b = r[i] >> 5;
+      if (last[b] != t) {
+        last[b] = t;
+        ++ptr[b + 1];
+      }
+    }
+  }
+  for (int b = 0; b < nb; ++b) ptr[b + 1] += ptr[b];
+  child.resize(ptr[nb]);
+  std::vector<int> fill(ptr.begin(), ptr.end() - 1);
+  std::fill(last.begin(), last.end(), -1);
+  for (int t = 0; t < nchildren; ++t) {
+    const int* r = rel(t);
+    for (int i = 0, n = cb(t); i < n; ++i) {
+      const int b = r[i] >> 5;
+      if (last[b] != t) {
+        last[b] = t;
+        child[fill[b]++] = t;
+      }
+    }
   }
 }
 
@@ -308,7 +325,7 @@ void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, 
   L.touch.clear();
   L.all = frontsOfLevel;
   L.small_max_m = L.large_max_m = 0;
-  L.panels = 0;
+  L.panels = L.static_panels = 0;
   L.small_flops = 0.0;
   L.assemble_bytes = 0.0;
   L.trailing_flops.clear();
@@ -361,6 +378,7 @@ void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, 
     // two CTAs per SM)
     L.trailing_grid = std::max(1, std::min(tiles * static_cast<int>(L.large.size()), 148));
     // fronts too tall for a full-width cluster panel take narrower panels
+    L.static_panels = L.panels;
     L.panel_width = panel_width_for(L.large_max_m, static_cast<int>(L.large.size()));
     if (L.panel_width != kPanelWidth) {
       L.panels = 0;
@@ -605,12 +623,8 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
     if (f.m > kSmallFrontMax)
       block_children(
           f.m, static_cast<int>(f.children.size()),
-          [&](int t) {
-            const LinkTmp& lt = ltmp[c->link_begin_static[s] + t];
-            rel.assign(mapPool.begin() + lt.rel, mapPool.begin() + lt.rel + lt.cb);
-            return rel;
-          },
-          c->fronts[s].blk_ptr, c->fronts[s].blk_child);
+          [&](int t) { return mapPool.data() + ltmp[c->link_begin_static[s] + t].rel; },
+          [&](int t) { return ltmp[c->link_begin_static[s] + t].cb; }, c->fronts[s].blk_ptr, c->fronts[s].blk_child);
     c->link_end_static[s] = static_cast<int>(ltmp.size());
   }
   c->d_maps = dupload(mapPool, c->stream);
@@ -631,6 +645,7 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   // A entries: (final column lo, pattern position of hi) -> value index
   struct AEnt {
     int col, pos, j, idx;
+    int block() const { return col - j % 32; }  // first column of the entry's 32-column block
   };
   std::vector<AEnt> ents;
   ents.reserve(c->nnz);
@@ -651,8 +666,7 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   // (or of the whole front) stays contiguous and the entries of a row of a
   // block are consecutive (the assembly's order)
   std::sort(ents.begin(), ents.end(), [](const AEnt& a, const AEnt& b) {
-    const int ka = a.col - a.j % 32, kb = b.col - b.j % 32;
-    if (ka != kb) return ka < kb;
+    if (a.block() != b.block()) return a.block() < b.block();
     return a.pos != b.pos ? a.pos < b.pos : a.col < b.col;
   });
   std::vector<int> acolptr(n + 1, 0), aj(ents.size()), apos(ents.size()), aidx(ents.size());
@@ -706,7 +720,7 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   std::vector<std::vector<int>> byLevel(numLevels);
   for (int s = 0; s < numSN; ++s) byLevel[c->fronts[s].level].push_back(s);
   c->levels.assign(numLevels, LevelLists());
-  c->level_iters.assign(numLevels, 0);
+  for (auto& v : c->level_iters) v.assign(numLevels, 0);
   c->graph_level_iters.clear();
   for (int l = 0; l < numLevels; ++l) {
     build_level_lists(c, byLevel[l], c->levels[l]);
@@ -886,6 +900,12 @@ void validate_tables(symla_gpu_ctx* c, int phase, const KernelOpts& ko, const ch
 constexpr int kSinglePanelMaxFronts = 148;
 constexpr int kSinglePanelMaxM = 1024;
 
+// Static pivoting runs its own panel kernel unless the single-CTA one is
+// asked for.
+bool use_static_panel(const symla_gpu_ctx* c, const LevelLists& L, const KernelOpts& ko) {
+  return ko.mode == SYMLA_MODE_STATIC && c->use_cluster_panel && L.cluster_ctas != 1;
+}
+
 void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko, int dynamic,
                             const int* d_large) {
   cudaStream_t st = c->stream;
@@ -896,11 +916,13 @@ void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, co
     // threshold (Bunch-Kaufman) mode, for levels of fewer large fronts than
     // SMs none taller than kSinglePanelMaxM rows: there the cluster's
     // barriers on every pivot-by-pivot decision cost more than its spread of
-    // rows saves (static pivoting never leaves the speculative path, so it
-    // keeps the cluster)
+    // rows saves. Static pivoting has its own kernel.
     const bool single = L.cluster_ctas == 1 || (L.cluster_ctas == 0 && ko.mode == SYMLA_MODE_THRESHOLD &&
                                                 nl < kSinglePanelMaxFronts && L.large_max_m <= kSinglePanelMaxM);
-    if (c->use_cluster_panel && !single && cluster_size_for(L.large_max_m, nl, L.panel_width) > 0) {
+    if (use_static_panel(c, L, ko)) {
+      launch_static_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, ko, c->d_glob, level, dynamic, st);
+      CK(cudaGetLastError());
+    } else if (c->use_cluster_panel && !single && cluster_size_for(L.large_max_m, nl, L.panel_width) > 0) {
       CK(launch_cluster_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, L.panel_width, ko, c->d_glob, level,
                               dynamic, st, L.cluster_ctas));
     } else {
@@ -973,14 +995,15 @@ void complete_level(symla_gpu_ctx* c, const LevelLists& L, int level, const Kern
 // Panel iterations to launch for a level before checking it on the host:
 // the planned count, or the most an earlier factorization of the same plan
 // needed (the same pattern usually pivots alike).
-int level_plan_iters(const symla_gpu_ctx* c, const LevelLists& L, int level) {
-  const int seen = level < static_cast<int>(c->level_iters.size()) ? c->level_iters[level] : 0;
-  return std::max(L.panels, seen);
+int level_plan_iters(const symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko) {
+  const auto& iters = c->level_iters[ko.mode == SYMLA_MODE_STATIC];
+  const int seen = level < static_cast<int>(iters.size()) ? iters[level] : 0;
+  return std::max(use_static_panel(c, L, ko) ? L.static_panels : L.panels, seen);
 }
 
 void launch_level(symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko, int dynamic,
                   const int* d_small, const int* d_large) {
-  const int iters = level_plan_iters(c, L, level);
+  const int iters = level_plan_iters(c, L, level, ko);
   FactorGlobals before{};
   if (c->profiling && !L.large.empty()) {
     CK(cudaMemcpyAsync(&before, c->d_glob, sizeof before, cudaMemcpyDeviceToHost, c->stream));
@@ -1026,8 +1049,8 @@ void complete_level(symla_gpu_ctx* c, const LevelLists& L, int level, const Kern
       launched += 4;
     }
   }
-  if (level < static_cast<int>(c->level_iters.size()))
-    c->level_iters[level] = std::max(c->level_iters[level], std::min(launched, 4 * L.panels + 64));
+  auto& iters = c->level_iters[ko.mode == SYMLA_MODE_STATIC];
+  if (level < static_cast<int>(iters.size())) iters[level] = std::max(iters[level], std::min(launched, 4 * L.panels + 64));
   CK(cudaGetLastError());
 }
 
@@ -1037,15 +1060,17 @@ void complete_level(symla_gpu_ctx* c, const LevelLists& L, int level, const Kern
 // return at once). Captured once per set of kernel options and iteration
 // counts and replayed; no host synchronisation inside. A level that ran past
 // its count raises it, so the next factorization recaptures with room.
-int graph_iters(const symla_gpu_ctx* c, const LevelLists& L, int level) {
-  const int n = level_plan_iters(c, L, level);
+int graph_iters(const symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko) {
+  const int n = level_plan_iters(c, L, level, ko);
+  // static pivoting needs exactly its plan
+  if (use_static_panel(c, L, ko)) return n;
   return n + n / 8 + 2;
 }
 
 void run_static_pass_graph(symla_gpu_ctx* c, const KernelOpts& ko) {
   cudaStream_t st = c->stream;
   std::vector<int> iters(c->numLevels);
-  for (int l = 0; l < c->numLevels; ++l) iters[l] = graph_iters(c, c->levels[l], l);
+  for (int l = 0; l < c->numLevels; ++l) iters[l] = graph_iters(c, c->levels[l], l, ko);
   const bool same = c->graph_exec && std::memcmp(&c->graph_ko, &ko, sizeof ko) == 0 && iters == c->graph_level_iters;
   if (!same) {
     if (c->graph_exec) {
@@ -1164,12 +1189,8 @@ void replan_front(symla_gpu_ctx* c, int s) {
   }
   if (f.m > kSmallFrontMax)
     block_children(
-        f.m, static_cast<int>(f.children.size()),
-        [&](int t) {
-          rel.assign(pool.begin() + offs[t].second, pool.begin() + offs[t].second + cbRowsOf[t].size());
-          return rel;
-        },
-        f.dyn_blk_ptr, f.dyn_blk_child);
+        f.m, static_cast<int>(f.children.size()), [&](int t) { return pool.data() + offs[t].second; },
+        [&](int t) { return static_cast<int>(cbRowsOf[t].size()); }, f.dyn_blk_ptr, f.dyn_blk_child);
   int* dmaps = dupload(pool, c->stream);
   c->dyn_allocs.push_back(dmaps);
   const int begin = static_cast<int>(c->hlinks.size());

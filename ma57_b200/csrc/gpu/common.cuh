@@ -66,6 +66,7 @@ struct FrontState {
                    // columns beyond ob_end is deferred to one far update
   int far;         // 1: the far update of [ob, k) is due after this panel
   int spec;        // consecutive panels whose speculative first pivot failed
+  int ticket;      // CTAs of the static panel in flight that have finished
   double perturb;
   double orig_max;
   double running_max;

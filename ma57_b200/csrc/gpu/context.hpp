@@ -39,7 +39,8 @@ struct LevelLists {
   int small_threads = 0;       // tile schedule (autotuner): small-front kernel width, 0 = by size
   int cluster_ctas = 0;        // panel cluster size, 0 = by size
   int update_rows = 0;         // rows per Schur-update tile (64 or 128), 0 = 128
-  int panels = 0;              // panel iterations needed
+  int panels = 0;              // panel iterations needed (threshold pivoting)
+  int static_panels = 0;       // and under static pivoting
   int panel_width = 32;        // pivots per panel (narrower for fronts too tall for a full-width cluster panel)
   double* d_panel_cols = nullptr;  // single-CTA panel kernel, fronts too tall for shared memory: 2 m per front
   int trailing_grid = 0;
@@ -161,7 +162,6 @@ struct symla_gpu_ctx {
   double* d_hscratch = nullptr;   // backward helper-part partial sums
   int hslot_count = 0;
   int* d_counter = nullptr;  // unfinished-front counter
-  int flag_count = 0;
   int solve_epoch = 0;
   int fwd_resident = 0, bwd_resident = 0;
   std::vector<int> solve_np;  // npiv per front the task lists were built for
@@ -230,8 +230,9 @@ struct symla_gpu_ctx {
   int graph_captures = 0, graph_resumes = 0;
   long long graph_kernels = 0;  // kernel nodes of the captured graph (counted per replay)
   // panel iterations per level: the most any factorization of this plan
-  // needed (0: within the plan), and the counts the captured graph holds
-  std::vector<int> level_iters, graph_level_iters;
+  // needed in each pivoting mode (0: within the plan), and the counts the
+  // captured graph holds
+  std::vector<int> level_iters[2], graph_level_iters;
 
   // instrumentation
   bool profiling = false;

@@ -41,7 +41,11 @@ bool panel_fits_shared(int max_m);
 cudaError_t launch_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m, int nb,
                          const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream,
                          double* cols);
-// Cluster panel (panel_cluster.cu): returns 0 from cluster_size_for when a
+// Static pivoting (panel_static.cu): panels of kPanelWidth pivots whatever the
+// front's size.
+void launch_static_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m,
+                         const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream);
+// Cluster panel (panel_cluster.cu), threshold pivoting: returns 0 from cluster_size_for when a
 // front is too large for it with nb-pivot panels (the single-CTA panel
 // kernel then runs).
 int cluster_size_for(int max_m, int count, int nb = kPanelWidth);

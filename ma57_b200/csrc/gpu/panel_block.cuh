@@ -1,0 +1,197 @@
+// The two halves of an unpivoted panel of at most 32 pivots, shared by the
+// static and the speculative panel kernels: the diagonal block's LDL^T by one
+// warp, and the rows below it.
+#pragma once
+
+#include "common.cuh"
+
+namespace symla_gpu {
+
+constexpr int kPanelMax = 32;    // pivots per panel
+constexpr int kBlkStride = 34;   // even: pairs of a row are one 16-byte load
+
+// The diagonal block in shared memory. In: db's lower triangle, the block's
+// current values. Out: L below the diagonal of db (d on it) and, transposed,
+// above the diagonal of dt; wv[i][c] = the current value of row i in column c
+// before scaling, d_c L(i, c); d, 1 / d and the applied perturbation.
+struct alignas(16) DiagBlock {
+  double db[kPanelMax][kBlkStride];
+  double dt[kPanelMax][kBlkStride];
+  double wv[kPanelMax][kBlkStride];
+  double dv[kPanelMax], iv[kPanelMax], pv[kPanelMax];
+};
+
+// Static pivoting (dense_kernel.hpp:982-1034): the pivot that replaces akk,
+// without a branch (a NaN is left alone).
+__device__ __forceinline__ double static_pivot(double akk, int sign, double floorv, double delta) {
+  const double t = sign == 0 ? fabs(akk) : (sign > 0 ? akk : -akk);
+  const bool up = sign > 0 || (sign == 0 && akk >= 0.0);
+  return t < floorv ? akk + (up ? delta : -delta) : akk;
+}
+
+// 1 / d: two Newton steps on the hardware's approximation (under one ulp off),
+// or the correctly rounded reciprocal where a step could overflow or lose
+// bits to underflow.
+__device__ __forceinline__ double pivot_reciprocal(double d) {
+  const double m = fabs(d);
+  if (!(m > 1e-290 && m < 1e290)) return __drcp_rn(d);  // uniform: every lane has the same pivot
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  double e = fma(-d, r, 1.0);
+  r = fma(r, e, r);
+  e = fma(-d, r, 1.0);
+  return fma(r, e, r);
+}
+
+// LDL^T of the np x np block by one warp, lane = row, in steps of eight
+// columns: the step's columns of the lane's row are brought up to date from
+// the earlier steps (left-looking, the row's values in registers, eight
+// independent sums), then every lane factors the 8 x 8 diagonal block
+// redundantly in registers while it eliminates its own row. No shuffle, and
+// three warp barriers per step instead of two per column. Entries past np are
+// garbage of which no row or column below np depends.
+//
+// What bounds it is the chain of 32 reciprocals, each followed by the update of the
+// next pivot (one warp, 255 registers allowed). Column by column, with the
+// row in shared memory, a column took 890 cycles (14 us per block); now it
+// takes 250 (4.1 us).
+template <bool Static>
+__device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane, int lane_sign, double floorv,
+                                                  double delta) {
+  double a[kPanelMax];  // the lane's row: values before scaling, by column
+#pragma unroll
+  for (int j0 = 0; j0 < kPanelMax; j0 += 8) {
+    if (j0 >= np) break;
+    double x[8];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(&B.db[lane][j0 + c]);
+      x[c] = v.x;
+      x[c + 1] = v.y;
+    }
+#pragma unroll
+    for (int t = 0; t < j0; t += 2)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const double2 l = *reinterpret_cast<const double2*>(&B.db[j0 + c][t]);
+        x[c] = fma(-a[t], l.x, x[c]);
+        x[c] = fma(-a[t + 1], l.y, x[c]);
+      }
+    if (lane >= j0 && lane < j0 + 8)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) B.db[lane][j0 + c] = x[c];
+    __syncwarp();
+    double T[8][8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int c = 0; c <= r; ++c) T[r][c] = B.db[j0 + r][j0 + c];
+    __syncwarp();
+    int sign[8];
+    if (Static)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) sign[c] = __shfl_sync(0xffffffffu, lane_sign, j0 + c);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int col = j0 + c;
+      const double akk = T[c][c];
+      double d = akk;
+      if (Static) d = static_pivot(akk, sign[c], floorv, delta);
+      const double inv = pivot_reciprocal(d);
+      double l[8];
+#pragma unroll
+      for (int r = c + 1; r < 8; ++r) l[r] = T[r][c] * inv;
+#pragma unroll
+      for (int r2 = c + 1; r2 < 8; ++r2)
+#pragma unroll
+        for (int r = r2; r < 8; ++r) T[r][r2] = fma(-T[r][c], l[r2], T[r][r2]);
+      const double v = x[c];
+      a[col] = v;
+#pragma unroll
+      for (int c2 = c + 1; c2 < 8; ++c2) x[c2] = fma(-v, l[c2], x[c2]);
+      // every lane stores: what lands on the other side of the diagonal is
+      // not read
+      const double li = v * inv;
+      B.db[lane][col] = lane == col ? d : li;
+      B.dt[col][lane] = li;
+      B.wv[lane][col] = v;
+      B.dv[col] = d;
+      B.iv[col] = inv;
+      if (Static) B.pv[col] = d - akk;
+    }
+    __syncwarp();
+  }
+}
+
+// A row below the block: a[t] becomes the row's current value in column t
+// (right-looking: a_c -= a_t L(c, t); L = a / d). Columns past np are computed
+// on garbage and not used. The loads of L are warp-uniform pairs. (Two rows
+// per thread would halve them, but leave no registers to load ahead with: the
+// pass then waits for every pair and took 10 us instead of 2.)
+__device__ __forceinline__ void panel_row(const DiagBlock& B, int np, double (&a)[kPanelMax]) {
+#pragma unroll
+  for (int t = 0; t < kPanelMax - 1; ++t) {
+    if ((t & 7) == 0 && t >= np) break;
+    if (!(t & 1)) a[t + 1] = fma(-a[t], B.dt[t][t + 1], a[t + 1]);
+#pragma unroll
+    for (int c = (t + 2) & ~1; c < kPanelMax; c += 2) {
+      const double2 l = *reinterpret_cast<const double2*>(&B.dt[t][c]);
+      a[c] = fma(-a[t], l.x, a[c]);
+      a[c + 1] = fma(-a[t], l.y, a[c + 1]);
+    }
+  }
+}
+
+// Column maxima of a warp's rows: lane c returns the largest |a[c]| over the
+// warp's lanes with `in` set (bit patterns of non-negative doubles order like
+// the values, and a NaN wins): per column a 32-bit reduction of the high words
+// and one of the low words that go with the largest.
+__device__ __forceinline__ unsigned long long warp_column_max(const double (&a)[kPanelMax], bool in, int np, int lane) {
+  unsigned hi = 0, lo = 0;
+#pragma unroll
+  for (int c = 0; c < kPanelMax; ++c) {
+    if ((c & 7) == 0 && c >= np) break;
+    const unsigned long long b = in ? static_cast<unsigned long long>(__double_as_longlong(fabs(a[c]))) : 0ull;
+    const unsigned h = static_cast<unsigned>(b >> 32);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, h);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, h == mh ? static_cast<unsigned>(b) : 0u);
+    if (lane == c) {
+      hi = mh;
+      lo = ml;
+    }
+  }
+  return lane < np ? static_cast<unsigned long long>(hi) << 32 | lo : 0ull;
+}
+
+// A row's L = a / d and -(L D) = -a in the packed operands (p: pivot q0 of the
+// row), and put(c, l) for every column c < np: eight columns at a time, so
+// that the loads of 1 / d do not wait for the stores before them.
+template <class Put>
+__device__ __forceinline__ void store_panel_row(const DiagBlock& B, int np, const double (&a)[kPanelMax], double* P,
+                                                int64_t pw, int prt, int q0, int i, Put&& put) {
+  double* p = P + packed_at(prt, q0, i);
+  const int64_t next = static_cast<int64_t>(prt) * kPkTile - 16 * kPkRow;  // to the next 16-pivot chunk
+#pragma unroll
+  for (int c0 = 0; c0 < kPanelMax; c0 += 8) {
+    if (c0 >= np) break;
+    double l[8];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 iv = *reinterpret_cast<const double2*>(&B.iv[c0 + c]);
+      l[c] = a[c0 + c] * iv.x;
+      l[c + 1] = a[c0 + c + 1] * iv.y;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c0 + c < np) {
+        put(c0 + c, l[c]);
+        p[0] = l[c];
+        p[pw] = -a[c0 + c];
+      }
+      p += kPkRow;
+      if (((q0 + c0 + c + 1) & 15) == 0) p += next;
+    }
+  }
+}
+
+}  // namespace symla_gpu

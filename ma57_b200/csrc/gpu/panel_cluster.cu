@@ -11,6 +11,8 @@
 // Bunch-Kaufman decision (dense_kernel.hpp:576-793). Two cluster barriers per
 // pivot in the common (1x1 at k) case.
 //
+// (Static pivoting has its own kernel, panel_static.cu.)
+//
 // The front in global memory holds the panel-start ("raw") values of every
 // non-pivoted column; row/column interchanges are applied to it and to the
 // shared-memory copies. The near and far updates of the panel follow in
@@ -29,12 +31,17 @@
 // accepted (identical values and decisions to the sequential path), and
 // the same launch finishes the panel on the sequential path from the first
 // failing pivot (measured: cheaper than a new panel + update launch pair).
+// A 32-pivot panel of 4096 rows accepted whole takes 23 us (33 us when the
+// block was factored column by column and the rows went through shared memory
+// once more for the maxima and for L), of which the block's chain is 4.1, the
+// row pass 5.6, the exchange of the maxima 1.7, the stores of L 2.3 us.
 #include <cooperative_groups.h>
 
 #include <cmath>
 
 #include "common.cuh"
 #include "factor_kernels.h"
+#include "panel_block.cuh"
 #include "reduce.cuh"
 
 namespace cg = cooperative_groups;
@@ -46,7 +53,7 @@ namespace {
 constexpr double kAlphaBK = 0.64038820320220756;  // (1 + sqrt(17)) / 8
 constexpr int kCT = 256;                           // threads per CTA
 constexpr int kNBMax = 34;                         // panel width + 2
-constexpr int kSpecMax = 32;                       // pivots per speculative panel (= panel width)
+constexpr int kSpecMax = kPanelMax;                // pivots per speculative panel (= panel width)
 constexpr int kSpecRetry = 2;                      // consecutive failed panel starts before one sequential decision first
 constexpr int kStageHalf = (kNBMax / 2) * (kNBMax / 2 + 1);  // >= np * p0 of any restart (np + p0 <= kNBMax)
 
@@ -63,7 +70,6 @@ struct ClusterShared {
   double fx_v[2][16];
   int fx_i[2][16];
   double fx_kk[2];
-  int fx_sign[2];
   double fx_k1[2];
   double fx_row[2][kNBMax];
   double red_v[kCT / 32];
@@ -72,13 +78,9 @@ struct ClusterShared {
   double rowA[kNBMax], rowB[kNBMax];  // row interchange staging
   double vA[2], vB[2];
   // speculative panel
-  double db[kSpecMax][kSpecMax + 1];  // diagonal block: raw lower triangle -> L, d on the diagonal
-  double wv[kSpecMax][kSpecMax + 1];  // wv[c][t] = d_t * L(c, t), t < c
-  double aabs[kSpecMax][kSpecMax + 1];  // |current value| of the diagonal-block column entries
-  double dv[kSpecMax], iv[kSpecMax];  // pivots (after static perturbation) and 1 / pivot
-  double pv[kSpecMax];                // applied perturbation (static mode)
+  DiagBlock blk;  // the panel's diagonal block
   double lamd[kSpecMax], rmd[kSpecMax];  // diagonal-block rows: lambda part, running-max part
-  double lamw[kCT / 32][kSpecMax], rvw[kCT / 32][kSpecMax];  // per warp, rows below the block
+  unsigned long long lamw[kCT / 32][kSpecMax], rvw[kCT / 32][kSpecMax];  // the same of each warp's rows below it
   double lamx[16][kSpecMax];          // per CTA partial lambda (exchange)
   int kstar;                          // accepted speculative pivots
 };
@@ -118,17 +120,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// 8-byte asynchronous global -> shared copy (no register round trip, so
-// the copies of a staging loop are all in flight at once)
-__device__ __forceinline__ void cp_async8(double* smem_dst, const double* gsrc) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// wait until at most the newest group of this thread's copies is in flight
-__device__ __forceinline__ void cp_async_wait_but_newest() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
 }  // namespace
 
 template <int CS>
@@ -158,7 +149,8 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   }
   extern __shared__ __align__(16) double dsm[];
   __shared__ __align__(8) uint64_t rows_bar;  // bulk staging of the rows below the block
-  __shared__ ClusterShared sh;
+  __shared__ __align__(16) ClusterShared sh;
+  DiagBlock& blk = sh.blk;
   const int m = f.m, effEnd = f.nelig;
   const int64_t ld = f.ld;
   double* F = f.F;
@@ -199,25 +191,13 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   if (ps == 0) {
     // max |entry| of the assembled front, accumulated by the assembly kernel
     double om = S.orig_max;
-    if (o.mode == 1) {
-      if (om < o.static_abs_floor) om = 1.0;
-    } else {
-      if (om < o.zero_tol) om = 1.0;
-    }
+    if (om < o.zero_tol) om = 1.0;
     S.orig_max = om;
     S.running_max = om;
     S.n_pos = S.n_neg = S.n_zero = 0;
-    S.num_perturbed = 0;
-    S.perturb = 0.0;
-    S.delta = o.front_delta ? o.front_delta[s] : (o.static_delta > 0.0 ? o.static_delta : 1.4901161193847656e-08 * om);
   }
   const double orig_max = S.orig_max;
-  for (int t = threadIdx.x; t < (kCT / 32) * kSpecMax; t += kCT) {
-    sh.lamw[t / kSpecMax][t % kSpecMax] = 0.0;
-    sh.rvw[t / kSpecMax][t % kSpecMax] = 0.0;
-  }
-  int n_pos = S.n_pos, n_neg = S.n_neg, n_zero = S.n_zero, nPert = S.num_perturbed;
-  double pert = S.perturb;
+  int n_pos = S.n_pos, n_neg = S.n_neg, n_zero = S.n_zero;
   double thread_rmax = S.running_max;  // includes orig_max at the first panel
   double rm_known = S.running_max;
 
@@ -416,12 +396,13 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   bool first_spec = true, spec_tried = false, any_seq = false, any_accept = false;
   int restarts = 0;
   double* lblk = stage;               // restart: L of the block rows for the earlier pivots (np x p0)
-  double* wblk = stage + kStageHalf;  // restart: D L(block row, :)^T (np x p0)
+  double* wblk = stage + kStageHalf;  // restart: D L(block row, :)^T, a row of np (made even) per earlier pivot
   while (k < pe) {
     if (try_spec) {
       try_spec = false;
       spec_tried = true;
       const int k0 = k, p0 = k0 - ps, np = pe - k0;
+      const int np2 = (np + 1) & ~1;  // row stride of wblk
       const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
       const int r0 = max(base, pe);
       if (!first_spec) ++restarts;
@@ -433,15 +414,18 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
       // 16-byte pairs (the extra slot before r0 and after rend is spare)
       const int s0 = r0 & ~1, e0 = (rend + 1) & ~1;
       const bool have_rows = r0 < rend;
-      // static pivoting: expected sign of block row `lane`, loaded now so the
-      // diagonal-block chain below reads it from a register
-      const int lane_sign = (o.mode == 1 && o.sign_final && warp == 0 && lane < np) ? o.sign_final[f.fidx[k0 + lane]] : 0;
       if (warp == 0) {
-        for (int j = 0; j < np; ++j)
-          for (int i = j + lane; i < np; i += 32) cp_async8(&sh.db[i][j], F + static_cast<int64_t>(k0 + j) * ld + k0 + i);
-        cp_async_commit();
+        // all columns' loads first: they must not wait for one another's stores
+        double v[kSpecMax];
+#pragma unroll
+        for (int j = 0; j < kSpecMax; ++j)
+          v[j] = (lane >= j && lane < np) ? F[static_cast<int64_t>(k0 + j) * ld + k0 + lane] : 0.0;
+#pragma unroll
+        for (int j = 0; j < kSpecMax; ++j) blk.db[lane][j] = v[j];
+        __syncwarp();
       } else if (threadIdx.x == 32 && have_rows) {
         const uint32_t bytes = static_cast<uint32_t>(e0 - s0) * sizeof(double);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier runs' accesses to these columns
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&rows_bar)),
                      "r"(bytes * static_cast<uint32_t>(np))
                      : "memory");
@@ -471,257 +455,183 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
             v = sh.Dd[tt] * lr[tt] + sh.Do[tt] * lr[tt + 1];
           else
             v = sh.Do[tt - 1] * lr[tt - 1] + sh.Dd[tt] * lr[tt];
-          wblk[t] = v;
+          wblk[tt * np2 + t / p0] = v;
         }
       }
-      if (p0 > 0) __syncthreads();  // wblk complete before any warp reads it
-      if (warp == 0) {
-        cp_async_wait_all();
-        __syncwarp();
-        if (p0 > 0) {
-          // current values of the diagonal block: raw - L_blk W^T
-          for (int t = lane; t < np * np; t += 32) {
-            const int i = t / np, j = t % np;
-            if (j <= i) {
-              double acc = 0.0;
-              for (int tt = 0; tt < p0; ++tt) acc += lblk[i * p0 + tt] * wblk[j * p0 + tt];
-              sh.db[i][j] -= acc;
-            }
+      if (p0 > 0) {
+        // current values of the diagonal block: raw - L_blk W^T, by every warp
+        __syncthreads();  // the block is staged, wblk is complete
+        for (int t = threadIdx.x; t < np * np; t += kCT) {
+          const int i = t / np, j = t % np;
+          if (j <= i) {
+            double acc = 0.0;
+            for (int tt = 0; tt < p0; ++tt) acc += lblk[i * p0 + tt] * wblk[tt * np2 + j];
+            blk.db[i][j] -= acc;
           }
-          __syncwarp();
-        }
-      } else {
-        if (have_rows) {
-          if (!mbar_wait_bounded(&rows_bar, rows_phase)) {
-            atomicCAS(&g->error, 0, kPanelErrTimeout);
-            mbar_wait_bounded(&rows_bar, rows_phase);  // the copies must land before the CTA moves on
-          }
-        }
-        if (p0 > 0) {
-          // this warp's own staged rows: subtract the earlier pivots, L_row W^T
-          for (int c = 0; c < np; ++c)
-            for (int i = r0 + threadIdx.x - 32; i < rend; i += kCT - 32) {
-              const int li = i - base;
-              double acc = 0.0;
-              for (int tt = 0; tt < p0; ++tt) acc += Lr[tt * R + li] * wblk[c * p0 + tt];
-              Lr[(p0 + c) * R + li] -= acc;
-            }
-        }
-      }
-      if (have_rows) rows_phase ^= 1;  // every thread: the barrier's phase of this staging is consumed
-      // diagonal block, left-looking: warp 0 of every CTA, lane = row (the
-      // row lives in sh.db, conflict-free with the odd row stride). The sums
-      // use four partial accumulators to shorten the dependency chain; |a| of
-      // the column values go to shared memory and are reduced afterwards.
-      if (warp == 0) {
-        const double floorv = fmax(o.static_abs_floor, o.static_rel_floor * orig_max);
-        const int lr = lane < np ? lane : 0;
-        for (int c = 0; c < np; ++c) {
-          double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-          int t = 0;
-          for (; t + 4 <= c; t += 4) {
-            s0 = fma(sh.db[lr][t], sh.wv[c][t], s0);
-            s1 = fma(sh.db[lr][t + 1], sh.wv[c][t + 1], s1);
-            s2 = fma(sh.db[lr][t + 2], sh.wv[c][t + 2], s2);
-            s3 = fma(sh.db[lr][t + 3], sh.wv[c][t + 3], s3);
-          }
-          for (; t < c; ++t) s0 = fma(sh.db[lr][t], sh.wv[c][t], s0);
-          const double a = sh.db[lr][c] - ((s0 + s1) + (s2 + s3));
-          const double akk = __shfl_sync(0xffffffffu, a, c);
-          double d = akk, applied = 0.0;
-          if (o.mode == 1) {
-            // static pivoting (dense_kernel.hpp:982-1034), as in the sequential path
-            const int sign = __shfl_sync(0xffffffffu, lane_sign, c);
-            bool need;
-            if (sign > 0)
-              need = akk < floorv;
-            else if (sign < 0)
-              need = akk > -floorv;
-            else
-              need = fabs(akk) < floorv;
-            if (need) {
-              const double sg = (sign != 0) ? static_cast<double>(sign) : (akk >= 0.0 ? 1.0 : -1.0);
-              d = akk + sg * S.delta;
-              applied = d - akk;
-            }
-          }
-          const double inv = __drcp_rn(d);
-          __syncwarp();
-          if (lane > c && lane < np) {
-            const double l = a * inv;
-            sh.db[lane][c] = l;
-            sh.aabs[c][lane] = fabs(a);
-            sh.wv[lane][c] = d * l;
-          } else if (lane == c) {
-            sh.db[c][c] = d;
-          }
-          if (lane == 0) {
-            sh.dv[c] = d;
-            sh.iv[c] = inv;
-            sh.pv[c] = applied;
-          }
-          __syncwarp();
-        }
-      }
-      __syncthreads();
-      // lambda and running-max parts of the diagonal-block rows
-      if (threadIdx.x < np) {
-        const int c = threadIdx.x;
-        double lm = 0.0, rv = fabs(sh.dv[c]);
-        for (int i = c + 1; i < np; ++i) {
-          const double v = sh.aabs[c][i];
-          if (k0 + i < effEnd) lm = fmax(lm, v);
-          rv = fmax(rv, v);
-        }
-        sh.lamd[c] = lm;
-        sh.rmd[c] = rv;
-      }
-      // rows below the block, left-looking: the raw block columns of this
-      // CTA's rows are in Lr (staged above; a restart first subtracts the
-      // earlier pivots, L_row W^T), then each thread takes one row at a time
-      // into registers and walks it pivot by pivot, touching only its own
-      // rows, so no synchronisation is needed between pivots; the L(c, t) are
-      // warp-uniform (broadcast) shared loads. Lr receives the current values
-      // a_ic = raw_ic - sum_t a_it L_ct (L = a_ic / d_c on write-back). Columns
-      // past np compute unused values (column c depends on columns t < c only).
-      for (int i = r0 + threadIdx.x; i < rend; i += kCT) {
-        const int li = i - base;
-        double a[kSpecMax];
-#pragma unroll
-        for (int c = 0; c < kSpecMax; ++c) a[c] = (c < np) ? Lr[(p0 + c) * R + li] : 0.0;
-#pragma unroll
-        for (int c = 1; c < kSpecMax; ++c) {
-          // sum_t L_it d_t L_ct = sum_t a_it L_ct (a_it = L_it d_t): even and
-          // odd t in two partial sums
-          double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-          for (int t = 0; t < c; ++t) {
-            if (t & 1)
-              s1 = fma(a[t], sh.db[c][t], s1);
-            else
-              s0 = fma(a[t], sh.db[c][t], s0);
-          }
-          a[c] -= s0 + s1;
-          asm volatile("" ::: "memory");  // keep the next pivot's loads from being hoisted (registers)
-        }
-#pragma unroll
-        for (int c = 0; c < kSpecMax; ++c)
-          if (c < np) Lr[(p0 + c) * R + li] = a[c];
-      }
-      __syncthreads();
-      // per pivot and warp: lambda part (eligible rows) and running-max part
-      // (all rows) of this CTA's rows below the block
-      for (int c = warp; c < np; c += kCT / 32) {
-        double lm = 0.0, rv = 0.0;
-        for (int i = r0 + lane; i < rend; i += 32) {
-          const double v = fabs(Lr[(p0 + c) * R + (i - base)]);
-          if (i < effEnd) lm = fmax(lm, v);
-          rv = fmax(rv, v);
-        }
-        lm = warp_max_nonneg(lm);
-        rv = warp_max_nonneg(rv);
-        if (lane == 0) {
-          sh.lamw[0][c] = lm;
-          sh.rvw[0][c] = rv;
-        }
-      }
-      __syncthreads();
-      int kstar = np;
-      if (o.mode != 1) {
-        // lambda per pivot: this CTA's part to every CTA of the cluster
-        if (threadIdx.x < np) {
-          const double lc = sh.lamw[0][threadIdx.x];
-          for (int dd = 0; dd < CS; ++dd) *cluster.map_shared_rank(&sh.lamx[q][threadIdx.x], dd) = lc;
-        }
-        cluster.sync();
-        if (warp == 0) {
-          // the sequential path's 1x1-at-k decision (dense_kernel.hpp:576-600),
-          // one lane per pivot; the first failing pivot ends the accepted prefix
-          bool fail = false;
-          if (lane < np) {
-            const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
-            double lam = sh.lamd[lane];
-            for (int dd = 0; dd < CS; ++dd) lam = fmax(lam, sh.lamx[dd][lane]);
-            const double akk = sh.dv[lane];
-            const bool pass = (lam <= o.zero_tol) ? (fabs(akk) > isolatedFloor) : (fabs(akk) >= kAlphaBK * lam);
-            fail = !pass;
-          }
-          const unsigned bad = __ballot_sync(0xffffffffu, fail);
-          if (lane == 0) sh.kstar = bad ? __ffs(bad) - 1 : np;
         }
         __syncthreads();
-        kstar = sh.kstar;
       }
+      if (warp == 0) {
+        factor_diag_block<false>(blk, np, lane, 0, 0.0, 0.0);
+      } else if (have_rows && !mbar_wait_bounded(&rows_bar, rows_phase)) {
+        atomicCAS(&g->error, 0, kPanelErrTimeout);
+        mbar_wait_bounded(&rows_bar, rows_phase);  // the copies must land before the CTA moves on
+      }
+      if (have_rows) rows_phase ^= 1;  // every thread: the barrier's phase of this staging is consumed
+      __syncthreads();
+      // lambda and running-max parts of the diagonal-block rows: a warp takes
+      // a column at a time, lane = row
+      for (int c = warp; c < np; c += kCT / 32) {
+        const double v = (lane > c && lane < np) ? fabs(blk.wv[lane][c]) : 0.0;
+        const double lm = warp_max_nonneg(k0 + lane < effEnd ? v : 0.0);
+        const double rv = warp_max_nonneg(v);
+        if (lane == 0) {
+          sh.lamd[c] = lm;
+          sh.rmd[c] = fmax(rv, fabs(blk.dv[c]));
+        }
+      }
+      // rows below the block: the raw block columns of this CTA's rows are in
+      // Lr (staged above; a restart subtracts the earlier pivots, L_row W^T);
+      // each thread takes one row at a time into registers and eliminates it,
+      // touching no other row, so no synchronisation is needed between
+      // pivots. Lr receives L. The packed operands of the updates are written
+      // here, before the pivots are accepted, while the values are in
+      // registers (a column that is not accepted is written again when it
+      // is), and the columns' maxima taken.
+      const bool mixed_rows = r0 < effEnd && rend > effEnd;  // some rows eligible, some not
+      sh.lamw[warp][lane] = 0;
+      sh.rvw[warp][lane] = 0;
+      for (int b0 = r0; b0 < rend; b0 += kCT) {
+        const int i = b0 + static_cast<int>(threadIdx.x), li = i - base;
+        if (b0 + 32 * warp >= rend) break;  // the whole warp is past the rows
+        const bool row = i < rend;
+        double a[kSpecMax];
+#pragma unroll
+        for (int c = 0; c < kSpecMax; ++c) a[c] = (row && c < np) ? Lr[(p0 + c) * R + li] : 0.0;
+        for (int tt = 0; tt < p0; ++tt) {
+          const double l = row ? Lr[tt * R + li] : 0.0;
+          const double* w = wblk + tt * np2;
+#pragma unroll
+          for (int c = 0; c < kSpecMax; c += 2)
+            if (c < np) {
+              const double2 wc = *reinterpret_cast<const double2*>(w + c);
+              a[c] = fma(-l, wc.x, a[c]);
+              a[c + 1] = fma(-l, wc.y, a[c + 1]);
+            }
+        }
+        panel_row(blk, np, a);
+        if (row) {
+          double* out = Lr + p0 * R + li;
+          store_panel_row(blk, np, a, f.P, f.pw, f.prt, k0 - S.ob, i, [&](int c, double l) { out[c * R] = l; });
+        }
+        if (mixed_rows) {
+          const unsigned long long mx = warp_column_max(a, row && i < effEnd, np, lane);
+          sh.lamw[warp][lane] = max(sh.lamw[warp][lane], mx);
+        }
+        const unsigned long long mx = warp_column_max(a, row, np, lane);
+        sh.rvw[warp][lane] = max(sh.rvw[warp][lane], mx);
+      }
+      __syncthreads();
+      // per pivot: this CTA's lambda part (eligible rows) to every CTA, and
+      // its running-max part (all rows) into warp 0's slot
+      if (warp == 0) {
+        unsigned long long lm = 0, rv = 0;
+        for (int w = 0; w < kCT / 32; ++w) {
+          lm = max(lm, sh.lamw[w][lane]);
+          rv = max(rv, sh.rvw[w][lane]);
+        }
+        if (!mixed_rows) lm = r0 < effEnd ? rv : 0;
+        sh.lamw[0][lane] = lm;
+        sh.rvw[0][lane] = rv;
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < CS * kSpecMax; t += kCT)
+        *cluster.map_shared_rank(&sh.lamx[q][t % kSpecMax], t / kSpecMax) =
+            __longlong_as_double(static_cast<long long>(sh.lamw[0][t % kSpecMax]));
+      cluster.sync();
+      if (warp == 0) {
+        // the sequential path's 1x1-at-k decision (dense_kernel.hpp:576-600),
+        // one lane per pivot; the first failing pivot ends the accepted prefix
+        bool fail = false;
+        if (lane < np) {
+          const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
+          double lam = sh.lamd[lane];
+          for (int dd = 0; dd < CS; ++dd) lam = fmax(lam, sh.lamx[dd][lane]);
+          const double akk = blk.dv[lane];
+          const bool pass = (lam <= o.zero_tol) ? (fabs(akk) > isolatedFloor) : (fabs(akk) >= kAlphaBK * lam);
+          fail = !pass;
+        }
+        const unsigned bad = __ballot_sync(0xffffffffu, fail);
+        if (lane == 0) sh.kstar = bad ? __ffs(bad) - 1 : np;
+      }
+      __syncthreads();
+      const int kstar = sh.kstar;
       if (first_spec) spec_carry = kstar > 0 ? 0 : spec_carry + 1;
       first_spec = false;
       if (kstar > 0) {
         any_accept = true;
-        for (int c = 0; c < kstar; ++c) {
-          const double iv = sh.iv[c];
-          for (int i = r0 + threadIdx.x; i < rend; i += kCT) {
-            const double a = Lr[(p0 + c) * R + (i - base)];
-            F[static_cast<int64_t>(k0 + c) * ld + i] = a * iv;
-            put_packed(k0 + c, i, a * iv, a);
+        for (int i = r0 + threadIdx.x; i < rend; i += kCT) {
+          const double* l = Lr + p0 * R + (i - base);
+          double* out = F + static_cast<int64_t>(k0) * ld + i;
+          for (int c = 0; c < kstar; c += 8) {
+            double v[8];  // loads ahead of the stores
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = c + j < kstar ? l[(c + j) * R] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (c + j < kstar) out[static_cast<int64_t>(c + j) * ld] = v[j];
           }
         }
         if (q == 0) {
-          for (int c = 0; c < kstar; ++c)
-            for (int i = c + threadIdx.x; i < np; i += kCT) {
-              F[static_cast<int64_t>(k0 + c) * ld + k0 + i] = sh.db[i][c];
-              // block rows past the accepted pivots are rows of the updates
-              if (i >= kstar) put_packed(k0 + c, k0 + i, sh.db[i][c], sh.wv[i][c]);
-            }
+          for (int t = threadIdx.x; t < kstar * np; t += kCT) {
+            const int c = t / np, i = t % np;
+            if (i < c) continue;
+            F[static_cast<int64_t>(k0 + c) * ld + k0 + i] = blk.db[i][c];
+            // block rows past the accepted pivots are rows of the updates
+            if (i >= kstar) put_packed(k0 + c, k0 + i, blk.db[i][c], blk.wv[i][c]);
+          }
           for (int c = threadIdx.x; c < kstar; c += kCT) {
-            f.Dd[k0 + c] = sh.dv[c];
+            f.Dd[k0 + c] = blk.dv[c];
             f.Do[k0 + c] = 0.0;
             f.pk[k0 + c] = 0;
           }
         }
         // inertia of the accepted pivots (only thread 0's counters are
-        // written back): one ballot each over warp 0's lanes; the
-        // perturbations (static mode) are summed in pivot order
+        // written back): one ballot each over warp 0's lanes
         if (warp == 0) {
           const bool in = lane < kstar;
-          const double d = in ? sh.dv[lane] : 0.0;
+          const double d = in ? blk.dv[lane] : 0.0;
           const unsigned pos = __ballot_sync(0xffffffffu, in && d > 0);
           const unsigned neg = __ballot_sync(0xffffffffu, in && d < 0);
           const unsigned zer = __ballot_sync(0xffffffffu, in && !(d > 0) && !(d < 0));
-          const unsigned per = __ballot_sync(0xffffffffu, in && sh.pv[lane] != 0.0);
           if (lane == 0) {
             n_pos += __popc(pos);
             n_neg += __popc(neg);
             n_zero += __popc(zer);
-            if (per)
-              for (int c = 0; c < kstar; ++c)
-                if (sh.pv[c] != 0.0) {
-                  pert += fabs(sh.pv[c]);
-                  ++nPert;
-                }
           }
         }
         if (threadIdx.x < kstar) {
           // running max of the accepted columns (one thread per column)
-          thread_rmax = fmax(thread_rmax, fmax(sh.rmd[threadIdx.x], sh.rvw[0][threadIdx.x]));
+          thread_rmax = fmax(thread_rmax, fmax(sh.rmd[threadIdx.x],
+                                               __longlong_as_double(static_cast<long long>(sh.rvw[0][threadIdx.x]))));
         }
         k = k0 + kstar;
         if (k < pe) {
           // The sequential decision at k needs, for the accepted pivots: L
-          // of this CTA's rows in Lr (below the block: a / d as written to F;
-          // block rows: sh.db), D in sh.Dd/Do/pk, and w = D L(k, :)^T (the
-          // earlier pivots' part from wblk, the run's part from sh.wv).
+          // of this CTA's rows in Lr (there for the rows below the block;
+          // block rows: blk.db), D in sh.Dd/Do/pk, and w = D L(k, :)^T (the
+          // earlier pivots' part from wblk, the run's part from blk.wv).
           for (int c = 0; c < kstar; ++c) {
-            const double iv = sh.iv[c];
-            for (int i = r0 + threadIdx.x; i < rend; i += kCT) Lr[(p0 + c) * R + (i - base)] *= iv;
             for (int i = max(base, k0 + c + 1) + threadIdx.x; i < min(rend, pe); i += kCT)
-              Lr[(p0 + c) * R + (i - base)] = sh.db[i - k0][c];
+              Lr[(p0 + c) * R + (i - base)] = blk.db[i - k0][c];
           }
           if (threadIdx.x < kstar) {
-            sh.Dd[p0 + threadIdx.x] = sh.dv[threadIdx.x];
+            sh.Dd[p0 + threadIdx.x] = blk.dv[threadIdx.x];
             sh.Do[p0 + threadIdx.x] = 0.0;
             sh.pk[p0 + threadIdx.x] = 0;
-            sh.w[p0 + threadIdx.x] = sh.wv[kstar][threadIdx.x];
+            sh.w[p0 + threadIdx.x] = blk.wv[kstar][threadIdx.x];
           }
-          for (int t = threadIdx.x; t < p0; t += kCT) sh.w[t] = wblk[kstar * p0 + t];
+          for (int t = threadIdx.x; t < p0; t += kCT) sh.w[t] = wblk[t * np2 + kstar];
           __syncthreads();
         }
       }
@@ -736,11 +646,9 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     // fast-path exchange: partial argmax (threshold) and the values every
     // CTA needs to continue without a second barrier
     ArgMax am{0.0, -1};
-    if (o.mode != 1) {
-      for (int i = max(base, k + 1) + threadIdx.x; i < min(rend, effEnd); i += kCT)
-        am = argmax_combine(am, ArgMax{fabs(vk[i - base]), i});
-      am = block_argmax<kCT>(am, sh.red_v, sh.red_i);
-    }
+    for (int i = max(base, k + 1) + threadIdx.x; i < min(rend, effEnd); i += kCT)
+      am = argmax_combine(am, ArgMax{fabs(vk[i - base]), i});
+    am = block_argmax<kCT>(am, sh.red_v, sh.red_i);
     const bool haveNext = (k + 1 < pe) && (k + 1 < m);
     const int o1 = haveNext ? owner(k + 1) : -1;
     // one thread per destination CTA
@@ -748,10 +656,7 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
       const int dd = threadIdx.x;
       remote(sh.fx_v[b], dd)[q] = am.v;
       remote(sh.fx_i[b], dd)[q] = am.i;
-      if (q == owner(k)) {
-        remote(sh.fx_kk, dd)[b] = vk[k - base];
-        remote(sh.fx_sign, dd)[b] = (o.mode == 1 && o.sign_final) ? o.sign_final[f.fidx[k]] : 0;
-      }
+      if (q == owner(k)) remote(sh.fx_kk, dd)[b] = vk[k - base];
       if (q == o1) remote(sh.fx_k1, dd)[b] = vk[k + 1 - base];
     }
     if (q == o1)
@@ -763,35 +668,6 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     // global stores of this step are not read by other CTAs in this launch
     cluster.sync();
     const double akk = sh.fx_kk[b];
-
-    if (o.mode == 1) {
-      // static pivoting (dense_kernel.hpp:982-1034), decided by every CTA
-      const int sign = sh.fx_sign[b];
-      const double floorv = fmax(o.static_abs_floor, o.static_rel_floor * orig_max);
-      bool need;
-      if (sign > 0)
-        need = akk < floorv;
-      else if (sign < 0)
-        need = akk > -floorv;
-      else
-        need = fabs(akk) < floorv;
-      double d = akk;
-      if (need) {
-        const double sg = (sign != 0) ? static_cast<double>(sign) : (akk >= 0.0 ? 1.0 : -1.0);
-        d = akk + sg * S.delta;
-        const double applied = d - akk;
-        if (applied != 0.0) {
-          pert += fabs(applied);
-          ++nPert;
-        }
-      }
-      finish_1x1(p, d, vk);
-      if (haveNext) local_w_next(p, d, sh.fx_row[b], sh.fx_k1[b]);
-      __syncthreads();
-      ++k;
-      try_spec = true;
-      continue;
-    }
 
     ArgMax gm{sh.fx_v[b][0], sh.fx_i[b][0]};
     for (int dd = 1; dd < CS; ++dd) gm = argmax_combine(gm, ArgMax{sh.fx_v[b][dd], sh.fx_i[b][dd]});
@@ -959,12 +835,12 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
   if (q == 0 && threadIdx.x == 0) {
     FrontState& W = st[s];
     W.orig_max = orig_max;
-    W.delta = S.delta;
+    W.delta = 0.0;
     W.n_pos = n_pos;
     W.n_neg = n_neg;
     W.n_zero = n_zero;
-    W.num_perturbed = nPert;
-    W.perturb = pert;
+    W.num_perturbed = 0;
+    W.perturb = 0.0;
     W.panel_start = ps;
     W.k = k;
     W.npiv = k;

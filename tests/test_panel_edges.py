@@ -1,0 +1,80 @@
+"""Panels of large fronts (one dense front, natural order). Static pivoting at
+the edges of the 32-pivot panels, the 96-row CTAs and the 256-pivot outer
+blocks, against the CPU oracle: inertia, perturbed pivots and residual.
+Threshold pivoting beyond the single-CTA panel's sizes."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from ma57_b200 import Mode, OrderingType, SymLDLT
+from ma57_b200.matrices import Stream, lower
+from oracle.pyoracle import OracleSymLDLT
+
+
+def quasi_definite(n, n1, weak):
+    """Dense [[-E, A^T], [A, F]] of n1 + (n - n1), rows interleaved; `weak`
+    diagonal entries have the wrong sign and are perturbed."""
+    st = Stream(1000 * n + n1)
+    G = st.normal(n * n).reshape(n, n) / np.sqrt(n)
+    K = G @ G.T + np.eye(n)
+    sign = np.where((np.arange(n) * n1) % n < n1, -1, 1)
+    S = np.outer(sign, sign)
+    K = np.where(S > 0, K * sign[:, None], (G + G.T) / 4)
+    for i in range(weak):
+        j = (i * 37 + 5) % n
+        K[j, j] = -1e-3 * sign[j]
+    return K, sign
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [129, 160, 161, 225, 256, 257, 289, 545, 801])
+@pytest.mark.parametrize("weak", [0, 3])
+def test_static_dense_front(n, weak):
+    K, sign = quasi_definite(n, n // 3, weak)
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setMode(Mode.StaticRegularized)
+    s.setOrdering(OrderingType.Natural)
+    s.setExpectedSignPattern(sign)
+    s.setStaticPivotFloor(1e-8)
+    s.setInitialRegularizationDelta(10.0)
+    s.analyzePattern(A)
+    s.factorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.setExpectedSignPattern(sign)
+    o.set(mode=1, initial_delta=10.0)
+    o.factorize(A)
+    assert s.inertia().as_tuple() == o.inertia()
+    assert s.numPerturbedPivots() == o.info()["num_perturbed"] >= weak
+    assert abs(s.totalPerturbation() - o.info()["total_perturbation"]) <= 1e-9 * max(1.0, s.totalPerturbation())
+    if weak == 0:
+        X = st = Stream(n).normal(2 * n).reshape(2, n).T
+        B = np.asfortranarray(K @ X)
+        R = K @ s.solve(B) - B
+        bw = np.abs(R).max() / (np.abs(K).sum(axis=1).max() * np.abs(X).max() + np.abs(B).max())
+        assert bw < 100 * n * 2.0 ** -53  # backward stable on a quasi-definite matrix
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1025, 1057, 1288])
+def test_threshold_dense_front(n):
+    """The cluster panel on a front whose pivots need interchanges and 2x2
+    blocks (runs that stop inside a panel and start again): inertia from the
+    eigenvalues, backward error of a solve."""
+    st = Stream(n)
+    G = st.normal(n * n).reshape(n, n)
+    K = (G + G.T) / 2
+    K[np.arange(0, n, 3), np.arange(0, n, 3)] += 3 * np.sqrt(n)
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    A = lower(sp.csc_matrix(K))
+    s.analyzePattern(A)
+    s.factorize(A)
+    w = np.linalg.eigvalsh(K)
+    assert np.abs(w).min() > 1e-9 * np.abs(w).max()
+    assert s.inertia().as_tuple() == (int((w > 0).sum()), int((w < 0).sum()), 0)
+    x = Stream(n + 1).normal(n)
+    b = K @ x
+    r = K @ s.solve(b) - b
+    # Bunch-Kaufman growth on a random matrix is far below the 1e3 allowed here
+    assert np.abs(r).max() < 1e3 * n * 2.0 ** -53 * np.abs(K).sum(axis=1).max() * np.abs(x).max()
