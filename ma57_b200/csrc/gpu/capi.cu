@@ -397,13 +397,10 @@ void free_level_device(LevelLists& L) {
   dfree(L.d_tasks);
   dfree(L.d_touch);
   dfree(L.d_all);
-  dfree(L.d_fwd_tasks);
-  dfree(L.d_bwd_tasks);
   dfree(L.d_tcmaps);
   dfree(L.d_tcws);
   L.d_small = L.d_large = L.d_touch = L.d_all = nullptr;
   L.d_tasks = nullptr;
-  L.d_fwd_tasks = L.d_bwd_tasks = nullptr;
   L.d_tcmaps = nullptr;
   L.d_tcws = nullptr;
   L.tc_grid = 0;
@@ -1433,73 +1430,133 @@ void ensure_workspace(symla_gpu_ctx* c, int nrhs) {
   c->w_dirty = false;
 }
 
+// Right-hand-side groups (of solve_rhs_chunk()) solved side by side at most.
+constexpr int kSolveChunks = 4;
+
 // (Re)build the pipelined solve task lists when the fronts' sizes or pivot
-// counts differ from the ones the lists were built for.
-void ensure_solve_tasks(symla_gpu_ctx* c) {
+// counts differ from the ones the lists were built for, and size what every
+// right-hand-side group has of its own for nchunks groups.
+void ensure_solve_tasks(symla_gpu_ctx* c, int nchunks) {
+  SolvePlan& p = c->splan;
   std::vector<int> np(c->numSN);
   for (int s = 0; s < c->numSN; ++s) np[s] = c->hstate[s].npiv;
-  bool same = (np == c->solve_np) && c->d_flags != nullptr && !c->w_dirty;
-  if (same) return;
-  const int RB = solve_block_rows();
-  std::vector<int> fbase(c->numSN);
-  int total = 0;
-  for (int s = 0; s < c->numSN; ++s) {
-    fbase[s] = total;
-    total += (c->hdesc[s].m + RB - 1) / RB;
-  }
-  if (total > c->flag_count || !c->d_flags) {
-    dfree(c->d_flags);
-    c->d_flags = dalloc<int>(std::max(1, total));
-    CK(cudaMemsetAsync(c->d_flags, 0, std::max(1, total) * sizeof(int), c->stream));
-    c->flag_count = total;
-    c->solve_epoch = 0;
-  }
-  dfree(c->d_flag_base);
-  c->d_flag_base = dupload(fbase, c->stream);
-  // Task shapes per level. Forward: one row block per task (the non-pivot
-  // row blocks of a front run concurrently). Backward: with many fronts (at
-  // least two per resident CTA) a small front is one task, whose blocks run
-  // in order in one CTA with no waits on other CTAs; otherwise a task is one
-  // block, and a block with many ancestor-row chunks is split into parts
-  // (helpers first) so that one CTA does not walk all of them.
-  int slots = 0;
-  for (auto& L : c->levels) {
-    L.fwd_tasks.clear();
-    L.bwd_tasks.clear();
-    const bool whole = static_cast<int>(L.all.size()) >= 2 * std::min(c->fwd_resident, c->bwd_resident);
-    for (int s : L.all) {
-      const int m = c->hdesc[s].m;
-      const int nbp = (np[s] + RB - 1) / RB;
-      for (int rb = 0; rb * RB < m; ++rb) L.fwd_tasks.push_back(make_int4(s, rb, 0, 0));
-      if (whole && m <= 8 * RB) {
-        if (nbp > 0) L.bwd_tasks.push_back(make_int4(s, -1, 0, 0));
-        continue;
-      }
-      const int nanc = (m - np[s] + RB - 1) / RB;
-      const int P = std::max(1, std::min(8, nanc / 4));
-      for (int cb = nbp - 1; cb >= 0; --cb) {
-        const int h0 = slots;
-        for (int p = 1; p < P; ++p) L.bwd_tasks.push_back(make_int4(s, cb, p, (P << 20) | (h0 + p - 1)));
-        L.bwd_tasks.push_back(make_int4(s, cb, 0, (P << 20) | h0));
-        slots += P - 1;
-      }
+  const bool same = (np == c->solve_np) && c->d_fwd_tasks != nullptr && !c->w_dirty;
+  if (!same) {
+    const int RB = solve_block_rows(), tiny_rows = solve_tiny_rows();
+    std::vector<int4> fwd, bwd;
+    std::vector<int> tables(4 * static_cast<size_t>(c->numSN));
+    int* fbase = tables.data();
+    int* fneed = fbase + c->numSN;
+    int* bwait = fneed + c->numSN;
+    int* bneed = bwait + c->numSN;
+    std::vector<int> tiny;
+    auto is_tiny = [&](int s) { return c->hdesc[s].m <= tiny_rows; };
+    auto pivot_blocks = [&](int s) { return (np[s] + RB - 1) / RB; };
+    int total = 0;
+    for (int s = 0; s < c->numSN; ++s) {
+      fbase[s] = total;
+      total += (c->hdesc[s].m + RB - 1) / RB;
+      fneed[s] = 0;
+      for (int ch : c->fronts[s].children) fneed[s] += is_tiny(ch) ? 1 : (c->hdesc[ch].m + RB - 1) / RB;
     }
-    dfree(L.d_fwd_tasks);
-    dfree(L.d_bwd_tasks);
-    L.d_fwd_tasks = dupload(L.fwd_tasks, c->stream);
-    L.d_bwd_tasks = dupload(L.bwd_tasks, c->stream);
+    for (int s = c->numSN - 1; s >= 0; --s) {  // parents have larger indices
+      const int a = c->fronts[s].parent;
+      bwait[s] = a < 0 ? -1 : (np[a] > 0 ? a : bwait[a]);
+      bneed[s] = bwait[s] < 0 ? 0 : (is_tiny(bwait[s]) ? 1 : pivot_blocks(bwait[s]));
+    }
+    // Task shapes per level. Fronts of at most tiny_rows rows: eight to a
+    // task. Others forward: one row block per task (the non-pivot row blocks
+    // of a front run concurrently). Backward: with many fronts (at least two
+    // per resident CTA) a small front is one task, whose blocks run in order
+    // in one CTA with no waits on other CTAs; otherwise a task is one block,
+    // and a block with many ancestor-row chunks is split into parts (helpers
+    // first) so that one CTA does not walk all of them.
+    int slots = 0;
+    for (auto& L : c->levels) {
+      L.fwd_task0 = static_cast<int>(fwd.size());
+      int run = 0;
+      const int first = static_cast<int>(tiny.size());
+      for (int s : L.all)
+        if (is_tiny(s)) {
+          if (run % 8 == 0) fwd.push_back(make_int4(first + run, -2, 0, 0));
+          ++fwd.back().z;
+          ++run;
+          tiny.push_back(s);
+        }
+      for (int s : L.all)
+        if (!is_tiny(s))
+          for (int rb = 0; rb * RB < c->hdesc[s].m; ++rb) fwd.push_back(make_int4(s, rb, 0, 0));
+      L.fwd_ntasks = static_cast<int>(fwd.size()) - L.fwd_task0;
+    }
+    for (int l = c->numLevels - 1; l >= 0; --l) {
+      auto& L = c->levels[l];
+      L.bwd_task0 = static_cast<int>(bwd.size());
+      for (int t = L.fwd_task0; t < L.fwd_task0 + L.fwd_ntasks && fwd[t].y == -2; ++t) bwd.push_back(fwd[t]);
+      const bool whole = static_cast<int>(L.all.size()) >= 2 * std::min(c->fwd_resident, c->bwd_resident);
+      for (int s : L.all) {
+        if (is_tiny(s)) continue;
+        const int m = c->hdesc[s].m, nbp = pivot_blocks(s);
+        if (whole && m <= 8 * RB) {
+          if (nbp > 0) bwd.push_back(make_int4(s, -1, 0, 0));
+          continue;
+        }
+        const int P = std::max(1, std::min(8, solve_ancestor_chunks(m, np[s]) / 4));
+        for (int cb = nbp - 1; cb >= 0; --cb) {
+          const int h0 = slots;
+          for (int q = 1; q < P; ++q) bwd.push_back(make_int4(s, cb, q, (P << 20) | (h0 + q - 1)));
+          bwd.push_back(make_int4(s, cb, 0, (P << 20) | h0));
+          slots += P - 1;
+        }
+      }
+      L.bwd_ntasks = static_cast<int>(bwd.size()) - L.bwd_task0;
+    }
+    dfree(c->d_fwd_tasks);
+    dfree(c->d_bwd_tasks);
+    dfree(c->d_stables);
+    c->d_fwd_tasks = c->d_bwd_tasks = nullptr;
+    c->d_stables = nullptr;
+    c->fwd_ntasks = static_cast<int>(fwd.size());
+    c->bwd_ntasks = static_cast<int>(bwd.size());
+    tables.insert(tables.end(), tiny.begin(), tiny.end());
+    c->d_bwd_tasks = dupload(bwd, c->stream);
+    c->d_stables = dupload(tables, c->stream);
+    c->d_fwd_tasks = dupload(fwd, c->stream);
+    CK(cudaStreamSynchronize(c->stream));
+    p.fwd_tasks = c->d_fwd_tasks;
+    p.bwd_tasks = c->d_bwd_tasks;
+    p.flag_base = c->d_stables;
+    p.fwd_need = p.flag_base + c->numSN;
+    p.bwd_wait = p.fwd_need + c->numSN;
+    p.bwd_need = p.bwd_wait + c->numSN;
+    p.tiny = p.bwd_need + c->numSN;
+    p.nflags = total;
+    p.nfronts = c->numSN;
+    p.nslots = slots;
+    c->solve_np = np;
+    c->solve_chunks = 0;  // the per-group state is sized anew
   }
-  if (slots > c->hslot_count || !c->d_hflags) {
+  if (nchunks > c->solve_chunks) {
+    dfree(c->d_flags);
+    dfree(c->d_counters);
     dfree(c->d_hflags);
     dfree(c->d_hscratch);
-    c->d_hflags = dalloc<int>(std::max(1, slots));
-    CK(cudaMemsetAsync(c->d_hflags, 0, std::max(1, slots) * sizeof(int), c->stream));
-    c->d_hscratch = dalloc<double>(static_cast<size_t>(std::max(1, slots)) * RB * solve_rhs_chunk());
-    c->hslot_count = std::max(1, slots);
-    c->solve_epoch = std::max(c->solve_epoch, 0);
+    c->d_flags = c->d_counters = c->d_hflags = nullptr;
+    c->d_hscratch = nullptr;
+    c->solve_chunks = 0;
+    const size_t nf = static_cast<size_t>(nchunks) * std::max(1, p.nflags);
+    const size_t nh = static_cast<size_t>(nchunks) * std::max(1, p.nslots);
+    c->d_flags = dalloc<int>(nf);
+    c->d_hflags = dalloc<int>(nh);
+    c->d_hscratch = dalloc<double>(nh * solve_block_rows() * solve_rhs_chunk());
+    c->d_counters = dalloc<int>(2 * static_cast<size_t>(nchunks) * std::max(1, c->numSN));
+    CK(cudaMemsetAsync(c->d_flags, 0, nf * sizeof(int), c->stream));
+    CK(cudaMemsetAsync(c->d_hflags, 0, nh * sizeof(int), c->stream));
+    c->solve_epoch = 0;
+    p.flags = c->d_flags;
+    p.hflags = c->d_hflags;
+    p.hscratch = c->d_hscratch;
+    c->solve_chunks = nchunks;
   }
-  c->solve_np = np;
-  CK(cudaStreamSynchronize(c->stream));
 }
 
 // X := A^{-1} B for device B (ldb) into device X (ldx), both in the
@@ -1508,7 +1565,8 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
   cudaStream_t st = c->stream;
   ensure_vectors(c, nrhs);
   ensure_workspace(c, nrhs);
-  ensure_solve_tasks(c);
+  const int chunk = solve_rhs_chunk();
+  ensure_solve_tasks(c, std::min(kSolveChunks, (nrhs + chunk - 1) / chunk));
   if constexpr (kCheckedBuild) {
     KernelOpts ko;
     std::memset(&ko, 0, sizeof ko);
@@ -1522,32 +1580,48 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
   const int n = c->n;
   launch_permute_in(n, nrhs, c->d_perm, dB, ldb, c->d_Bp, st, c->d_check);
   CK(cudaEventRecord(c->ev[2], st));
-  const int chunk = solve_rhs_chunk();
-  for (int c0 = 0; c0 < nrhs; c0 += chunk) {
-    const int nc = std::min(chunk, nrhs - c0);
+  for (int c0 = 0; c0 < nrhs; c0 += kSolveChunks * chunk) {
+    const int nc = std::min(kSolveChunks * chunk, nrhs - c0), groups = (nc + chunk - 1) / chunk;
+    CK(cudaMemsetAsync(c->d_counters, 0, 2 * static_cast<size_t>(groups) * c->numSN * sizeof(int), st));
+    // every level in one launch, or (profiling) a launch per level
+    SolvePlan p = c->splan;
+    p.counters = c->d_counters;
     const int ef = ++c->solve_epoch;
-    for (int l = 0; l < c->numLevels; ++l) {
-      const auto& L = c->levels[l];
-      const int nt = static_cast<int>(L.fwd_tasks.size());
-      const int grid = std::min(nt, c->fwd_resident);
-      c->cur_level = l;
-      timed(c, SYMLA_KERNEL_FORWARD, 0.0, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs, [&] {
-        CK(launch_forward_pipelined(c->d_desc, c->d_links, c->d_state, L.d_fwd_tasks, nt, grid, c->d_flag_base,
-                                    c->d_flags, ef, c->d_solve_err, c->wait_ns, nrhs, c0, c->d_Bp, n, st));
+    auto forward = [&](int level, int task0, int ntasks, double bytes) {
+      c->cur_level = level;
+      timed(c, SYMLA_KERNEL_FORWARD, 0.0, bytes, [&] {
+        CK(launch_forward_pipelined(c->d_desc, c->d_links, c->d_state, p, task0, ntasks, groups,
+                                    static_cast<int>(std::min<long long>(static_cast<long long>(ntasks) * groups,
+                                                                         c->fwd_resident)),
+                                    ef, c->d_solve_err, c->wait_ns, nrhs, c0, c->d_Bp, n, st));
       });
-    }
+    };
+    auto backward = [&](int level, int eb, int task0, int ntasks, double bytes) {
+      c->cur_level = level;
+      timed(c, SYMLA_KERNEL_BACKWARD, 0.0, bytes, [&] {
+        CK(launch_backward_pipelined(c->d_desc, c->d_state, p, task0, ntasks, groups,
+                                     static_cast<int>(std::min<long long>(static_cast<long long>(ntasks) * groups,
+                                                                          c->bwd_resident)),
+                                     eb, c->d_solve_err, c->wait_ns, nrhs, c0, c->d_Xf, n, st));
+      });
+    };
+    if (c->profiling)
+      for (int l = 0; l < c->numLevels; ++l) {
+        const auto& L = c->levels[l];
+        forward(l, L.fwd_task0, L.fwd_ntasks, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs);
+      }
+    else
+      forward(-1, 0, c->fwd_ntasks, 0.0);
     if (c0 == 0) CK(cudaEventRecord(c->ev[3], st));
+    p.counters = c->d_counters + static_cast<size_t>(groups) * c->numSN;
     const int eb = ++c->solve_epoch;
-    for (int l = c->numLevels - 1; l >= 0; --l) {
-      const auto& L = c->levels[l];
-      const int nt = static_cast<int>(L.bwd_tasks.size());
-      const int grid = std::min(nt, c->bwd_resident);
-      c->cur_level = l;
-      timed(c, SYMLA_KERNEL_BACKWARD, 0.0, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs, [&] {
-        CK(launch_backward_pipelined(c->d_desc, c->d_state, L.d_bwd_tasks, nt, grid, c->d_flag_base, c->d_flags,
-                                     c->d_hflags, c->d_hscratch, eb, c->d_solve_err, c->wait_ns, nrhs, c0, c->d_Xf, n, st));
-      });
-    }
+    if (c->profiling)
+      for (int l = c->numLevels - 1; l >= 0; --l) {
+        const auto& L = c->levels[l];
+        backward(l, eb, L.bwd_task0, L.bwd_ntasks, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs);
+      }
+    else
+      backward(-1, eb, 0, c->bwd_ntasks, 0.0);
   }
   c->cur_level = -1;
   CK(cudaEventRecord(c->ev[4], st));
@@ -1708,7 +1782,7 @@ extern "C" void symla_gpu_destroy(symla_gpu_ctx* c) {
                   c->d_glob, c->d_a_colptr, c->d_a_j, c->d_a_pos, c->d_a_idx, c->d_values, c->d_sign_final,
                   c->d_front_delta, c->d_perm, c->d_rowptr, c->d_colind, c->d_vidx, c->d_srowptr, c->d_svidx, c->d_W,
                   c->d_Bp, c->d_Z, c->d_Xf, c->d_B, c->d_X, c->d_R, c->d_dX, c->d_Xn, c->d_Rn, c->d_norms,
-                  c->d_scratch_int, c->d_flag_base, c->d_flags, c->d_solve_err, c->d_counter,
+                  c->d_scratch_int, c->d_fwd_tasks, c->d_bwd_tasks, c->d_stables, c->d_flags, c->d_counters, c->d_solve_err, c->d_counter,
                   c->d_tcws, c->d_tc_err, c->d_tc_guard, c->d_hflags, c->d_hscratch,
                   c->d_gmres, c->d_zero, c->d_gpart, c->d_gcoef, c->d_check, c->d_ranges, c->d_packed};
   for (void* p : ptrs) dfree(p);

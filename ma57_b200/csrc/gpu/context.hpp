@@ -53,10 +53,8 @@ struct LevelLists {
   std::vector<double> trailing_flops;  // per panel iteration
   double solve_bytes_fixed = 0.0;
   double solve_bytes_per_rhs = 0.0;
-  // pipelined solve tasks {front, block}
-  std::vector<int4> fwd_tasks, bwd_tasks;
-  int4* d_fwd_tasks = nullptr;
-  int4* d_bwd_tasks = nullptr;
+  // the level's range of the solve's task lists
+  int fwd_task0 = 0, fwd_ntasks = 0, bwd_task0 = 0, bwd_ntasks = 0;
   // device copies (static plan)
   int* d_small = nullptr;
   int* d_large = nullptr;
@@ -155,12 +153,17 @@ struct symla_gpu_ctx {
   size_t scratch_int_cap = 0;
 
   // pipelined solve
-  int* d_flag_base = nullptr;
+  symla_gpu::SolvePlan splan{};   // task lists and their per-group state, see solve_kernels.cu
+  int4* d_fwd_tasks = nullptr;
+  int4* d_bwd_tasks = nullptr;
+  int* d_stables = nullptr;       // tiny list and the per-front tables
+  int fwd_ntasks = 0, bwd_ntasks = 0;
   int* d_flags = nullptr;
-  int* d_solve_err = nullptr;
+  int* d_counters = nullptr;      // forward, then backward
   int* d_hflags = nullptr;        // backward helper-part flags (one per slot)
   double* d_hscratch = nullptr;   // backward helper-part partial sums
-  int hslot_count = 0;
+  int solve_chunks = 0;           // right-hand-side groups the flags, counters and slots are sized for
+  int* d_solve_err = nullptr;
   int* d_counter = nullptr;  // unfinished-front counter
   int solve_epoch = 0;
   int fwd_resident = 0, bwd_resident = 0;

@@ -105,21 +105,40 @@ void launch_permute_in(int n, int nrhs, const int* perm, const double* B, int ld
                        CheckWord* chk = nullptr);
 void launch_permute_out(int n, int nrhs, const int* perm, const double* X, double* Xout, int ldx, cudaStream_t stream,
                         CheckWord* chk = nullptr);
-// Pipelined level solves (one cooperative launch per level; see
-// solve_kernels.cu). tasks: int4 (see the kernels); flags indexed by
-// flag_base[front] + block, compared against epoch; every wait on another
-// CTA's flag gives up after wait_ns of the global timer (error word set).
+// Pipelined solves (one cooperative launch each way; see solve_kernels.cu).
+// Flags are indexed by flag_base[front] + block and compared against epoch,
+// counters by front (zero at the start of a launch); groups of
+// solve_rhs_chunk() right-hand sides side by side have their own of both
+// (strides nflags, nfronts) and of the helper slots (nslots). Every wait on
+// another CTA gives up after wait_ns of the global timer (error word set).
+struct SolvePlan {
+  const int4* fwd_tasks;
+  const int4* bwd_tasks;
+  const int* tiny;      // fronts of the warp-per-front tasks
+  const int* flag_base;
+  const int* fwd_need;  // per front: tasks of its children
+  const int* bwd_wait;  // per front: nearest ancestor with pivots, or -1
+  const int* bwd_need;  // and that ancestor's tasks
+  int* flags;
+  int* counters;
+  int* hflags;
+  double* hscratch;
+  int nflags, nfronts, nslots;
+};
 int solve_block_rows();
 int solve_rhs_chunk();
+int solve_tiny_rows();
+int solve_ancestor_chunks(int m, int np);
 cudaError_t solve_max_resident(int device, int* fwd_ctas, int* bwd_ctas);
+// tasks [task0, task0 + ntasks) for nchunks groups of right-hand sides from c0
 cudaError_t launch_forward_pipelined(const FrontDesc* fronts, const ChildLink* links, const FrontState* st,
-                                     const int4* tasks, int ntasks, int grid, const int* flag_base, int* flags,
-                                     int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0,
-                                     const double* Bp, int n, cudaStream_t stream);
-cudaError_t launch_backward_pipelined(const FrontDesc* fronts, const FrontState* st, const int4* tasks, int ntasks,
-                                      int grid, const int* flag_base, int* flags, int* hflags, double* hscratch,
-                                      int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0, double* X,
-                                      int n, cudaStream_t stream);
+                                     const SolvePlan& p, int task0, int ntasks, int nchunks, int grid, int epoch,
+                                     int* err, unsigned long long wait_ns, int nrhs, int c0, const double* Bp, int n,
+                                     cudaStream_t stream);
+cudaError_t launch_backward_pipelined(const FrontDesc* fronts, const FrontState* st, const SolvePlan& p, int task0,
+                                      int ntasks, int nchunks, int grid, int epoch, int* err,
+                                      unsigned long long wait_ns, int nrhs, int c0, double* X, int n,
+                                      cudaStream_t stream);
 
 // Residual R = B - sym(A) X in the original index space (full symmetric CSR
 // gathered from the stored lower triangle); rowptr/colind/vidx describe it.

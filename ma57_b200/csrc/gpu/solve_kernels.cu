@@ -13,15 +13,27 @@
 //   refine.hpp:116     R = B - A.selfadjointView<Lower>() * X
 //
 // Work decomposition: every front is cut into 64-row blocks (forward) or
-// 64-column blocks of its pivot range (backward). One cooperative launch per
-// tree level runs all blocks of all fronts of that level; a block that needs
-// the solution of an earlier block of the same front waits for that block's
-// flag (release/acquire), so the triangular solve of a large front is
-// pipelined across many SMs instead of running in one CTA. Each CTA walks its
-// blocks in increasing task order and a block only waits on blocks with a
-// smaller task index, and the launch is cooperative (all CTAs resident), so
-// the waits always end; every wait is still bounded and reports a timeout
-// through the error word instead of spinning forever.
+// 64-column blocks of its pivot range (backward); fronts of at most 32 rows
+// are taken whole by one warp, eight to a task. One cooperative launch runs
+// the tasks of all tree levels, for up to four groups of 16 right-hand sides
+// side by side. A block that needs the solution of an earlier block of the
+// same front waits for that block's flag (release/acquire), so the triangular
+// solve of a large front is pipelined across many SMs instead of running in
+// one CTA; a front waits for its children (forward) or its nearest ancestor
+// with pivots (backward) on a counter that their tasks raise. Each CTA walks
+// its tasks in increasing order and a task only waits on tasks with a smaller
+// index, and the launch is cooperative (all CTAs resident), so the waits
+// always end; every wait is still bounded and reports a timeout through the
+// error word instead of spinning forever.
+//
+// What bounds it: the chain of a top front's blocks (flag, right-hand sides
+// from L2, one tile product, the diagonal block's substitution, store, flag),
+// and below the top the latency of a task's dependent loads. A launch
+// per level, one warp's worth of work per 256-thread CTA for tiny fronts, the
+// groups one after another and scalar tile products took 1.93 ms for one
+// right-hand side on a 40^3 27-point grid and 10.6 ms for 37 on 48^3; now 1.23
+// and 4.7 ms. A top front's block takes 7.2 us of its chain with 16
+// right-hand sides, 9.6 before.
 //
 // Sign convention: a front's workspace rows for its own pivots hold y after
 // the forward pass; its remaining rows hold the negated forwarded delta
@@ -56,42 +68,38 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Wait until flags[idx] >= epoch; false once wait_ns of the global timer or
-// wait_ns / 64 unsuccessful probes (each sleeps 64 ns) have passed (the
-// timeout is recorded in the error word), or another CTA raised an error.
-__device__ bool wait_flag(const int* flags, int idx, int epoch, int* err, unsigned long long wait_ns) {
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    if (ld_acquire(flags + idx) < epoch) {
-      const unsigned long long t0 = global_ns();
-      const unsigned long long max_probes = wait_ns / 64;
-      for (unsigned long long it = 1; ld_acquire(flags + idx) < epoch; ++it) {
-        if (ld_acquire(err) != 0) {
-          ok = 0;
-          break;
-        }
-        if (it > max_probes || global_ns() - t0 > wait_ns) {
-          atomicCAS(err, 0, kSolveErrTimeout);
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
-      }
+// Wait until *p >= target; false once wait_ns of the global timer or
+// wait_ns / 32 unsuccessful probes have passed (the timeout is recorded in
+// the error word), or another CTA raised an error. One thread.
+__device__ __forceinline__ bool wait_ge(const int* p, int target, int* err, unsigned long long wait_ns) {
+  if (ld_acquire(p) >= target) return true;
+  const unsigned long long t0 = global_ns();
+  const unsigned long long max_probes = wait_ns / 32;
+  for (unsigned long long it = 1; ld_acquire(p) < target; ++it) {
+    if ((it & 15) == 0 && ld_acquire(err) != 0) return false;
+    if (it > max_probes || global_ns() - t0 > wait_ns) {
+      atomicCAS(err, 0, kSolveErrTimeout);
+      return false;
     }
-    s_ok = ok;
+    __nanosleep(32);
   }
-  __syncthreads();
-  const bool ok = s_ok != 0;
-  __syncthreads();
-  return ok;
+  return true;
 }
 
-__device__ __forceinline__ void publish(int* flags, int idx, int epoch) {
+// The same for the whole CTA (a block barrier).
+__device__ __forceinline__ bool cta_wait_ge(const int* p, int target, int* err, unsigned long long wait_ns) {
+  const bool ok = threadIdx.x != 0 || wait_ge(p, target, err, wait_ns);
+  return !__syncthreads_or(!ok);
+}
+
+// After the CTA's stores: raise flag (if any) to epoch and add one to the
+// counter (if any).
+__device__ __forceinline__ void publish(int* flag, int epoch, int* counter) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    st_release(flags + idx, epoch);
+    if (flag) st_release(flag, epoch);
+    if (counter) atomicAdd(counter, 1);
   }
 }
 }  // namespace
@@ -126,20 +134,26 @@ __device__ __forceinline__ bool solve_index_ok(bool ok, int* err) {
 }
 
 // Shared-memory layout of both pipelined kernels (dynamic, doubles):
-//   acc[kRB][kRhsChunk + 1]   the task's result block
-//   xb [kRB][kRhsChunk + 1]   the right-hand-side block of the current tile
-//   Lb [2][kRB][kRB + 1]      double-buffered L tiles (odd stride: rows and
-//                             columns are both conflict-free)
+//   T  [2][64][68]  double-buffered L tiles, column-major as the front stores
+//                   them (a column's 64 rows consecutive: 16-byte copies, and
+//                   a stride that keeps the fragment loads of both products
+//                   conflict-free); the backward diagonal block is read along
+//                   rows and takes a stride of 65 instead
+//   xb [64][20]     the right-hand-side block of the current tile
+//   acc[64][20]     the task's result block
 // Every L tile a task needs is known from its position alone, so the next
 // tile is copied (cp.async) while the current one is used and before the
 // flag that guards its right-hand side is awaited.
-constexpr int kAccStride = kRhsChunk + 1;
-constexpr int kTileStride = kRB + 1;
-constexpr size_t kSolveSmem = (2 * kRB * kAccStride + 2 * kRB * kTileStride) * sizeof(double);
+constexpr int kTS = 68;
+constexpr int kTSDiag = 65;
+constexpr int kXS = 20;
+constexpr size_t kSolveSmem = (2 * kRB * kTS + 2 * kRB * kXS) * sizeof(double);
+constexpr int kTinyRows = 32;  // fronts of at most this many rows: one warp each
 
-__device__ __forceinline__ void scp_async8(double* smem_dst, const double* gsrc) {
+template <int Bytes>
+__device__ __forceinline__ void scp_async(double* smem_dst, const double* gsrc) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(gsrc), "n"(Bytes) : "memory");
 }
 __device__ __forceinline__ void scp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -148,27 +162,173 @@ __device__ __forceinline__ void scp_wait() {
 }
 
 // Tile (rows [i0, i0 + ni), columns [j0, j0 + nj)) of a front into T,
-// T[ii * kTileStride + jj]; entries outside the ranges are zero.
+// T[jj * kTS + ii]; entries outside the ranges are zero. i0 is even and the
+// front's columns start on 16-byte boundaries.
 __device__ __forceinline__ void stage_tile(double* T, const double* F, int64_t ld, int i0, int ni, int j0, int nj) {
+  for (int t = threadIdx.x; t < kRB * kRB / 2; t += kST) {
+    const int ii = 2 * (t % (kRB / 2)), jj = t / (kRB / 2);
+    double* d = T + jj * kTS + ii;
+    const double* src = F + static_cast<int64_t>(j0 + jj) * ld + i0 + ii;
+    if (ii + 1 < ni && jj < nj) {
+      scp_async<16>(d, src);
+    } else {
+      d[1] = 0.0;
+      if (ii < ni && jj < nj)
+        scp_async<8>(d, src);
+      else
+        d[0] = 0.0;
+    }
+  }
+  scp_commit();
+}
+// An n x n diagonal block at (q0, q0) into T[jj * kTSDiag + ii].
+__device__ __forceinline__ void stage_diag(double* T, const double* F, int64_t ld, int q0, int n) {
   for (int t = threadIdx.x; t < kRB * kRB; t += kST) {
     const int ii = t % kRB, jj = t / kRB;
-    double* d = T + ii * kTileStride + jj;
-    if (ii < ni && jj < nj)
-      scp_async8(d, F + static_cast<int64_t>(j0 + jj) * ld + i0 + ii);
-    else
-      *d = 0.0;
+    if (ii < n && jj < n) scp_async<8>(T + jj * kTSDiag + ii, F + static_cast<int64_t>(q0 + jj) * ld + q0 + ii);
   }
   scp_commit();
 }
 
+// c (16 x 8) += a (16 x 8) * b (8 x 8) on the FP64 tensor path; fragments as in
+// update_mma_kernel
+__device__ __forceinline__ void solve_dmma(double* c, const double* a, const double* b) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// The 64 x 64 by 64 x 16 product of a tile, summed over a block's tiles in
+// registers: warp w takes rows 16 (w & 3) and, of the right-hand sides, the
+// eight from 8 (w >> 2); with at most eight of them, warps 4 .. 7 take the
+// second half of the tile's inner dimension of the same eight instead.
+// Trans: the product with the tile's transpose (backward).
+template <bool Trans>
+struct TileProduct {
+  double p[2][4];
+  __device__ TileProduct() {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[h][e] = 0.0;
+  }
+  __device__ __forceinline__ void add(const double* T, const double* xb, int nc) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int r0 = 16 * (warp & 3), hi = warp >> 2;
+    const bool split = nc <= 8;
+    const int k0 = split ? 32 * hi : 0, c0 = split ? 0 : 8 * hi;
+    const int ksteps = split ? 4 : 8;
+#pragma unroll 4
+    for (int ks = 0; ks < ksteps; ++ks) {
+      const int k = k0 + 8 * ks;
+      double a[4], b[2];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = r0 + g + 8 * (r & 1), kk = k + t + 4 * (r >> 1);
+        a[r] = Trans ? T[row * kTS + kk] : T[kk * kTS + row];
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) b[r] = xb[(k + t + 4 * r) * kXS + c0 + g];
+      solve_dmma(p[ks & 1], a, b);
+    }
+  }
+  // acc[row][c] -= the product for row < rows, c < nc (a block barrier inside
+  // when the inner dimension was split)
+  __device__ __forceinline__ void subtract_into(double* acc, int rows, int nc) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int r0 = 16 * (warp & 3), hi = warp >> 2;
+    const bool split = nc <= 8;
+    const int c0 = split ? 0 : 8 * hi;
+    auto put = [&] {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = r0 + g + 8 * (e >> 1), c = c0 + 2 * t + (e & 1);
+        if (row < rows && c < nc) acc[row * kXS + c] -= p[0][e] + p[1][e];
+      }
+    };
+    if (!split || hi == 0) put();
+    if (split) {
+      __syncthreads();
+      if (hi == 1) put();
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------
+// Forward: one front of at most 32 rows by one warp, lane = row.
+__device__ bool forward_tiny(const FrontDesc* __restrict__ fronts, const ChildLink* __restrict__ links,
+                             const FrontState* __restrict__ st, int s, const SolvePlan& pl, int* counters, int* err,
+                             unsigned long long wait_ns, int nc, int c0, const double* __restrict__ Bp, int n) {
+  const int lane = threadIdx.x & 31;
+  const FrontDesc f = fronts[s];
+  const int m = f.m, np = st[s].npiv;
+  const int64_t ld = f.ld;
+  double y[kRhsChunk];
+#pragma unroll
+  for (int c = 0; c < kRhsChunk; ++c) y[c] = 0.0;
+  const int gi = lane < np ? f.fidx[lane] : 0;
+  if (lane < np && solve_index_ok(in_range(gi, 0, n), err))
+#pragma unroll
+    for (int c = 0; c < kRhsChunk; ++c)
+      if (c < nc) y[c] = Bp[gi + static_cast<int64_t>(c0 + c) * n];
+  const int need = pl.fwd_need[s];
+  if (need > 0) {
+    const bool ok = lane != 0 || wait_ge(counters + s, need, err, wait_ns);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    __syncwarp();
+    if (lane < m) {
+      const int pre = f.lperm[lane];
+      for (int ch = f.ch_begin; ch < f.ch_end; ++ch) {
+        const ChildLink L = links[ch];
+        const int a = L.invmap[pre];
+        if (a < 0) continue;
+        const FrontDesc& cf = fronts[L.child];
+        const int cnp = st[L.child].npiv;
+        if (solve_index_ok(cnp >= 0 && cnp + a < cf.m, err)) {
+          const double* w = cf.W + cnp + a + static_cast<int64_t>(c0) * cf.wld;
+#pragma unroll
+          for (int c = 0; c < kRhsChunk; ++c)
+            if (c < nc) y[c] += w[static_cast<int64_t>(c) * cf.wld];
+        }
+      }
+    }
+    __syncwarp();
+  }
+  for (int j0 = 0; j0 < np; j0 += 4) {
+    double l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = j0 + q;
+      // (the slot below a 2x2 pivot's first column holds d21, not L)
+      l[q] = (j < np && lane > j && lane < m && !(f.pk[j] == 1 && lane == j + 1)) ? f.F[j * ld + lane] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j0 + q < np)
+#pragma unroll
+        for (int c = 0; c < kRhsChunk; ++c)
+          if (c < nc) y[c] = fma(-l[q], __shfl_sync(0xffffffffu, y[c], j0 + q), y[c]);
+  }
+  if (lane < m) {
+    double* w = f.W + lane + static_cast<int64_t>(c0) * f.wld;
+#pragma unroll
+    for (int c = 0; c < kRhsChunk; ++c)
+      if (c < nc) w[static_cast<int64_t>(c) * f.wld] = y[c];
+  }
+  __syncwarp();
+  if (lane == 0 && f.parent >= 0) {
+    __threadfence();
+    atomicAdd(counters + f.parent, 1);
+  }
+  return true;
+}
+
 // Forward: one row block (front s, block rb). Returns false when a wait
 // ended in an error (the CTA then leaves the launch).
 __device__ bool forward_block(const FrontDesc* __restrict__ fronts, const ChildLink* __restrict__ links,
-                              const FrontState* __restrict__ st, int s, int rb, const int* __restrict__ flag_base,
-                              int* flags, int epoch, int* err, unsigned long long wait_ns, int nc, int c0,
+                              const FrontState* __restrict__ st, int s, int rb, const SolvePlan& pl, int* flags,
+                              int* counters, int epoch, int* err, unsigned long long wait_ns, int nc, int c0,
                               const double* __restrict__ Bp, int n, double* acc, double* xb, double* Lb0) {
-  const int row = threadIdx.x % kRB, cg = threadIdx.x / kRB;  // product layout: a row, 4 right-hand sides
   const FrontDesc f = fronts[s];
   const int m = f.m, np = st[s].npiv;
   const int r0 = rb * kRB, r1 = min(r0 + kRB, m), nr = r1 - r0;
@@ -179,6 +339,7 @@ __device__ bool forward_block(const FrontDesc* __restrict__ fronts, const ChildL
   const int jend = min(rb, nbp);
   const bool hasDiag = r0 < np;
   const int ntiles = jend + (hasDiag ? 1 : 0);
+  const int fbase = pl.flag_base[s];
   // pivot kinds the steps below need, loaded before any wait: a 2x2 pivot
   // ending at row r0 - 1 (its d21 slot sits in the last earlier tile) and
   // one starting at this thread's row of the diagonal block
@@ -186,7 +347,7 @@ __device__ bool forward_block(const FrontDesc* __restrict__ fronts, const ChildL
   const bool own_pair = hasDiag && threadIdx.x + 1 < min(r1, np) - r0 && f.pk[r0 + threadIdx.x] == 1;
   // tile tt: pivot block tt (tt < jend) or the diagonal block
   auto stage = [&](int tt) {
-    double* T = Lb0 + (tt & 1) * kRB * kTileStride;
+    double* T = Lb0 + (tt & 1) * kRB * kTS;
     if (tt < jend) {
       const int j0 = tt * kRB;
       stage_tile(T, f.F, ld, r0, nr, j0, min(j0 + kRB, np) - j0);
@@ -197,6 +358,11 @@ __device__ bool forward_block(const FrontDesc* __restrict__ fronts, const ChildL
   if (ntiles > 0) stage(0);
   // 1. Bp for pivot rows plus the children's forwarded rows, gathered
   //    through each row's pre-pivot position
+  const int need = pl.fwd_need[s];
+  if (need > 0 && !cta_wait_ge(counters + s, need, err, wait_ns)) {
+    scp_wait<0>();
+    return false;
+  }
   for (int t = threadIdx.x; t < nr * nc; t += kST) {
     const int ii = t % nr, c = t / nr;
     const int i = r0 + ii;
@@ -214,144 +380,206 @@ __device__ bool forward_block(const FrontDesc* __restrict__ fronts, const ChildL
       const int cnp = st[L.child].npiv;
       if (solve_index_ok(cnp >= 0 && cnp + a < cf.m, err)) v += cf.W[cnp + a + static_cast<int64_t>(c0 + c) * cf.wld];
     }
-    acc[ii * kAccStride + c] = v;
+    acc[ii * kXS + c] = v;
   }
-  for (int tt = 0; tt < ntiles; ++tt) {
+  TileProduct<false> prod;
+  for (int tt = 0; tt < jend; ++tt) {
+    // 2. contribution of finished pivot block tt
     const bool more = tt + 1 < ntiles;
     if (more) stage(tt + 1);
-    double* T = Lb0 + (tt & 1) * kRB * kTileStride;
-    if (tt < jend) {
-      // 2. contribution of finished pivot block j = tt
-      const int j = tt;
-      if (!wait_flag(flags, flag_base[s] + j, epoch, err, wait_ns)) {
-        scp_wait<0>();
-        return false;
-      }
-      const int j0 = j * kRB, nj = min(j0 + kRB, np) - j0;
-      for (int t = threadIdx.x; t < kRB * nc; t += kST) {
-        const int jj = t % kRB, c = t / kRB;
-        xb[jj * kAccStride + c] = (jj < nj) ? W[j0 + jj + static_cast<int64_t>(c0 + c) * wld] : 0.0;
-      }
-      if (more)
-        scp_wait<1>();
-      else
-        scp_wait<0>();
-      __syncthreads();
-      // a 2x2 pivot straddling the block boundary: its d21 slot in L is not
-      // an L entry
-      if (threadIdx.x == 0 && j == rb - 1 && r0 - 1 >= j0 && pair_before) T[r0 - 1 - j0] = 0.0;
-      __syncthreads();
-      if (row < nr) {
-        double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
-        const int cb4 = cg * 4;
-#pragma unroll 8
-        for (int jj = 0; jj < nj; ++jj) {
-          const double l = T[row * kTileStride + jj];
-          const double* y = xb + jj * kAccStride + cb4;
-          p0 = fma(l, y[0], p0);
-          p1 = fma(l, y[1], p1);
-          p2 = fma(l, y[2], p2);
-          p3 = fma(l, y[3], p3);
-        }
-        double* a = acc + row * kAccStride + cb4;
-        if (cb4 + 0 < nc) a[0] -= p0;
-        if (cb4 + 1 < nc) a[1] -= p1;
-        if (cb4 + 2 < nc) a[2] -= p2;
-        if (cb4 + 3 < nc) a[3] -= p3;
-      }
-      __syncthreads();
-    } else {
-      // 3. the block's own pivot columns: unit-lower solve for its pivot
-      //    rows and the matching update of its non-pivot rows
+    double* T = Lb0 + (tt & 1) * kRB * kTS;
+    if (!cta_wait_ge(flags + fbase + tt, epoch, err, wait_ns)) {
       scp_wait<0>();
+      return false;
+    }
+    const int j0 = tt * kRB, nj = min(j0 + kRB, np) - j0;
+    for (int t = threadIdx.x; t < kRB * kRhsChunk; t += kST) {
+      const int jj = t % kRB, c = t / kRB;
+      xb[jj * kXS + c] = (jj < nj && c < nc) ? W[j0 + jj + static_cast<int64_t>(c0 + c) * wld] : 0.0;
+    }
+    if (more)
+      scp_wait<1>();
+    else
+      scp_wait<0>();
+    __syncthreads();
+    // a 2x2 pivot straddling the block boundary: its d21 slot in L is not
+    // an L entry
+    if (pair_before && tt == rb - 1) {
+      if (threadIdx.x == 0) T[(r0 - 1 - j0) * kTS] = 0.0;
       __syncthreads();
-      const int npv = min(r1, np) - r0;
-      if (own_pair) T[(threadIdx.x + 1) * kTileStride + threadIdx.x] = 0.0;  // d21 slot of a 2x2 pivot
-      __syncthreads();
-      // a warp takes right-hand sides c and c + 8 together: the two
-      // substitution chains interleave (each step is a shuffle and an FMA)
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      constexpr int NW = kST / 32;
-      for (int c = warp; c < nc; c += 2 * NW) {
-        const int cb = c + NW;
-        const bool two = cb < nc;
-        double y0 = (lane < nr) ? acc[lane * kAccStride + c] : 0.0;
-        double y1 = (lane + 32 < nr) ? acc[(lane + 32) * kAccStride + c] : 0.0;
-        double z0 = (two && lane < nr) ? acc[lane * kAccStride + cb] : 0.0;
-        double z1 = (two && lane + 32 < nr) ? acc[(lane + 32) * kAccStride + cb] : 0.0;
-        for (int jj = 0; jj < npv; ++jj) {
-          const double yj = __shfl_sync(0xffffffffu, jj < 32 ? y0 : y1, jj & 31);
-          const double zj = __shfl_sync(0xffffffffu, jj < 32 ? z0 : z1, jj & 31);
-          const double t0 = T[lane * kTileStride + jj], t1 = T[(lane + 32) * kTileStride + jj];
-          if (lane > jj) {
-            y0 -= t0 * yj;
-            z0 -= t0 * zj;
-          }
-          if (lane + 32 > jj) {
-            y1 -= t1 * yj;
-            z1 -= t1 * zj;
-          }
+    }
+    prod.add(T, xb, nc);
+    __syncthreads();
+  }
+  if (jend > 0) prod.subtract_into(acc, nr, nc);
+  if (hasDiag) {
+    // 3. the block's own pivot columns: unit-lower solve for its pivot
+    //    rows and the matching update of its non-pivot rows
+    double* T = Lb0 + (jend & 1) * kRB * kTS;
+    scp_wait<0>();
+    __syncthreads();
+    const int npv = min(r1, np) - r0;
+    if (own_pair) T[threadIdx.x * kTS + threadIdx.x + 1] = 0.0;  // d21 slot of a 2x2 pivot
+    __syncthreads();
+    // a warp takes right-hand sides c and c + 8 together: the two
+    // substitution chains interleave (each step is a shuffle and an FMA)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NW = kST / 32;
+    for (int c = warp; c < nc; c += 2 * NW) {
+      const int cb = c + NW;
+      const bool two = cb < nc;
+      double y0 = (lane < nr) ? acc[lane * kXS + c] : 0.0;
+      double y1 = (lane + 32 < nr) ? acc[(lane + 32) * kXS + c] : 0.0;
+      double z0 = (two && lane < nr) ? acc[lane * kXS + cb] : 0.0;
+      double z1 = (two && lane + 32 < nr) ? acc[(lane + 32) * kXS + cb] : 0.0;
+      const int nlow = min(npv, 32);
+#pragma unroll 8
+      for (int jj = 0; jj < nlow; ++jj) {
+        const double yj = __shfl_sync(0xffffffffu, y0, jj), zj = __shfl_sync(0xffffffffu, z0, jj);
+        const double t0 = T[jj * kTS + lane], t1 = T[jj * kTS + lane + 32];
+        if (lane > jj) {
+          y0 -= t0 * yj;
+          z0 -= t0 * zj;
         }
-        if (lane < nr) acc[lane * kAccStride + c] = y0;
-        if (lane + 32 < nr) acc[(lane + 32) * kAccStride + c] = y1;
-        if (two && lane < nr) acc[lane * kAccStride + cb] = z0;
-        if (two && lane + 32 < nr) acc[(lane + 32) * kAccStride + cb] = z1;
+        y1 -= t1 * yj;
+        z1 -= t1 * zj;
       }
-      __syncthreads();
+#pragma unroll 8
+      for (int jj = 32; jj < npv; ++jj) {
+        const double yj = __shfl_sync(0xffffffffu, y1, jj - 32), zj = __shfl_sync(0xffffffffu, z1, jj - 32);
+        const double t1 = T[jj * kTS + lane + 32];
+        if (lane + 32 > jj) {
+          y1 -= t1 * yj;
+          z1 -= t1 * zj;
+        }
+      }
+      if (lane < nr) acc[lane * kXS + c] = y0;
+      if (lane + 32 < nr) acc[(lane + 32) * kXS + c] = y1;
+      if (two && lane < nr) acc[lane * kXS + cb] = z0;
+      if (two && lane + 32 < nr) acc[(lane + 32) * kXS + cb] = z1;
     }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < nr * nc; t += kST) {
     const int ii = t % nr, c = t / nr;
-    W[r0 + ii + static_cast<int64_t>(c0 + c) * wld] = acc[ii * kAccStride + c];
+    W[r0 + ii + static_cast<int64_t>(c0 + c) * wld] = acc[ii * kXS + c];
   }
-  if (hasDiag) publish(flags, flag_base[s] + rb, epoch);
+  publish(hasDiag ? flags + fbase + rb : nullptr, epoch, f.parent >= 0 ? counters + f.parent : nullptr);
   __syncthreads();
   return true;
 }
 
-// Forward task = int4 {front, row block, 0, 0}, or {front, -1, 0, 0} for the
-// whole front (its row blocks in order, in this CTA). Flag of a pivot row
-// block at flag_base[front] + row block.
+// Forward task = int4 {front, row block, 0, 0} or {first, -2, count, 0}: the
+// fronts pl.tiny[first ..], a warp each. Flag of a pivot row block at
+// flag_base[front] + row block. Task t of the launch is task t / nchunks of
+// the list for right-hand-side group t % nchunks (16 from c0 + 16 of it),
+// whose flags and counters are its own.
 __global__ void __launch_bounds__(kST, 2) forward_pipelined_kernel(
     const FrontDesc* __restrict__ fronts, const ChildLink* __restrict__ links, const FrontState* __restrict__ st,
-    const int4* __restrict__ tasks, int ntasks, const int* __restrict__ flag_base, int* flags, int epoch, int* err,
-    unsigned long long wait_ns, int nrhs, int c0, const double* __restrict__ Bp, int n) {
-  extern __shared__ double ssm[];
-  double* acc = ssm;
-  double* xb = acc + kRB * kAccStride;
-  double* Lb0 = xb + kRB * kAccStride;
-  const int nc = min(kRhsChunk, nrhs - c0);
-  for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+    SolvePlan pl, int task0, int ntasks, int nchunks, int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0,
+    const double* __restrict__ Bp, int n) {
+  extern __shared__ __align__(16) double ssm[];
+  double* Lb0 = ssm;
+  double* xb = Lb0 + 2 * kRB * kTS;
+  double* acc = xb + kRB * kXS;
+  for (int t = blockIdx.x; t < ntasks * nchunks; t += gridDim.x) {
     if (ld_acquire(err) != 0) return;
-    const int4 tk = tasks[task];
-    const int s = tk.x;
+    const int chunk = t % nchunks, cc0 = c0 + chunk * kRhsChunk, nc = min(kRhsChunk, nrhs - cc0);
+    const int4 tk = pl.fwd_tasks[task0 + t / nchunks];
+    int* flags = pl.flags + static_cast<int64_t>(chunk) * pl.nflags;
+    int* counters = pl.counters + static_cast<int64_t>(chunk) * pl.nfronts;
     if (tk.y >= 0) {
-      if (!forward_block(fronts, links, st, s, tk.y, flag_base, flags, epoch, err, wait_ns, nc, c0, Bp, n, acc, xb, Lb0)) return;
+      if (!forward_block(fronts, links, st, tk.x, tk.y, pl, flags, counters, epoch, err, wait_ns, nc, cc0, Bp, n, acc,
+                         xb, Lb0))
+        return;
     } else {
-      const int nb = (fronts[s].m + kRB - 1) / kRB;
-      for (int rb = 0; rb < nb; ++rb)
-        if (!forward_block(fronts, links, st, s, rb, flag_base, flags, epoch, err, wait_ns, nc, c0, Bp, n, acc, xb, Lb0))
-          return;
+      const int w = threadIdx.x >> 5;
+      const bool ok = w >= tk.z || forward_tiny(fronts, links, st, pl.tiny[tk.x + w], pl, counters, err, wait_ns, nc,
+                                                cc0, Bp, n);
+      if (__syncthreads_or(!ok)) return;
     }
   }
 }
 
 // ---------------------------------------------------------------------------
+// z = (D^{-1} y)_q of a front's pivot q (w: a right-hand side's column of W)
+__device__ __forceinline__ double d_inverse(const FrontDesc& f, const double* w, int q) {
+  const int8_t kind = f.pk[q];
+  if (kind == 0) return w[q] / f.Dd[q];
+  const int a = kind == 1 ? q : q - 1;
+  const double d11 = f.Dd[a], d21 = f.Do[a], d22 = f.Dd[a + 1];
+  const double det = d11 * d22 - d21 * d21;
+  return (kind == 1 ? d22 * w[q] - d21 * w[q + 1] : -d21 * w[q - 1] + d11 * w[q]) / det;
+}
+
+// Backward: one front of at most 32 rows by one warp; lanes below npiv hold
+// its unknowns, the others its ancestors' values.
+__device__ bool backward_tiny(const FrontDesc* __restrict__ fronts, const FrontState* __restrict__ st, int s,
+                              const SolvePlan& pl, int* counters, int* err, unsigned long long wait_ns, int nc, int c0,
+                              double* __restrict__ X, int n) {
+  const int lane = threadIdx.x & 31;
+  const FrontDesc f = fronts[s];
+  const int m = f.m, np = st[s].npiv;
+  const int64_t ld = f.ld;
+  double x[kRhsChunk];
+#pragma unroll
+  for (int c = 0; c < kRhsChunk; ++c)
+    x[c] = (lane < np && c < nc) ? d_inverse(f, f.W + static_cast<int64_t>(c0 + c) * f.wld, lane) : 0.0;
+  const int gi = lane < m ? f.fidx[lane] : 0;
+  const bool idx_ok = lane < m && solve_index_ok(in_range(gi, 0, n), err);
+  const bool pair = lane < np && f.pk[lane] == 1;
+  const int anc = pl.bwd_wait[s];
+  if (anc >= 0) {
+    const bool ok = lane != 0 || wait_ge(counters + anc, pl.bwd_need[s], err, wait_ns);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    __syncwarp();
+    if (lane >= np && idx_ok)
+#pragma unroll
+      for (int c = 0; c < kRhsChunk; ++c)
+        if (c < nc) x[c] = X[gi + static_cast<int64_t>(c0 + c) * n];
+  }
+  // row r's value is final once every row below it has been applied
+  for (int r0 = m - 1; r0 > 0; r0 -= 4) {
+    double l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 - q;
+      l[q] = (r > lane && lane < np && !(pair && r == lane + 1)) ? f.F[lane * ld + r] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (r0 - q > 0)
+#pragma unroll
+        for (int c = 0; c < kRhsChunk; ++c)
+          if (c < nc) x[c] = fma(-l[q], __shfl_sync(0xffffffffu, x[c], r0 - q), x[c]);
+  }
+  if (lane < np && idx_ok)
+#pragma unroll
+    for (int c = 0; c < kRhsChunk; ++c)
+      if (c < nc) X[gi + static_cast<int64_t>(c0 + c) * n] = x[c];
+  __syncwarp();
+  if (lane == 0 && np > 0) {
+    __threadfence();
+    atomicAdd(counters + s, 1);
+  }
+  return true;
+}
+
 // Backward: pivot column block cb of front s. The tiles are the ancestor
 // rows [np, m) in 64-row chunks, then the later pivot blocks, then the
 // diagonal block. A main part (part 0) does ancestor chunks [a0, a1), the
 // later blocks, adds its helper parts' partial sums (slots hslot0 ..
 // hslot0 + nh - 1, in slot order) and finishes the block; a helper part
 // only sums its ancestor chunks into its scratch slot and raises its flag.
+// (np need not be a multiple of 64: an ancestor chunk starts at an even row,
+// at or one before its first, so that its columns stay 16-byte aligned.)
 __device__ bool backward_block(const FrontDesc* __restrict__ fronts, const FrontState* __restrict__ st, int s, int cb,
-                               bool helper, int a0, int a1, int hslot0, int nh, const int* __restrict__ flag_base,
-                               int* flags, int* hflags, double* hscratch, int epoch, int* err,
+                               bool helper, int a0, int a1, int hslot0, int nh, const SolvePlan& pl, int* flags,
+                               int* hflags, double* hscratch, int* counters, int epoch, int* err,
                                unsigned long long wait_ns, int nc, int c0, double* __restrict__ X, int n, double* acc,
                                double* xb, double* Lb0) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = kST / 32;
-  const int col = threadIdx.x % kRB, cg = threadIdx.x / kRB;
   const FrontDesc f = fronts[s];
   const int m = f.m, np = st[s].npiv;
   const int q0 = cb * kRB, q1 = min(q0 + kRB, np), nq = q1 - q0;
@@ -362,6 +590,7 @@ __device__ bool backward_block(const FrontDesc* __restrict__ fronts, const Front
   const int nanc = a1 - a0;
   const int nlater = helper ? 0 : nbp - 1 - cb;
   const int ntiles = nanc + nlater + (helper ? 0 : 1);
+  const int fbase = pl.flag_base[s];
   // loaded before any wait: the 2x2 pivot kinds the steps below need and
   // the rows the block's solution is written to
   static_assert(kST % kRB == 0, "a thread keeps one tile row in the gathers");
@@ -369,212 +598,214 @@ __device__ bool backward_block(const FrontDesc* __restrict__ fronts, const Front
   const bool pair_at_end = nq > 0 && f.pk[q1 - 1] == 1;
   const bool own_pair = threadIdx.x + 1 < nq && f.pk[q0 + threadIdx.x] == 1;
   if (!helper && threadIdx.x < nq) s_row[threadIdx.x] = f.fidx[q0 + threadIdx.x];
+  const int anc0 = np & ~1;  // ancestor chunks: rows [anc0 + 64 a, ...) without those below np
   auto tile_rows = [&](int tt, int& i0, int& i1) {
     if (tt < nanc) {
-      i0 = np + (a0 + tt) * kRB;
+      i0 = anc0 + (a0 + tt) * kRB;
       i1 = min(i0 + kRB, m);
-    } else if (tt < nanc + nlater) {
+    } else {
       const int j = nbp - 1 - (tt - nanc);
       i0 = j * kRB;
       i1 = min(i0 + kRB, np);
-    } else {
-      i0 = q0;
-      i1 = q1;
     }
   };
   auto stage = [&](int tt) {
-    int i0, i1;
-    tile_rows(tt, i0, i1);
-    stage_tile(Lb0 + (tt & 1) * kRB * kTileStride, f.F, ld, i0, i1 - i0, q0, nq);
+    double* T = Lb0 + (tt & 1) * kRB * kTS;
+    if (tt < nanc + nlater) {
+      int i0, i1;
+      tile_rows(tt, i0, i1);
+      stage_tile(T, f.F, ld, i0, i1 - i0, q0, nq);
+    } else {
+      stage_diag(T, f.F, ld, q0, nq);
+    }
   };
   if (ntiles > 0) stage(0);
   if (helper) {
-    for (int t = threadIdx.x; t < kRB * nc; t += kST) acc[(t % kRB) * kAccStride + t / kRB] = 0.0;
+    for (int t = threadIdx.x; t < kRB * nc; t += kST) acc[(t % kRB) * kXS + t / kRB] = 0.0;
   } else {
     // 1. z = D^{-1} y for the block's pivots (a 2x2 partner may sit in the
     //    neighbouring block; y is complete in W after the forward pass)
     for (int t = threadIdx.x; t < nq * nc; t += kST) {
       const int qq = t % nq, c = t / nq;
-      const int q = q0 + qq;
-      const double* w = W + static_cast<int64_t>(c0 + c) * wld;
-      const int8_t kind = f.pk[q];
-      double z;
-      if (kind == 0) {
-        z = w[q] / f.Dd[q];
-      } else if (kind == 1) {
-        const double d11 = f.Dd[q], d21 = f.Do[q], d22 = f.Dd[q + 1];
-        const double det = d11 * d22 - d21 * d21;
-        z = (d22 * w[q] - d21 * w[q + 1]) / det;
-      } else {
-        const double d11 = f.Dd[q - 1], d21 = f.Do[q - 1], d22 = f.Dd[q];
-        const double det = d11 * d22 - d21 * d21;
-        z = (-d21 * w[q - 1] + d11 * w[q]) / det;
-      }
-      acc[qq * kAccStride + c] = z;
+      acc[qq * kXS + c] = d_inverse(f, W + static_cast<int64_t>(c0 + c) * wld, q0 + qq);
     }
   }
-  for (int tt = 0; tt < ntiles; ++tt) {
+  // the ancestors' values are complete once the nearest ancestor with pivots is
+  const int anc = nanc > 0 ? pl.bwd_wait[s] : -1;
+  if (anc >= 0 && !cta_wait_ge(counters + anc, pl.bwd_need[s], err, wait_ns)) {
+    scp_wait<0>();
+    return false;
+  }
+  TileProduct<true> prod;
+  for (int tt = 0; tt < nanc + nlater; ++tt) {
+    // 2. minus L(rows of the tile, block)^T x(rows of the tile); later pivot
+    //    blocks of this front are waited for
     const bool more = tt + 1 < ntiles;
     if (more) stage(tt + 1);
-    double* T = Lb0 + (tt & 1) * kRB * kTileStride;
+    double* T = Lb0 + (tt & 1) * kRB * kTS;
     int i0, i1;
     tile_rows(tt, i0, i1);
-    if (tt < nanc + nlater) {
-      // 2. minus L(rows of the tile, block)^T x(rows of the tile): the
-      //    ancestor rows are final from earlier levels; later pivot blocks of
-      //    this front are waited for
-      const int ni = i1 - i0;
-      // this thread's tile row (the same for every t below), before the wait
-      const int my_ii = threadIdx.x % kRB;
-      const int my_gi = my_ii < ni ? f.fidx[i0 + my_ii] : 0;
-      if (tt >= nanc) {
-        const int j = nbp - 1 - (tt - nanc);
-        if (!wait_flag(flags, flag_base[s] + j, epoch, err, wait_ns)) {
-          scp_wait<0>();
-          return false;
-        }
-      }
-      for (int t = threadIdx.x; t < kRB * nc; t += kST) {
-        const int ii = t % kRB, c = t / kRB;
-        double xv = 0.0;
-        if (ii < ni) {
-          const int gi = my_gi;
-          if (solve_index_ok(in_range(gi, 0, n), err)) xv = X[gi + static_cast<int64_t>(c0 + c) * n];
-        }
-        xb[ii * kAccStride + c] = xv;
-      }
-      if (more)
-        scp_wait<1>();
-      else
+    const int first = tt < nanc ? np : i0;  // rows of the tile before it are not the tile's
+    // this thread's tile row (the same for every t below), before the wait
+    const int my_i = i0 + static_cast<int>(threadIdx.x) % kRB;
+    const bool mine = my_i >= first && my_i < i1;
+    const int my_gi = mine ? f.fidx[my_i] : 0;
+    if (tt >= nanc) {
+      const int j = nbp - 1 - (tt - nanc);
+      if (!cta_wait_ge(flags + fbase + j, epoch, err, wait_ns)) {
         scp_wait<0>();
-      __syncthreads();
-      // a 2x2 pivot straddling the block boundary: d21 is not an L entry
-      if (threadIdx.x == 0 && i0 == q1 && pair_at_end) T[nq - 1] = 0.0;
-      __syncthreads();
-      if (col < nq) {
-        double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0;
-        const int cb4 = cg * 4;
-#pragma unroll 8
-        for (int ii = 0; ii < ni; ++ii) {
-          const double l = T[ii * kTileStride + col];
-          const double* x = xb + ii * kAccStride + cb4;
-          p0 = fma(l, x[0], p0);
-          p1 = fma(l, x[1], p1);
-          p2 = fma(l, x[2], p2);
-          p3 = fma(l, x[3], p3);
-        }
-        double* a = acc + col * kAccStride + cb4;
-        if (cb4 + 0 < nc) a[0] -= p0;
-        if (cb4 + 1 < nc) a[1] -= p1;
-        if (cb4 + 2 < nc) a[2] -= p2;
-        if (cb4 + 3 < nc) a[3] -= p3;
+        return false;
       }
-      __syncthreads();
-    } else {
-      // helper parts' partial sums, in slot order (deterministic)
-      for (int h = 0; h < nh; ++h) {
-        if (!wait_flag(hflags, hslot0 + h, epoch, err, wait_ns)) {
-          scp_wait<0>();
-          return false;
-        }
-        const double* part = hscratch + static_cast<int64_t>(hslot0 + h) * kRB * kRhsChunk;
-        for (int t = threadIdx.x; t < nq * nc; t += kST) {
-          const int qq = t % nq, c = t / nq;
-          acc[qq * kAccStride + c] += part[c * kRB + qq];
-        }
-        __syncthreads();
-      }
-      // 3. transposed unit-lower solve on the diagonal block
+    }
+    const bool load = mine && solve_index_ok(in_range(my_gi, 0, n), err);
+    for (int t = threadIdx.x; t < kRB * kRhsChunk; t += kST) {
+      const int c = t / kRB;
+      xb[(t % kRB) * kXS + c] = (load && c < nc) ? X[my_gi + static_cast<int64_t>(c0 + c) * n] : 0.0;
+    }
+    if (more)
+      scp_wait<1>();
+    else
       scp_wait<0>();
-      __syncthreads();
-      if (own_pair) T[(threadIdx.x + 1) * kTileStride + threadIdx.x] = 0.0;  // d21 slot of a 2x2 pivot
-      __syncthreads();
-      // right-hand sides c and c + NW together (interleaved chains)
-      for (int c = warp; c < nc; c += 2 * NW) {
-        const int cb = c + NW;
-        const bool two = cb < nc;
-        double x0 = (lane < nq) ? acc[lane * kAccStride + c] : 0.0;
-        double x1 = (lane + 32 < nq) ? acc[(lane + 32) * kAccStride + c] : 0.0;
-        double u0 = (two && lane < nq) ? acc[lane * kAccStride + cb] : 0.0;
-        double u1 = (two && lane + 32 < nq) ? acc[(lane + 32) * kAccStride + cb] : 0.0;
-        for (int jj = nq - 1; jj >= 0; --jj) {
-          // x[jj] is final once every row below it has been applied; row jj
-          // of Ltop then updates the unknowns above it
-          const double xj = __shfl_sync(0xffffffffu, jj < 32 ? x0 : x1, jj & 31);
-          const double uj = __shfl_sync(0xffffffffu, jj < 32 ? u0 : u1, jj & 31);
-          const double t0 = T[jj * kTileStride + lane], t1 = T[jj * kTileStride + lane + 32];
-          if (lane < jj) {
-            x0 -= t0 * xj;
-            u0 -= t0 * uj;
-          }
-          if (lane + 32 < jj) {
-            x1 -= t1 * xj;
-            u1 -= t1 * uj;
-          }
-        }
-        if (lane < nq) acc[lane * kAccStride + c] = x0;
-        if (lane + 32 < nq) acc[(lane + 32) * kAccStride + c] = x1;
-        if (two && lane < nq) acc[lane * kAccStride + cb] = u0;
-        if (two && lane + 32 < nq) acc[(lane + 32) * kAccStride + cb] = u1;
-      }
+    __syncthreads();
+    // a 2x2 pivot straddling the block boundary: its d21 slot (row q1) is not
+    // an L entry; the pivot row before an odd np is not the chunk's
+    const bool odd_row = first > i0, straddle = pair_at_end && i0 == q1;
+    if (odd_row || straddle) {
+      if (odd_row && threadIdx.x < kRB) T[threadIdx.x * kTS] = 0.0;
+      if (straddle && threadIdx.x == 0) T[(nq - 1) * kTS] = 0.0;
       __syncthreads();
     }
+    prod.add(T, xb, nc);
+    __syncthreads();
   }
+  if (nanc + nlater > 0) prod.subtract_into(acc, nq, nc);
+  __syncthreads();
   if (helper) {
     // acc holds minus the helper's partial sum; the main part adds it
     double* part = hscratch + static_cast<int64_t>(hslot0) * kRB * kRhsChunk;
     for (int t = threadIdx.x; t < nq * nc; t += kST) {
       const int qq = t % nq, c = t / nq;
-      part[c * kRB + qq] = acc[qq * kAccStride + c];
+      part[c * kRB + qq] = acc[qq * kXS + c];
     }
-    publish(hflags, hslot0, epoch);
-  } else {
+    publish(hflags + hslot0, epoch, nullptr);
+    __syncthreads();
+    return true;
+  }
+  // helper parts' partial sums, in slot order (deterministic)
+  for (int h = 0; h < nh; ++h) {
+    if (!cta_wait_ge(hflags + hslot0 + h, epoch, err, wait_ns)) {
+      scp_wait<0>();
+      return false;
+    }
+    const double* part = hscratch + static_cast<int64_t>(hslot0 + h) * kRB * kRhsChunk;
     for (int t = threadIdx.x; t < nq * nc; t += kST) {
       const int qq = t % nq, c = t / nq;
-      const int gi = s_row[qq];
-      if (solve_index_ok(in_range(gi, 0, n), err)) X[gi + static_cast<int64_t>(c0 + c) * n] = acc[qq * kAccStride + c];
+      acc[qq * kXS + c] += part[c * kRB + qq];
     }
-    publish(flags, flag_base[s] + cb, epoch);
   }
+  // 3. transposed unit-lower solve on the diagonal block
+  double* T = Lb0 + ((nanc + nlater) & 1) * kRB * kTS;
+  scp_wait<0>();
+  __syncthreads();
+  if (own_pair) T[threadIdx.x * kTSDiag + threadIdx.x + 1] = 0.0;  // d21 slot of a 2x2 pivot
+  __syncthreads();
+  // right-hand sides c and c + NW together (interleaved chains)
+  for (int c = warp; c < nc; c += 2 * NW) {
+    const int cb2 = c + NW;
+    const bool two = cb2 < nc;
+    double x0 = (lane < nq) ? acc[lane * kXS + c] : 0.0;
+    double x1 = (lane + 32 < nq) ? acc[(lane + 32) * kXS + c] : 0.0;
+    double u0 = (two && lane < nq) ? acc[lane * kXS + cb2] : 0.0;
+    double u1 = (two && lane + 32 < nq) ? acc[(lane + 32) * kXS + cb2] : 0.0;
+    // x[jj] is final once every row below it has been applied; row jj of
+    // Ltop then updates the unknowns above it
+#pragma unroll 8
+    for (int jj = nq - 1; jj >= 32; --jj) {
+      const double xj = __shfl_sync(0xffffffffu, x1, jj - 32), uj = __shfl_sync(0xffffffffu, u1, jj - 32);
+      const double t0 = T[lane * kTSDiag + jj];
+      x0 -= t0 * xj;
+      u0 -= t0 * uj;
+      if (lane + 32 < jj) {
+        const double t1 = T[(lane + 32) * kTSDiag + jj];
+        x1 -= t1 * xj;
+        u1 -= t1 * uj;
+      }
+    }
+#pragma unroll 8
+    for (int jj = min(nq, 32) - 1; jj >= 0; --jj) {
+      const double xj = __shfl_sync(0xffffffffu, x0, jj), uj = __shfl_sync(0xffffffffu, u0, jj);
+      if (lane < jj) {
+        const double t0 = T[lane * kTSDiag + jj];
+        x0 -= t0 * xj;
+        u0 -= t0 * uj;
+      }
+    }
+    if (lane < nq) acc[lane * kXS + c] = x0;
+    if (lane + 32 < nq) acc[(lane + 32) * kXS + c] = x1;
+    if (two && lane < nq) acc[lane * kXS + cb2] = u0;
+    if (two && lane + 32 < nq) acc[(lane + 32) * kXS + cb2] = u1;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nq * nc; t += kST) {
+    const int qq = t % nq, c = t / nq;
+    const int gi = s_row[qq];
+    if (solve_index_ok(in_range(gi, 0, n), err)) X[gi + static_cast<int64_t>(c0 + c) * n] = acc[qq * kXS + c];
+  }
+  publish(flags + fbase + cb, epoch, counters + s);
   __syncthreads();
   return true;
 }
 
+// Number of 64-row ancestor chunks of a front (from the even row at or
+// before np).
+__host__ __device__ inline int ancestor_chunks(int m, int np) { return m > np ? (m - (np & ~1) + kRB - 1) / kRB : 0; }
+
 // Backward task = int4 {front, column block, part, aux}:
-//   {s, -1, 0, 0}            the whole front (blocks last to first, this CTA)
+//   {first, -2, count, 0}     the fronts pl.tiny[first ..], a warp each
+//   {s, -1, 0, 0}             the whole front (blocks last to first, this CTA)
 //   {s, cb, 0, P << 20 | h0}  main part of block cb with P parts in all; its
 //                             helpers hold scratch slots h0 .. h0 + P - 2
 //   {s, cb, p, P << 20 | h}   helper part p (1 <= p < P) in slot h
 // The ancestor chunks of a block are split evenly over its P parts. Helpers
 // are listed before their main part, and later blocks of a front before
-// earlier ones, so every wait is on a task with a smaller index.
+// earlier ones, so every wait is on a task with a smaller index. Tasks of the
+// launch as in forward_pipelined_kernel.
 __global__ void __launch_bounds__(kST, 2) backward_pipelined_kernel(
-    const FrontDesc* __restrict__ fronts, const FrontState* __restrict__ st, const int4* __restrict__ tasks,
-    int ntasks, const int* __restrict__ flag_base, int* flags, int* hflags, double* hscratch, int epoch, int* err,
-    unsigned long long wait_ns, int nrhs, int c0, double* __restrict__ X, int n) {
-  extern __shared__ double ssm[];
-  double* acc = ssm;
-  double* xb = acc + kRB * kAccStride;
-  double* Lb0 = xb + kRB * kAccStride;
-  const int nc = min(kRhsChunk, nrhs - c0);
-  for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+    const FrontDesc* __restrict__ fronts, const FrontState* __restrict__ st, SolvePlan pl, int task0, int ntasks,
+    int nchunks, int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0, double* __restrict__ X, int n) {
+  extern __shared__ __align__(16) double ssm[];
+  double* Lb0 = ssm;
+  double* xb = Lb0 + 2 * kRB * kTS;
+  double* acc = xb + kRB * kXS;
+  for (int t = blockIdx.x; t < ntasks * nchunks; t += gridDim.x) {
     if (ld_acquire(err) != 0) return;
-    const int4 tk = tasks[task];
+    const int chunk = t % nchunks, cc0 = c0 + chunk * kRhsChunk, nc = min(kRhsChunk, nrhs - cc0);
+    const int4 tk = pl.bwd_tasks[task0 + t / nchunks];
+    int* flags = pl.flags + static_cast<int64_t>(chunk) * pl.nflags;
+    int* counters = pl.counters + static_cast<int64_t>(chunk) * pl.nfronts;
+    int* hflags = pl.hflags + static_cast<int64_t>(chunk) * pl.nslots;
+    double* hscratch = pl.hscratch + static_cast<int64_t>(chunk) * pl.nslots * kRB * kRhsChunk;
+    if (tk.y == -2) {
+      const int w = threadIdx.x >> 5;
+      const bool ok = w >= tk.z || backward_tiny(fronts, st, pl.tiny[tk.x + w], pl, counters, err, wait_ns, nc, cc0, X, n);
+      if (__syncthreads_or(!ok)) return;
+      continue;
+    }
     const int s = tk.x;
     const int m = fronts[s].m, np = st[s].npiv;
-    const int nanc = (m - np + kRB - 1) / kRB;
+    const int nanc = ancestor_chunks(m, np);
     if (tk.y < 0) {
       const int nbp = (np + kRB - 1) / kRB;
       for (int cb = nbp - 1; cb >= 0; --cb)
-        if (!backward_block(fronts, st, s, cb, false, 0, nanc, 0, 0, flag_base, flags, hflags, hscratch, epoch, err,
-                            wait_ns, nc, c0, X, n, acc, xb, Lb0))
+        if (!backward_block(fronts, st, s, cb, false, 0, nanc, 0, 0, pl, flags, hflags, hscratch, counters, epoch, err,
+                            wait_ns, nc, cc0, X, n, acc, xb, Lb0))
           return;
     } else {
       const int P = tk.w >> 20, slot = tk.w & ((1 << 20) - 1), p = tk.z;
       const int a0 = static_cast<int>(static_cast<long long>(nanc) * p / P);
       const int a1 = static_cast<int>(static_cast<long long>(nanc) * (p + 1) / P);
-      if (!backward_block(fronts, st, s, tk.y, p > 0, a0, a1, slot, p > 0 ? 1 : P - 1, flag_base, flags, hflags,
-                          hscratch, epoch, err, wait_ns, nc, c0, X, n, acc, xb, Lb0))
+      if (!backward_block(fronts, st, s, tk.y, p > 0, a0, a1, slot, p > 0 ? 1 : P - 1, pl, flags, hflags, hscratch,
+                          counters, epoch, err, wait_ns, nc, cc0, X, n, acc, xb, Lb0))
         return;
     }
   }
@@ -683,6 +914,8 @@ inline unsigned grid_for(long long work, int threads) {
 
 int solve_block_rows() { return kRB; }
 int solve_rhs_chunk() { return kRhsChunk; }
+int solve_tiny_rows() { return kTinyRows; }
+int solve_ancestor_chunks(int m, int np) { return ancestor_chunks(m, np); }
 
 cudaError_t solve_max_resident(int device, int* fwd_ctas, int* bwd_ctas) {
   int sms = 0, a = 0, b = 0;
@@ -704,25 +937,23 @@ cudaError_t solve_max_resident(int device, int* fwd_ctas, int* bwd_ctas) {
 }
 
 cudaError_t launch_forward_pipelined(const FrontDesc* fronts, const ChildLink* links, const FrontState* st,
-                                     const int4* tasks, int ntasks, int grid, const int* flag_base, int* flags,
-                                     int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0,
-                                     const double* Bp, int n, cudaStream_t stream) {
+                                     const SolvePlan& p, int task0, int ntasks, int nchunks, int grid, int epoch,
+                                     int* err, unsigned long long wait_ns, int nrhs, int c0, const double* Bp, int n,
+                                     cudaStream_t stream) {
   if (ntasks <= 0) return cudaSuccess;
-  void* args[] = {(void*)&fronts, (void*)&links, (void*)&st,  (void*)&tasks, (void*)&ntasks,
-                  (void*)&flag_base, (void*)&flags, (void*)&epoch, (void*)&err, (void*)&wait_ns,
-                  (void*)&nrhs, (void*)&c0,     (void*)&Bp,    (void*)&n};
+  void* args[] = {(void*)&fronts, (void*)&links, (void*)&st, (void*)&p, (void*)&task0, (void*)&ntasks, (void*)&nchunks,
+                  (void*)&epoch, (void*)&err, (void*)&wait_ns, (void*)&nrhs, (void*)&c0, (void*)&Bp, (void*)&n};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(forward_pipelined_kernel), dim3(grid), dim3(kST),
                                      args, kSolveSmem, stream);
 }
 
-cudaError_t launch_backward_pipelined(const FrontDesc* fronts, const FrontState* st, const int4* tasks, int ntasks,
-                                      int grid, const int* flag_base, int* flags, int* hflags, double* hscratch,
-                                      int epoch, int* err, unsigned long long wait_ns, int nrhs, int c0, double* X,
-                                      int n, cudaStream_t stream) {
+cudaError_t launch_backward_pipelined(const FrontDesc* fronts, const FrontState* st, const SolvePlan& p, int task0,
+                                      int ntasks, int nchunks, int grid, int epoch, int* err,
+                                      unsigned long long wait_ns, int nrhs, int c0, double* X, int n,
+                                      cudaStream_t stream) {
   if (ntasks <= 0) return cudaSuccess;
-  void* args[] = {(void*)&fronts, (void*)&st,    (void*)&tasks, (void*)&ntasks, (void*)&flag_base,
-                  (void*)&flags,  (void*)&hflags, (void*)&hscratch, (void*)&epoch, (void*)&err,
-                  (void*)&wait_ns, (void*)&nrhs,   (void*)&c0,    (void*)&X,     (void*)&n};
+  void* args[] = {(void*)&fronts, (void*)&st, (void*)&p, (void*)&task0, (void*)&ntasks, (void*)&nchunks, (void*)&epoch,
+                  (void*)&err, (void*)&wait_ns, (void*)&nrhs, (void*)&c0, (void*)&X, (void*)&n};
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(backward_pipelined_kernel), dim3(grid), dim3(kST),
                                      args, kSolveSmem, stream);
 }
