@@ -11,12 +11,11 @@ constexpr int kPanelMax = 32;    // pivots per panel
 constexpr int kBlkStride = 34;   // even: pairs of a row are one 16-byte load
 
 // The diagonal block in shared memory. In: db's lower triangle, the block's
-// current values. Out: L below the diagonal of db (d on it) and, transposed,
-// above the diagonal of dt; wv[i][c] = the current value of row i in column c
-// before scaling, d_c L(i, c); d, 1 / d and the applied perturbation.
+// current values. Out: L below the diagonal of db (d on it); wv[i][c] = the
+// current value of row i in column c before scaling, d_c L(i, c); d, 1 / d and
+// the applied perturbation.
 struct alignas(16) DiagBlock {
   double db[kPanelMax][kBlkStride];
-  double dt[kPanelMax][kBlkStride];
   double wv[kPanelMax][kBlkStride];
   double dv[kPanelMax], iv[kPanelMax], pv[kPanelMax];
 };
@@ -43,18 +42,31 @@ __device__ __forceinline__ double pivot_reciprocal(double d) {
   return fma(r, e, r);
 }
 
+// a / d from 1 / d with one residual step. a times the rounded 1 / d alone
+// would be off by the same relative error in the whole column, and the updates
+// (which take L D as the values before the division) would carry it into the
+// whole Schur complement.
+__device__ __forceinline__ double pivot_quotient(double a, double d, double inv) {
+  const double q = a * inv;
+  return fma(fma(-q, d, a), inv, q);
+}
+
 // LDL^T of the np x np block by one warp, lane = row, in steps of eight
 // columns: the step's columns of the lane's row are brought up to date from
 // the earlier steps (left-looking, the row's values in registers, eight
 // independent sums), then every lane factors the 8 x 8 diagonal block
 // redundantly in registers while it eliminates its own row. No shuffle, and
-// three warp barriers per step instead of two per column. Entries past np are
-// garbage of which no row or column below np depends.
+// three warp barriers per step instead of two per column. Products are summed
+// apart and subtracted from an entry once per step: subtracting them one by
+// one would round each time at the size of the entry, which on a diagonally
+// heavy matrix is far above that of the sum. Entries past np are garbage of
+// which no row or column below np depends.
 //
 // What bounds it is the chain of 32 reciprocals, each followed by the update of the
 // next pivot (one warp, 255 registers allowed). Column by column, with the
 // row in shared memory, a column took 890 cycles (14 us per block); now it
-// takes 250 (4.1 us).
+// takes about 260 (keeping the sums apart costs the 64^3 stencil's panels 0.4
+// of 32.4 ms, the quotients' residual step 0.9).
 template <bool Static>
 __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane, int lane_sign, double floorv,
                                                   double delta) {
@@ -62,58 +74,67 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
 #pragma unroll
   for (int j0 = 0; j0 < kPanelMax; j0 += 8) {
     if (j0 >= np) break;
-    double x[8];
+    double x[8], xs[8];  // the lane's row: values at the step's start, the step's sums
 #pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-      const double2 v = *reinterpret_cast<const double2*>(&B.db[lane][j0 + c]);
-      x[c] = v.x;
-      x[c + 1] = v.y;
-    }
+    for (int c = 0; c < 8; ++c) xs[c] = 0.0;
 #pragma unroll
     for (int t = 0; t < j0; t += 2)
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const double2 l = *reinterpret_cast<const double2*>(&B.db[j0 + c][t]);
-        x[c] = fma(-a[t], l.x, x[c]);
-        x[c] = fma(-a[t + 1], l.y, x[c]);
+        xs[c] = fma(a[t], l.x, xs[c]);
+        xs[c] = fma(a[t + 1], l.y, xs[c]);
       }
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(&B.db[lane][j0 + c]);
+      x[c] = v.x - xs[c];
+      x[c + 1] = v.y - xs[c + 1];
+      xs[c] = xs[c + 1] = 0.0;
+    }
     if (lane >= j0 && lane < j0 + 8)
 #pragma unroll
       for (int c = 0; c < 8; ++c) B.db[lane][j0 + c] = x[c];
     __syncwarp();
-    double T[8][8];
+    double U[8][8];  // sums of the 8 x 8 block's entries
+    double T[8];     // the pivot column's values
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < 8; ++r) {
+      T[r] = B.db[j0 + r][j0];
 #pragma unroll
-      for (int c = 0; c <= r; ++c) T[r][c] = B.db[j0 + r][j0 + c];
-    __syncwarp();
+      for (int c = 0; c <= r; ++c) U[r][c] = 0.0;
+    }
     int sign[8];
     if (Static)
 #pragma unroll
       for (int c = 0; c < 8; ++c) sign[c] = __shfl_sync(0xffffffffu, lane_sign, j0 + c);
+    __syncwarp();
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const int col = j0 + c;
-      const double akk = T[c][c];
+      double next[8];  // the next column's values at the step's start
+#pragma unroll
+      for (int r = c + 1; r < 8; ++r) next[r] = B.db[j0 + r][col + 1];
+      const double akk = T[c];
       double d = akk;
       if (Static) d = static_pivot(akk, sign[c], floorv, delta);
       const double inv = pivot_reciprocal(d);
       double l[8];
 #pragma unroll
-      for (int r = c + 1; r < 8; ++r) l[r] = T[r][c] * inv;
+      for (int r = c + 1; r < 8; ++r) l[r] = pivot_quotient(T[r], d, inv);
 #pragma unroll
       for (int r2 = c + 1; r2 < 8; ++r2)
 #pragma unroll
-        for (int r = r2; r < 8; ++r) T[r][r2] = fma(-T[r][c], l[r2], T[r][r2]);
-      const double v = x[c];
+        for (int r = r2; r < 8; ++r) U[r][r2] = fma(T[r], l[r2], U[r][r2]);
+      const double v = x[c] - xs[c];
       a[col] = v;
 #pragma unroll
-      for (int c2 = c + 1; c2 < 8; ++c2) x[c2] = fma(-v, l[c2], x[c2]);
-      // every lane stores: what lands on the other side of the diagonal is
-      // not read
-      const double li = v * inv;
+      for (int c2 = c + 1; c2 < 8; ++c2) xs[c2] = fma(v, l[c2], xs[c2]);
+#pragma unroll
+      for (int r = c + 1; r < 8; ++r) T[r] = next[r] - U[r][c + 1];
+      // every lane stores: what lands above the diagonal is not read
+      const double li = pivot_quotient(v, d, inv);
       B.db[lane][col] = lane == col ? d : li;
-      B.dt[col][lane] = li;
       B.wv[lane][col] = v;
       B.dv[col] = d;
       B.iv[col] = inv;
@@ -123,22 +144,29 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
   }
 }
 
-// A row below the block: a[t] becomes the row's current value in column t
-// (right-looking: a_c -= a_t L(c, t); L = a / d). Columns past np are computed
-// on garbage and not used. The loads of L are warp-uniform pairs. (Two rows
-// per thread would halve them, but leave no registers to load ahead with: the
-// pass then waits for every pair and took 10 us instead of 2.)
+// A row below the block: a[c] becomes the row's current value in column c,
+// the raw one minus sum_t a_t L(c, t) (L = a / d), the sum formed apart in
+// four parts. Columns past np are computed on garbage and not used. The loads
+// of L are warp-uniform pairs. (Two rows per thread would halve them, but
+// leave no registers to load ahead with: the pass then waits for every pair
+// and took 10 us instead of 2.)
 __device__ __forceinline__ void panel_row(const DiagBlock& B, int np, double (&a)[kPanelMax]) {
 #pragma unroll
-  for (int t = 0; t < kPanelMax - 1; ++t) {
-    if ((t & 7) == 0 && t >= np) break;
-    if (!(t & 1)) a[t + 1] = fma(-a[t], B.dt[t][t + 1], a[t + 1]);
+  for (int c = 1; c < kPanelMax; ++c) {
+    if ((c & 7) == 0 && c >= np) break;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
-    for (int c = (t + 2) & ~1; c < kPanelMax; c += 2) {
-      const double2 l = *reinterpret_cast<const double2*>(&B.dt[t][c]);
-      a[c] = fma(-a[t], l.x, a[c]);
-      a[c + 1] = fma(-a[t], l.y, a[c + 1]);
+    for (int t = 0; t < c; t += 2) {
+      const double2 l = *reinterpret_cast<const double2*>(&B.db[c][t]);
+      if (t & 2) {
+        s2 = fma(a[t], l.x, s2);
+        if (t + 1 < c) s3 = fma(a[t + 1], l.y, s3);
+      } else {
+        s0 = fma(a[t], l.x, s0);
+        if (t + 1 < c) s1 = fma(a[t + 1], l.y, s1);
+      }
     }
+    a[c] -= (s0 + s1) + (s2 + s3);
   }
 }
 
@@ -165,7 +193,7 @@ __device__ __forceinline__ unsigned long long warp_column_max(const double (&a)[
 
 // A row's L = a / d and -(L D) = -a in the packed operands (p: pivot q0 of the
 // row), and put(c, l) for every column c < np: eight columns at a time, so
-// that the loads of 1 / d do not wait for the stores before them.
+// that the loads of d and 1 / d do not wait for the stores before them.
 template <class Put>
 __device__ __forceinline__ void store_panel_row(const DiagBlock& B, int np, const double (&a)[kPanelMax], double* P,
                                                 int64_t pw, int prt, int q0, int i, Put&& put) {
@@ -178,8 +206,9 @@ __device__ __forceinline__ void store_panel_row(const DiagBlock& B, int np, cons
 #pragma unroll
     for (int c = 0; c < 8; c += 2) {
       const double2 iv = *reinterpret_cast<const double2*>(&B.iv[c0 + c]);
-      l[c] = a[c0 + c] * iv.x;
-      l[c + 1] = a[c0 + c + 1] * iv.y;
+      const double2 dv = *reinterpret_cast<const double2*>(&B.dv[c0 + c]);
+      l[c] = pivot_quotient(a[c0 + c], dv.x, iv.x);
+      l[c + 1] = pivot_quotient(a[c0 + c + 1], dv.y, iv.y);
     }
 #pragma unroll
     for (int c = 0; c < 8; ++c) {

@@ -31,9 +31,9 @@
 // accepted (identical values and decisions to the sequential path), and
 // the same launch finishes the panel on the sequential path from the first
 // failing pivot (measured: cheaper than a new panel + update launch pair).
-// A 32-pivot panel of 4096 rows accepted whole takes 23 us (33 us when the
+// A 32-pivot panel of 4096 rows accepted whole takes 24 us (33 us when the
 // block was factored column by column and the rows went through shared memory
-// once more for the maxima and for L), of which the block's chain is 4.1, the
+// once more for the maxima and for L), of which the block's chain is about 4, the
 // row pass 5.6, the exchange of the maxima 1.7, the stores of L 2.3 us.
 #include <cooperative_groups.h>
 
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     for (int t = threadIdx.x; t <= p; t += kCT) {
       double v;
       if (t == p) {
-        v = d * (vk1 * (1.0 / d));
+        v = vk1;
       } else {
         const int kind = sh.pk[t];
         if (kind == 0)
@@ -362,12 +362,12 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     else
       ++n_zero;
     thread_rmax = fmax(thread_rmax, fabs(d));
-    const double inv = 1.0 / d;
+    const double inv = pivot_reciprocal(d);
     for (int i = max(base, k + 1) + threadIdx.x; i < rend; i += kCT) {
       const int li = i - base;
       const double a = col[li];
       thread_rmax = fmax(thread_rmax, fabs(a));
-      const double l = a * inv;
+      const double l = pivot_quotient(a, d, inv);
       Lr[p * R + li] = l;
       F[k * ld + i] = l;
       put_packed(k, i, l, a);
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
           for (int c = 0; c < kSpecMax; c += 2)
             if (c < np) {
               const double2 wc = *reinterpret_cast<const double2*>(w + c);
-              a[c] = fma(-l, wc.x, a[c]);
+              a[c] = fma(-l, wc.x, a[c]);  // (a restart's few earlier pivots)
               a[c + 1] = fma(-l, wc.y, a[c + 1]);
             }
         }
