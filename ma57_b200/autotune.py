@@ -1,8 +1,6 @@
 """Front-size-to-tile-shape schedule chosen by measurement.
 
-Three launch shapes depend on front size and have no single best value:
-the width of the small-front kernel (a warp per front for fronts of at most
-32 rows, or 128 or 256 threads per front), the
+Two launch shapes depend on front size and have no single best value: the
 number of CTAs in the panel cluster of the large fronts (2, 4, 8 or 16; more
 CTAs hold fewer rows each but occupy more SMs; or 1, the single-CTA panel
 kernel, whose pivot-by-pivot decisions need no cluster barriers) and the
@@ -23,7 +21,6 @@ import math
 
 from . import _lib as L
 
-SMALL_BUCKETS = (48, 128)                    # small-front kernel, by the level's largest small front
 LARGE_BUCKETS = (512, 2048, 8192, 1 << 30)  # panel cluster, by the level's largest large front
 
 
@@ -51,15 +48,15 @@ def _bucket(value, edges):
 
 
 def apply(solver, schedule):
-    """schedule: {"small": {bucket: threads}, "large": {bucket: ctas},
-    "update": {bucket: tile rows}} (missing entries: the default shape)."""
+    """schedule: {"small": {}, "large": {bucket: ctas}, "update": {bucket:
+    tile rows}} (missing entries: the default shape; small fronts take their
+    kernel by size)."""
     lib = L.load()
     for lv, info in enumerate(level_info(solver)):
-        st = schedule["small"].get(_bucket(info["small_max_m"], SMALL_BUCKETS), 0) if info["small"] else 0
         lb = _bucket(info["large_max_m"], LARGE_BUCKETS)
         cl = schedule["large"].get(lb, 0) if info["large"] else 0
         ur = schedule.get("update", {}).get(lb, 0) if info["large"] else 0
-        if lib.symla_gpu_set_level_schedule(solver._ctx.h, lv, st, cl) != L.SYMLA_OK:
+        if lib.symla_gpu_set_level_schedule(solver._ctx.h, lv, 0, cl) != L.SYMLA_OK:
             raise RuntimeError(L.last_error())
         if lib.symla_gpu_set_level_update_rows(solver._ctx.h, lv, ur) != L.SYMLA_OK:
             raise RuntimeError(L.last_error())
@@ -78,14 +75,12 @@ def tune(solver, A, reps: int = 2):
     pattern of A must be analyzed and factorized once). Returns the chosen
     schedule (installed) and the measured default / tuned factorization ms."""
     info = level_info(solver)
-    small_b = sorted({_bucket(i["small_max_m"], SMALL_BUCKETS) for i in info if i["small"]})
     large_b = sorted({_bucket(i["large_max_m"], LARGE_BUCKETS) for i in info if i["large"]})
     schedule = {"small": {}, "large": {}, "update": {}}
     apply(solver, schedule)
     base = _factor_ms(solver, A, reps)
     best = base
-    for kind, buckets, cands in (("small", small_b, (32, 128, 256)), ("large", large_b, (1, 2, 4, 8, 16)),
-                                 ("update", large_b, (64, 128))):
+    for kind, buckets, cands in (("large", large_b, (1, 2, 4, 8, 16)), ("update", large_b, (64, 128))):
         for b in buckets:
             for cand in cands:
                 trial = {k: dict(v) for k, v in schedule.items()}

@@ -24,7 +24,7 @@ NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 HOST_SRCS = ["host/symbolic.cpp", "host/amd.cpp", "host/metis_order.cpp"]
-CUDA_SRCS = ["gpu/capi.cu", "gpu/factor_kernels.cu", "gpu/solve_kernels.cu", "gpu/panel_cluster.cu", "gpu/panel_static.cu", "gpu/schur_tc.cu", "gpu/noalloc.cu", "gpu/mlp.cu"]
+CUDA_SRCS = ["gpu/capi.cu", "gpu/factor_kernels.cu", "gpu/solve_kernels.cu", "gpu/panel_cluster.cu", "gpu/panel_static.cu", "gpu/panel_shared.cu", "gpu/small_front.cu", "gpu/schur_tc.cu", "gpu/noalloc.cu", "gpu/mlp.cu"]
 # benchmark tooling, its own library (bench.py loads it; not part of the C ABI)
 BENCH_SRC = "bench/fp64_peak.cu"
 BENCH_LIB = LIBDIR / "libsymla_bench.so"

@@ -252,6 +252,12 @@ void build_maps(const std::vector<int>& cbRows, const std::unordered_map<int, in
   }
 }
 
+// Fewest warp-sized fronts that get a launch of their own in a level with
+// larger small fronts: below that a CTA each is at most a few waves and done
+// sooner (a level of 141 fronts of up to 57 rows takes 0.16 ms with the two
+// launches, about 0.1 with one; of 8866 of up to 86 rows 0.38, and 0.5 as CTAs).
+constexpr int kWarpFrontsMin = 1024;
+
 // The children (offsets) of a front with a row in each 32-column block, from
 // their extend-add maps: rel(t) points at child t's map to the front's rows,
 // cb(t) entries.
@@ -372,6 +378,17 @@ void build_level_lists(symla_gpu_ctx* c, const std::vector<int>& frontsOfLevel, 
       tiles = std::max(tiles, nt * (nt + 1) / 2);
     }
   }
+  // small fronts: those a warp can take first, the others by size, the largest
+  // first (the level ends with its last CTA)
+  std::stable_sort(L.small.begin(), L.small.end(), [&](int a, int b) {
+    const int ma = c->fronts[a].m, mb = c->fronts[b].m;
+    const bool wa = ma <= kWarpFrontMax, wb = mb <= kWarpFrontMax;
+    return wa != wb ? wa : (!wa && ma > mb);
+  });
+  L.small_warp = static_cast<int>(std::count_if(L.small.begin(), L.small.end(),
+                                                [&](int s) { return c->fronts[s].m <= kWarpFrontMax; }));
+  // a few of them are not worth a launch of their own beside the others'
+  if (L.small_warp < kWarpFrontsMin && L.small_warp < static_cast<int>(L.small.size())) L.small_warp = 0;
   if (!L.large.empty()) {
     // one grid over the tiles of every front of the level, in 128 x 128
     // tiles up to one per SM (the update launchers double it: 128 x 64 tiles,
@@ -895,7 +912,7 @@ void validate_tables(symla_gpu_ctx* c, int phase, const KernelOpts& ko, const ch
 
 // Default choice of the single-CTA panel kernel (see launch_panel_iteration).
 constexpr int kSinglePanelMaxFronts = 148;
-constexpr int kSinglePanelMaxM = 1024;
+constexpr int kSinglePanelMaxM = kPanelSharedRows;
 
 // Static pivoting runs its own panel kernel unless the single-CTA one is
 // asked for.
@@ -911,9 +928,13 @@ void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, co
   timed(c, SYMLA_KERNEL_PANEL, 0.0, 0.0, [&] {
     // the single-CTA panel when asked for (cluster size 1) or, by default in
     // threshold (Bunch-Kaufman) mode, for levels of fewer large fronts than
-    // SMs none taller than kSinglePanelMaxM rows: there the cluster's
-    // barriers on every pivot-by-pivot decision cost more than its spread of
-    // rows saves. Static pivoting has its own kernel.
+    // SMs none taller than kSinglePanelMaxM rows, those whose panel fits one
+    // CTA's shared memory: there the cluster's barriers on every
+    // pivot-by-pivot decision cost more than its spread of rows saves (per
+    // level of a 20^3 7-point grid it is 0.1 to 2 ms slower, of a 27^3
+    // 27-point one, whose pivots mostly pass the first test, 0.06 ms faster to
+    // 0.1 slower; at 898 rows 0.4 ms faster). Static pivoting has its own
+    // kernel.
     const bool single = L.cluster_ctas == 1 || (L.cluster_ctas == 0 && ko.mode == SYMLA_MODE_THRESHOLD &&
                                                 nl < kSinglePanelMaxFronts && L.large_max_m <= kSinglePanelMaxM);
     if (use_static_panel(c, L, ko)) {
@@ -922,6 +943,9 @@ void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, co
     } else if (c->use_cluster_panel && !single && cluster_size_for(L.large_max_m, nl, L.panel_width) > 0) {
       CK(launch_cluster_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, L.panel_width, ko, c->d_glob, level,
                               dynamic, st, L.cluster_ctas));
+    } else if (L.large_max_m <= kPanelSharedRows) {
+      CK(launch_shared_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, L.panel_width, ko, c->d_glob, level,
+                             dynamic, st));
     } else {
       // fronts too tall for shared memory keep their two working columns in
       // a global buffer (allocated with the level's lists)
@@ -974,8 +998,13 @@ void launch_level_planned(symla_gpu_ctx* c, const LevelLists& L, int level, cons
   c->cur_level = level;
   if (!L.small.empty())
     timed(c, SYMLA_KERNEL_SMALL, L.small_flops, 0.0, [&] {
-      launch_factor_small(c->d_desc, c->d_links, c->d_state, d_small, static_cast<int>(L.small.size()),
-                          L.small_max_m, c->d_a_colptr, ko, c->d_glob, level, dynamic, st, L.small_threads);
+      const int ns = static_cast<int>(L.small.size());
+      const int nw = L.small_warp;
+      launch_factor_small(c->d_desc, c->d_links, c->d_state, d_small, nw, c->d_a_colptr, ko, c->d_glob, level, dynamic,
+                          st);
+      if (nw > 0 && ns > nw) ++c->launches;
+      launch_small_front(c->d_desc, c->d_links, c->d_state, d_small + nw, ns - nw, L.small_max_m, c->d_a_colptr, ko,
+                         c->d_glob, level, dynamic, st);
     });
   if (!L.large.empty()) {
     timed(c, SYMLA_KERNEL_ASSEMBLE, 0.0, L.assemble_bytes, [&] {
@@ -1747,6 +1776,8 @@ extern "C" int symla_gpu_create(const symla_symbolic* sym, int n, const int* col
     if (!configured[device]) {
       CK(configure_factor_kernels());
       CK(configure_cluster_panel());
+      CK(configure_shared_panel());
+      CK(configure_small_front());
       CK(configure_tc_far());
       configured[device] = true;
     }

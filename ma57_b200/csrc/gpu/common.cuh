@@ -169,4 +169,14 @@ struct KernelOpts {
   CheckWord* chk;               // status word of the bounds checks (checked build)
 };
 
+// A stored entry e of the front's own columns: (local column, local row,
+// value index), or false (checked build) when it lies outside the front.
+__device__ __forceinline__ bool a_entry(const KernelOpts& o, const FrontDesc& f, int e, int& j, int& i, int& idx) {
+  j = o.a_j[e];
+  const int pos = o.a_pos[e];
+  idx = o.a_idx[e];
+  i = pos < f.ncols ? pos : pos + f.nextra;
+  return check(a_entry_ok(j, pos, idx, f.ncols, f.nextra, f.m, o.nnz), o.chk, kChkAEntry, e);
+}
+
 }  // namespace symla_gpu

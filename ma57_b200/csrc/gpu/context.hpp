@@ -34,9 +34,10 @@ struct HostFront {
 struct LevelLists {
   std::vector<int> small;      // fronts with m <= kSmallFrontMax
   int small_max_m = 0;
+  int small_warp = 0;          // of them, the first so many (m <= kWarpFrontMax) take a warp each
   std::vector<int> large;      // other fronts
   int large_max_m = 0;
-  int small_threads = 0;       // tile schedule (autotuner): small-front kernel width, 0 = by size
+  int small_threads = 0;       // tile schedule: kept and reported, the kernel goes by front size
   int cluster_ctas = 0;        // panel cluster size, 0 = by size
   int update_rows = 0;         // rows per Schur-update tile (64 or 128), 0 = 128
   int panels = 0;              // panel iterations needed (threshold pivoting)

@@ -54,16 +54,6 @@ __device__ __forceinline__ double gather_children(const FrontDesc* fronts, const
   return v;
 }
 
-// A stored entry e of the front's own columns: (local column, local row,
-// value index), or false (checked build) when it lies outside the front.
-__device__ __forceinline__ bool a_entry(const KernelOpts& o, const FrontDesc& f, int e, int& j, int& i, int& idx) {
-  j = o.a_j[e];
-  const int pos = o.a_pos[e];
-  idx = o.a_idx[e];
-  i = pos < f.ncols ? pos : pos + f.nextra;
-  return check(a_entry_ok(j, pos, idx, f.ncols, f.nextra, f.m, o.nnz), o.chk, kChkAEntry, e);
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -210,18 +200,17 @@ __global__ void __launch_bounds__(256, 4) assemble_kernel(const FrontDesc* __res
 }
 
 // ---------------------------------------------------------------------------
-// Small fronts: one CTA per front, the whole front in shared memory
-// (assembly, factorization and write-back in one launch).
+// Fronts of at most 32 rows: one warp per front, kWarpFronts per CTA, the
+// whole front in shared memory (assembly, factorization and write-back in one
+// launch; warp barriers and shuffle reductions only). Larger small fronts:
+// small_front.cu.
 namespace {
 
-// Warp mode of the small-front kernel: fronts of at most kWarpFrontMax rows,
-// kWarpFronts per CTA, each in a fixed slice of kWarpFrontDoubles of the
-// dynamic shared memory (the m x (m | 1) front plus its two index arrays).
-constexpr int kWarpFrontMax = 32;
+// A front has a fixed slice of kWarpFrontDoubles of the dynamic shared memory
+// (the m x (m | 1) front plus its two index arrays).
 constexpr int kWarpFronts = 8;
 constexpr int kWarpFrontDoubles = kWarpFrontMax * (kWarpFrontMax | 1) + kWarpFrontMax;
 
-template <int NT>
 struct SmallFront {
   double* S;
   int lds;
@@ -232,7 +221,7 @@ struct SmallFront {
 };
 
 // Calls fn(i, j) once for every entry i >= j of a t x t lower triangle,
-// spread over the CTA's NT threads. The triangle is folded into a
+// spread over a warp. The triangle is folded into a
 // (t + 1) x ceil(t / 2) rectangle: rectangle column c holds triangle column
 // c (rows c..t-1) in its rows c..t-1 and triangle column t-1-c in the rest
 // (rows 0..c-1 -> triangle rows t-c..t-1, row t -> the diagonal), the middle
@@ -241,8 +230,9 @@ struct SmallFront {
 // conflicts), and each thread's position advances by a precomputed step, so
 // there is one integer division per call instead of one per entry, and no
 // thread idles on the upper half.
-template <int NT, class Fn>
+template <class Fn>
 __device__ __forceinline__ void for_lower(int t, int tid, Fn&& fn) {
+  constexpr int NT = 32;
   const int R = t + 1, C = (t + 1) >> 1;
   int q = tid % R, c = tid / R;  // position c R + q, advancing by NT
   const int dq = NT % R, dc = NT / R;
@@ -262,36 +252,10 @@ __device__ __forceinline__ void for_lower(int t, int tid, Fn&& fn) {
   }
 }
 
-// The threads that factor one small front: the whole CTA (NT = 128 or 256)
-// or one warp (NT = 32; the CTA then holds kWarpFronts fronts, one per
-// warp, and no block-wide barrier is used).
-template <int NT>
-__device__ __forceinline__ void grp_sync() {
-  if constexpr (NT == 32)
-    __syncwarp();
-  else
-    __syncthreads();
-}
-template <int NT>
-__device__ __forceinline__ ArgMax grp_argmax(ArgMax a, double* sv, int* si) {
-  if constexpr (NT == 32)
-    return warp_argmax(a);
-  else
-    return block_argmax<NT>(a, sv, si);
-}
-template <int NT>
-__device__ __forceinline__ double grp_max(double v, double* sv) {
-  if constexpr (NT == 32)
-    return warp_max(v);
-  else
-    return block_max<NT>(v, sv);
-}
-
 // Symmetric swap of positions i < j in lower storage over the whole front.
-template <int NT>
-__device__ void smem_swap(SmallFront<NT>& F, int* fi, int* lp, int i, int j, int tid) {
+__device__ void smem_swap(SmallFront& F, int* fi, int* lp, int i, int j, int tid) {
   const int m = F.m;
-  for (int t = tid; t < m - 1; t += NT) {
+  for (int t = tid; t < m - 1; t += 32) {
     if (t < i) {  // row swap in columns c < i
       const int c = t;
       double a = F.at(i, c);
@@ -321,44 +285,42 @@ __device__ void smem_swap(SmallFront<NT>& F, int* fi, int* lp, int i, int j, int
     lp[i] = lp[j];
     lp[j] = a;
   }
-  grp_sync<NT>();
+  __syncwarp();
 }
 
 }  // namespace
 
-template <int NT>
-__global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
+__global__ void __launch_bounds__(32 * kWarpFronts)
     factor_small_kernel(const FrontDesc* __restrict__ fronts, const ChildLink* __restrict__ links, FrontState* st,
                         const int* __restrict__ front_list, int count, const int* __restrict__ a_colptr, KernelOpts o,
                         FactorGlobals* g, int level, int dynamic) {
   if (level_aborted(g, level, dynamic)) return;
   extern __shared__ double smem_all[];
-  __shared__ double red_v[NT / 32];
-  __shared__ int red_i[NT / 32];
-  // warp mode: warp w of the CTA factors list entry kWarpFronts blockIdx + w
-  // in its own slice of shared memory
-  const int tid = NT == 32 ? static_cast<int>(threadIdx.x & 31) : static_cast<int>(threadIdx.x);
-  const int grp = NT == 32 ? static_cast<int>(threadIdx.x >> 5) : 0;
-  const int entry = NT == 32 ? static_cast<int>(blockIdx.x) * kWarpFronts + grp : static_cast<int>(blockIdx.x);
-  if (entry >= count) return;  // (warp mode only: the whole warp leaves)
-  double* smem = smem_all + (NT == 32 ? static_cast<size_t>(grp) * kWarpFrontDoubles : 0);
+  constexpr int NT = 32;
+  // warp w of the CTA factors list entry kWarpFronts blockIdx + w in its own
+  // slice of shared memory
+  const int tid = static_cast<int>(threadIdx.x & 31);
+  const int grp = static_cast<int>(threadIdx.x >> 5);
+  const int entry = static_cast<int>(blockIdx.x) * kWarpFronts + grp;
+  if (entry >= count) return;  // the whole warp leaves
+  double* smem = smem_all + static_cast<size_t>(grp) * kWarpFrontDoubles;
 
   const int s = front_list[entry];
   const FrontDesc f = fronts[s];
   const int m = f.m;
-  SmallFront<NT> F{smem, m | 1, m};
+  SmallFront F{smem, m | 1, m};
   int* fi = reinterpret_cast<int*>(smem + static_cast<size_t>(F.lds) * m);
   int* lp = fi + m;  // local pivot permutation
 
   // ---- assembly (multifrontal.hpp:498-535), children summed in fixed order
-  for_lower<NT>(m, tid, [&](int i, int j) {
+  for_lower(m, tid, [&](int i, int j) {
     F.at(i, j) = gather_children(fronts, links, st, f.ch_begin, f.ch_end, i, j, o.chk);
   });
   for (int t = tid; t < m; t += NT) {
     fi[t] = f.fidx[t];
     lp[t] = t;
   }
-  grp_sync<NT>();
+  __syncwarp();
   {
     const int e0 = a_colptr[f.a_begin], e1 = a_colptr[f.a_begin + f.ncols];
     for (int e = e0 + tid; e < e1; e += NT) {
@@ -366,12 +328,12 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
       if (a_entry(o, f, e, j, i, idx)) F.at(i, j) += o.values[idx];
     }
   }
-  grp_sync<NT>();
+  __syncwarp();
 
   // ---- orig_max over the whole front (dense_kernel.hpp:413, :934)
   double tmax = 0.0;
-  for_lower<NT>(m, tid, [&](int i, int j) { tmax = fmax(tmax, fabs(F.at(i, j))); });
-  double orig_max = grp_max<NT>(tmax, red_v);
+  for_lower(m, tid, [&](int i, int j) { tmax = fmax(tmax, fabs(F.at(i, j))); });
+  double orig_max = warp_max(tmax);
   const bool isStatic = (o.mode == 1);
   if (isStatic) {
     if (orig_max < o.static_abs_floor) orig_max = 1.0;
@@ -420,7 +382,7 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         ++n_neg;
       else
         ++n_zero;
-      grp_sync<NT>();
+      __syncwarp();
       if (tid == 0) F.at(k, k) = d;
       thread_rmax = fmax(thread_rmax, fabs(d));
       for (int i = k + 1 + tid; i < m; i += NT) {
@@ -428,14 +390,14 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         thread_rmax = fmax(thread_rmax, fabs(a));
         F.at(i, k) = a / d;
       }
-      grp_sync<NT>();
-      for_lower<NT>(m - k - 1, tid, [&](int ii, int jj) {
+      __syncwarp();
+      for_lower(m - k - 1, tid, [&](int ii, int jj) {
         const int i = k + 1 + ii, j = k + 1 + jj;
         const double v = F.at(i, j) - (F.at(i, k) * d) * F.at(j, k);
         F.at(i, j) = v;
         thread_rmax = fmax(thread_rmax, fabs(v));
       });
-      grp_sync<NT>();
+      __syncwarp();
     }
     for (int t = tid; t < effEnd; t += NT) {
         f.Dd[t] = F.at(t, t);
@@ -450,7 +412,7 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         const double v = fabs(F.at(i, k));
         am = argmax_combine(am, ArgMax{v, i});
       }
-      am = grp_argmax<NT>(am, red_v, red_i);
+      am = warp_argmax(am);
       const double lambda = am.v;
       const int r = am.i;
       const double akk = F.at(k, k);
@@ -464,7 +426,7 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         double sm = 0.0;
         for (int i = k + tid; i < effEnd; i += NT)
           if (i != r) sm = fmax(sm, fabs(F.sym(i, r)));
-        const double sigma = grp_max<NT>(sm, red_v);
+        const double sigma = warp_max(sm);
         if (fabs(akk) * sigma >= kAlpha * lambda * lambda)
           dec = 0;
         else if (fabs(F.at(r, r)) >= kAlpha * sigma)
@@ -473,8 +435,8 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
           dec = 2;
       }
       if (dec == 3) break;
-      grp_sync<NT>();
-      if (dec == 1) smem_swap<NT>(F, fi, lp, k, r, tid);
+      __syncwarp();
+      if (dec == 1) smem_swap(F, fi, lp, k, r, tid);
       if (dec == 0 || dec == 1) {
         const double d = F.at(k, k);
         if (d > 0)
@@ -494,22 +456,22 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
           f.Do[k] = 0.0;
           f.pk[k] = 0;
         }
-        grp_sync<NT>();
-        for_lower<NT>(m - k - 1, tid, [&](int ii, int jj) {
+        __syncwarp();
+        for_lower(m - k - 1, tid, [&](int ii, int jj) {
           const int i = k + 1 + ii, j = k + 1 + jj;
           const double v = F.at(i, j) - (F.at(i, k) * d) * F.at(j, k);
           F.at(i, j) = v;
           thread_rmax = fmax(thread_rmax, fabs(v));
         });
-        grp_sync<NT>();
+        __syncwarp();
         k += 1;
         continue;
       }
       // 2x2 pivot
-      if (r != k + 1) smem_swap<NT>(F, fi, lp, k + 1, r, tid);
+      if (r != k + 1) smem_swap(F, fi, lp, k + 1, r, tid);
       const double d11 = F.at(k, k), d21 = F.at(k + 1, k), d22 = F.at(k + 1, k + 1);
       const double det = d11 * d22 - d21 * d21;
-      const double rm = fmax(orig_max, grp_max<NT>(thread_rmax, red_v));
+      const double rm = fmax(orig_max, warp_max(thread_rmax));
       const double rm1 = fmax(1.0, rm);
       if (fabs(det) <= o.zero_tol * rm1 * rm1) break;
       thread_rmax = fmax(thread_rmax, fmax(fabs(d11), fmax(fabs(d21), fabs(d22))));
@@ -542,8 +504,8 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         f.pk[k] = 1;
         f.pk[k + 1] = 2;
       }
-      grp_sync<NT>();
-      for_lower<NT>(m - k - 2, tid, [&](int ii, int jj) {
+      __syncwarp();
+      for_lower(m - k - 2, tid, [&](int ii, int jj) {
         const int i = k + 2 + ii, j = k + 2 + jj;
         const double l0i = F.at(i, k), l1i = F.at(i, k + 1);
         const double w0 = l0i * d11 + l1i * d21;
@@ -552,20 +514,20 @@ __global__ void __launch_bounds__(NT == 32 ? 32 * kWarpFronts : NT)
         F.at(i, j) = v;
         thread_rmax = fmax(thread_rmax, fabs(v));
       });
-      grp_sync<NT>();
+      __syncwarp();
       k += 2;
     }
   }
 
   // ---- write back (lower triangle of the whole front, permuted indices)
-  grp_sync<NT>();
-  for_lower<NT>(m, tid, [&](int i, int j) { f.F[static_cast<int64_t>(j) * f.ld + i] = F.at(i, j); });
+  __syncwarp();
+  for_lower(m, tid, [&](int i, int j) { f.F[static_cast<int64_t>(j) * f.ld + i] = F.at(i, j); });
   for (int t = tid; t < m; t += NT) {
     f.fidx[t] = fi[t];
     f.lperm[t] = lp[t];
     f.lpos[lp[t]] = t;
   }
-  const double rmax = grp_max<NT>(thread_rmax, red_v);
+  const double rmax = warp_max(thread_rmax);
     if (tid == 0) {
     FrontState& S = st[s];
     S.npiv = k;
@@ -1328,27 +1290,13 @@ void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState
   assemble_kernel<<<ntasks, 256, 0, stream>>>(fronts, links, st, tasks, touch, o, g, level, dynamic);
 }
 
-size_t small_front_smem(int m) {
-  return static_cast<size_t>(m | 1) * m * sizeof(double) + 2 * static_cast<size_t>(m) * sizeof(int) + 16;
-}
-
 void launch_factor_small(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* list, int count,
-                         int max_m, const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
-                         cudaStream_t stream, int threads) {
+                         const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
+                         cudaStream_t stream) {
   if (count <= 0) return;
-  const size_t sm = small_front_smem(max_m);
-  if (max_m <= kWarpFrontMax && (threads == 32 || threads == 0)) {
-    // one warp per front, kWarpFronts fronts per CTA
-    const int grid = (count + kWarpFronts - 1) / kWarpFronts;
-    factor_small_kernel<32><<<grid, 32 * kWarpFronts, kWarpFronts * kWarpFrontDoubles * sizeof(double), stream>>>(
-        fronts, links, st, list, count, a_colptr, o, g, level, dynamic);
-  } else if (threads == 128 || (threads != 256 && max_m <= 48)) {
-    factor_small_kernel<128><<<count, 128, sm, stream>>>(fronts, links, st, list, count, a_colptr, o, g, level,
-                                                          dynamic);
-  } else {
-    factor_small_kernel<256><<<count, 256, sm, stream>>>(fronts, links, st, list, count, a_colptr, o, g, level,
-                                                          dynamic);
-  }
+  const int grid = (count + kWarpFronts - 1) / kWarpFronts;
+  factor_small_kernel<<<grid, 32 * kWarpFronts, kWarpFronts * kWarpFrontDoubles * sizeof(double), stream>>>(
+      fronts, links, st, list, count, a_colptr, o, g, level, dynamic);
 }
 
 // Dynamic shared memory the single-CTA panel kernel is configured for.
@@ -1503,12 +1451,8 @@ void launch_validate_fronts(const FrontDesc* fronts, const ChildLink* links, con
 
 cudaError_t configure_factor_kernels() {
   cudaError_t e;
-  e = cudaFuncSetAttribute(factor_small_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(factor_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(kWarpFronts * kWarpFrontDoubles * sizeof(double)));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(factor_small_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(factor_small_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPanelSmemMax));
   if (e != cudaSuccess) return e;

@@ -25,15 +25,21 @@ struct AsmTask {
 };
 
 cudaError_t configure_factor_kernels();
-size_t small_front_smem(int m);
 
 void launch_assemble(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const AsmTask* tasks,
                      int ntasks, const int* touch, const KernelOpts& o, const FactorGlobals* g, int level, int dynamic,
                      cudaStream_t stream);
+// Fronts of at most kWarpFrontMax rows, a warp each
+constexpr int kWarpFrontMax = 32;
 void launch_factor_small(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* list, int count,
-                         int max_m, const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
-                         cudaStream_t stream, int threads = 0);  // threads: 32 (a warp per front, fronts of
-                                                                 // <= 32 rows), 128, 256, or 0 (by front size)
+                         const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
+                         cudaStream_t stream);
+// Fronts of at most kSmallFrontMax rows, a CTA each (small_front.cu)
+size_t small_front_smem(int m);
+cudaError_t configure_small_front();
+void launch_small_front(const FrontDesc* fronts, const ChildLink* links, FrontState* st, const int* list, int count,
+                        int max_m, const int* a_colptr, const KernelOpts& o, FactorGlobals* g, int level, int dynamic,
+                        cudaStream_t stream);
 // Single-CTA panel kernel. Its two working columns (2 m doubles per front)
 // live in shared memory when panel_fits_shared(max_m), else in `cols`
 // (device, 2 max_m doubles per front of the list), which is then required.
@@ -41,6 +47,12 @@ bool panel_fits_shared(int max_m);
 cudaError_t launch_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m, int nb,
                          const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream,
                          double* cols);
+// The same for fronts of at most kPanelSharedRows rows, with the panel's L (and
+// two working columns) in shared memory (panel_shared.cu).
+constexpr int kPanelSharedRows = 784;
+cudaError_t configure_shared_panel();
+cudaError_t launch_shared_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m, int nb,
+                                const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream);
 // Static pivoting (panel_static.cu): panels of kPanelWidth pivots whatever the
 // front's size.
 void launch_static_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m,

@@ -76,6 +76,19 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
   return __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(mh) << 32) | ml));
 }
 
+// Warp argmax of non-negative (value, index >= 0) pairs, or index -1 for none:
+// the largest value, among equals the smallest index (argmax_combine's rule),
+// by three 32-bit reductions.
+__device__ __forceinline__ ArgMax warp_argmax_nonneg(ArgMax a) {
+  const unsigned long long b = a.i >= 0 ? static_cast<unsigned long long>(__double_as_longlong(a.v)) : 0ull;
+  const unsigned hi = static_cast<unsigned>(b >> 32), lo = static_cast<unsigned>(b);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const unsigned mi = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? static_cast<unsigned>(a.i) : ~0u);
+  return ArgMax{__longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(mh) << 32) | ml)),
+                static_cast<int>(mi)};
+}
+
 // atomicMax for non-negative doubles (IEEE order == integer order there). A
 // NaN is kept (its pattern orders above +Inf), so a maximum over values that
 // include a NaN reads NaN instead of a finite number.

@@ -1,7 +1,7 @@
 """Panels of large fronts (one dense front, natural order). Static pivoting at
 the edges of the 32-pivot panels, the 96-row CTAs and the 256-pivot outer
 blocks, against the CPU oracle: inertia, perturbed pivots and residual.
-Threshold pivoting beyond the single-CTA panel's sizes."""
+Threshold pivoting on both sides of the single-CTA panel's range."""
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -56,10 +56,11 @@ def test_static_dense_front(n, weak):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [1025, 1057, 1288])
+@pytest.mark.parametrize("n", [129, 255, 256, 257, 512, 513, 784, 785, 1025, 1057, 1288])
 def test_threshold_dense_front(n):
-    """The cluster panel on a front whose pivots need interchanges and 2x2
-    blocks (runs that stop inside a panel and start again): inertia from the
+    """Fronts whose pivots need interchanges and 2x2 blocks, at the edges of
+    the single-CTA panel's two widths and of its range, and in the cluster
+    panel (runs that stop inside a panel and start again): inertia from the
     eigenvalues, backward error of a solve."""
     st = Stream(n)
     G = st.normal(n * n).reshape(n, n)
