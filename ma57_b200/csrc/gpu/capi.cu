@@ -788,9 +788,48 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   CK(cudaStreamSynchronize(c->stream));
 }
 
+// Device memory of the re-planned fronts of the current factorization, from
+// the context's pool (a cudaMalloc for each of a front's eight arrays was most
+// of a re-planned factorization's time).
+template <typename T>
+T* dyn_alloc(symla_gpu_ctx* c, size_t count) {
+  const size_t bytes = (std::max<size_t>(1, count) * sizeof(T) + 255) & ~static_cast<size_t>(255);
+  while (c->dyn_chunk < c->dyn_pool.size() && c->dyn_off + bytes > c->dyn_pool[c->dyn_chunk].second) {
+    ++c->dyn_chunk;
+    c->dyn_off = 0;
+  }
+  if (c->dyn_chunk == c->dyn_pool.size()) {
+    const size_t size = std::max({bytes, c->dyn_total, static_cast<size_t>(1) << 20});
+    c->dyn_pool.push_back({dalloc<char>(size), size});
+    c->dyn_off = 0;
+  }
+  char* p = c->dyn_pool[c->dyn_chunk].first + c->dyn_off;
+  c->dyn_off += bytes;
+  return reinterpret_cast<T*>(p);
+}
+
+template <typename T>
+T* dyn_upload(symla_gpu_ctx* c, const std::vector<T>& v) {
+  T* p = dyn_alloc<T>(c, v.size());
+  if (!v.empty()) CK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+  return p;
+}
+
+void free_dyn_pool(symla_gpu_ctx* c) {
+  for (auto& b : c->dyn_pool) dfree(b.first);
+  c->dyn_pool.clear();
+}
+
 void free_dynamic(symla_gpu_ctx* c) {
   for (void* p : c->dyn_allocs) dfree(p);
   c->dyn_allocs.clear();
+  if (c->dyn_pool.size() > 1) {
+    // one chunk of the total from the next factorization that needs it
+    c->dyn_total = 0;
+    for (auto& b : c->dyn_pool) c->dyn_total += b.second;
+    free_dyn_pool(c);
+  }
+  c->dyn_chunk = c->dyn_off = 0;
   c->dyn_front_blocks.clear();
 }
 
@@ -1176,21 +1215,14 @@ void replan_front(symla_gpu_ctx* c, int s) {
   for (int t = 0; t < f.m; ++t) g2l[frontIdx[t]] = t;
 
   FrontDesc d = c->hdesc[s];
-  double* F = dalloc<double>(static_cast<size_t>(f.ld) * f.m);
-  c->dyn_allocs.push_back(F);
+  double* F = dyn_alloc<double>(c, static_cast<size_t>(f.ld) * f.m);
   c->dyn_front_blocks.push_back({F, static_cast<size_t>(f.ld) * f.m});
-  int* fidx = dupload(frontIdx, c->stream);
-  c->dyn_allocs.push_back(fidx);
-  int* lperm = dalloc<int>(f.m);
-  int* lpos = dalloc<int>(f.m);
-  c->dyn_allocs.push_back(lperm);
-  c->dyn_allocs.push_back(lpos);
-  double* Dd = dalloc<double>(f.nelig);
-  double* Do = dalloc<double>(f.nelig);
-  int8_t* pk = dalloc<int8_t>(f.nelig);
-  c->dyn_allocs.push_back(Dd);
-  c->dyn_allocs.push_back(Do);
-  c->dyn_allocs.push_back(pk);
+  int* fidx = dyn_upload(c, frontIdx);
+  int* lperm = dyn_alloc<int>(c, f.m);
+  int* lpos = dyn_alloc<int>(c, f.m);
+  double* Dd = dyn_alloc<double>(c, f.nelig);
+  double* Do = dyn_alloc<double>(c, f.nelig);
+  int8_t* pk = dyn_alloc<int8_t>(c, f.nelig);
   d.F = F;
   d.fidx = fidx;
   d.lperm = lperm;
@@ -1217,8 +1249,7 @@ void replan_front(symla_gpu_ctx* c, int s) {
     block_children(
         f.m, static_cast<int>(f.children.size()), [&](int t) { return pool.data() + offs[t].second; },
         [&](int t) { return static_cast<int>(cbRowsOf[t].size()); }, f.dyn_blk_ptr, f.dyn_blk_child);
-  int* dmaps = dupload(pool, c->stream);
-  c->dyn_allocs.push_back(dmaps);
+  int* dmaps = dyn_upload(c, pool);
   const int begin = static_cast<int>(c->hlinks.size());
   for (size_t t = 0; t < f.children.size(); ++t) {
     ChildLink L;
@@ -1808,6 +1839,7 @@ extern "C" void symla_gpu_destroy(symla_gpu_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   free_dynamic(c);
+  free_dyn_pool(c);
   for (auto& L : c->levels) free_level_device(L);
   void* ptrs[] = {c->d_arena, c->d_fidx, c->d_lperm, c->d_lpos, c->d_Dd, c->d_Do, c->d_pk, c->d_maps, c->d_desc, c->d_links, c->d_state,
                   c->d_glob, c->d_a_colptr, c->d_a_j, c->d_a_pos, c->d_a_idx, c->d_values, c->d_sign_final,
