@@ -959,8 +959,9 @@ bool use_static_panel(const symla_gpu_ctx* c, const LevelLists& L, const KernelO
   return ko.mode == SYMLA_MODE_STATIC && c->use_cluster_panel && L.cluster_ctas != 1;
 }
 
+// Panel iteration `it` of a level (from 0, consecutive), with its updates.
 void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, const KernelOpts& ko, int dynamic,
-                            const int* d_large) {
+                            const int* d_large, int it) {
   cudaStream_t st = c->stream;
   c->cur_level = level;
   const int nl = static_cast<int>(L.large.size());
@@ -977,7 +978,7 @@ void launch_panel_iteration(symla_gpu_ctx* c, const LevelLists& L, int level, co
     const bool single = L.cluster_ctas == 1 || (L.cluster_ctas == 0 && ko.mode == SYMLA_MODE_THRESHOLD &&
                                                 nl < kSinglePanelMaxFronts && L.large_max_m <= kSinglePanelMaxM);
     if (use_static_panel(c, L, ko)) {
-      launch_static_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, ko, c->d_glob, level, dynamic, st);
+      launch_static_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, ko, c->d_glob, level, dynamic, it, st);
       CK(cudaGetLastError());
     } else if (c->use_cluster_panel && !single && cluster_size_for(L.large_max_m, nl, L.panel_width) > 0) {
       CK(launch_cluster_panel(c->d_desc, c->d_state, d_large, nl, L.large_max_m, L.panel_width, ko, c->d_glob, level,
@@ -1050,7 +1051,7 @@ void launch_level_planned(symla_gpu_ctx* c, const LevelLists& L, int level, cons
       launch_assemble(c->d_desc, c->d_links, c->d_state, L.d_tasks, static_cast<int>(L.tasks.size()), L.d_touch, ko,
                       c->d_glob, level, dynamic, st);
     });
-    for (int it = 0; it < iters; ++it) launch_panel_iteration(c, L, level, ko, dynamic, d_large);
+    for (int it = 0; it < iters; ++it) launch_panel_iteration(c, L, level, ko, dynamic, d_large, it);
   }
 }
 
@@ -1110,8 +1111,7 @@ void complete_level(symla_gpu_ctx* c, const LevelLists& L, int level, const Kern
       CK(cudaMemcpy(&gl, c->d_glob, sizeof gl, cudaMemcpyDeviceToHost));
       if (!dynamic && gl.delay_level < level) break;  // aborted level, re-run by the delay path
       if (++guard > 4 * L.panels + 64) throw SymlaError(SYMLA_ERR_INTERNAL, "large front did not finish");
-      for (int it = 0; it < 4; ++it) launch_panel_iteration(c, L, level, ko, dynamic, d_large);
-      launched += 4;
+      for (int it = 0; it < 4; ++it) launch_panel_iteration(c, L, level, ko, dynamic, d_large, launched++);
     }
   }
   auto& iters = c->level_iters[ko.mode == SYMLA_MODE_STATIC];

@@ -54,9 +54,9 @@ cudaError_t configure_shared_panel();
 cudaError_t launch_shared_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m, int nb,
                                 const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream);
 // Static pivoting (panel_static.cu): panels of kPanelWidth pivots whatever the
-// front's size.
+// front's size; it = the panel's number, from 0 in consecutive launches.
 void launch_static_panel(const FrontDesc* fronts, FrontState* st, const int* list, int count, int max_m,
-                         const KernelOpts& o, FactorGlobals* g, int level, int dynamic, cudaStream_t stream);
+                         const KernelOpts& o, FactorGlobals* g, int level, int dynamic, int it, cudaStream_t stream);
 // Cluster panel (panel_cluster.cu), threshold pivoting: returns 0 from cluster_size_for when a
 // front is too large for it with nb-pivot panels (the single-CTA panel
 // kernel then runs).

@@ -56,6 +56,39 @@ def test_static_dense_front(n, weak):
 
 
 @pytest.mark.gpu
+def test_static_fronts_of_different_heights():
+    """Short and tall dense fronts in one level: the launches cover the tallest,
+    so most CTAs of a short front's column have no rows, and the short ones are
+    finished panels earlier. Every front as the oracle has it, and the same bits
+    at every repetition."""
+    sizes = [129, 801, 140, 545, 289, 1025, 130]
+    blocks = [quasi_definite(n, n // 3, 2) for n in sizes]
+    K, sign = sp.block_diag([b for b, _ in blocks], format="csc"), np.concatenate([g for _, g in blocks])
+    A = lower(K)
+    s = SymLDLT()
+    s.setMode(Mode.StaticRegularized)
+    s.setOrdering(OrderingType.Natural)
+    s.setExpectedSignPattern(sign)
+    s.setInitialRegularizationDelta(10.0)
+    s.analyzePattern(A)
+    s.factorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.setExpectedSignPattern(sign)
+    o.set(mode=1, initial_delta=10.0)
+    o.factorize(A)
+    assert s.inertia().as_tuple() == o.inertia()
+    assert s.numPerturbedPivots() == o.info()["num_perturbed"] >= 2 * len(sizes)
+    d0 = [f.Ddiag.copy() for f in s.numericFactor().fronts]
+    for fs, fo in zip(s.numericFactor().fronts, o.fronts()):
+        assert fs.nPivots == fo["nPivots"] and list(fs.rowIndices) == list(fo["rowIndices"])
+        np.testing.assert_allclose(fs.Ddiag, fo["Ddiag"], rtol=1e-9, atol=1e-9)
+    for _ in range(3):
+        s.refactorize(A)
+        for f, d in zip(s.numericFactor().fronts, d0):
+            np.testing.assert_array_equal(f.Ddiag, d)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [129, 255, 256, 257, 512, 513, 784, 785, 1025, 1057, 1288])
 def test_threshold_dense_front(n):
     """Fronts whose pivots need interchanges and 2x2 blocks, at the edges of
