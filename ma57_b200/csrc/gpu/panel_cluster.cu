@@ -289,6 +289,9 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     };
     if (q == oa) stage_row(b, sh.rowB, sh.vB);
     if (q == ob) stage_row(a, sh.rowA, sh.vA);
+    // a restart of the speculation copies the front's columns by bulk copies
+    // (the async proxy), which a plain fence does not order after these stores
+    asm volatile("fence.proxy.async.global;" ::: "memory");
     __threadfence();
     cluster.sync();
     auto write_row = [&](int row, const double* src, const double* vsrc) {
@@ -425,7 +428,9 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
         __syncwarp();
       } else if (threadIdx.x == 32 && have_rows) {
         const uint32_t bytes = static_cast<uint32_t>(e0 - s0) * sizeof(double);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier runs' accesses to these columns
+        // earlier runs' accesses to Lr, and interchanges of the front by any CTA
+        // of the cluster in this launch (ordered up to here by cluster barriers)
+        asm volatile("fence.proxy.async;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&rows_bar)),
                      "r"(bytes * static_cast<uint32_t>(np))
                      : "memory");

@@ -2,11 +2,14 @@
 the edges of the 32-pivot panels, the 96-row CTAs and the 256-pivot outer
 blocks, against the CPU oracle: inertia, perturbed pivots and residual.
 Threshold pivoting on both sides of the single-CTA panel's range."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
 
 from ma57_b200 import Mode, OrderingType, SymLDLT
+from ma57_b200 import _lib as L
 from ma57_b200.matrices import Stream, lower
 from oracle.pyoracle import OracleSymLDLT
 
@@ -112,3 +115,46 @@ def test_threshold_dense_front(n):
     r = K @ s.solve(b) - b
     # Bunch-Kaufman growth on a random matrix is far below the 1e3 allowed here
     assert np.abs(r).max() < 1e3 * n * 2.0 ** -53 * np.abs(K).sum(axis=1).max() * np.abs(x).max()
+
+
+def set_cluster(s, ctas):
+    """The panel's cluster size on every level (1: the single-CTA kernels)."""
+    lib = L.load()
+    for lv in range(int(s.plan_stats()["levels"])):
+        assert lib.symla_gpu_set_level_schedule(s._ctx.h, lv, 0, ctas) == L.SYMLA_OK
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ctas", [2, 4, 8, 16])
+def test_restart_after_interchange(ctas):
+    """Panels of one cluster that interchange rows of the front and then
+    speculate again on the rows just moved (read back from the front by bulk
+    copies): the pivots, kinds and factor of the CPU oracle, and the same bits
+    at every repetition."""
+    n = 600
+    st = Stream(n)
+    G = st.normal(n * n).reshape(n, n)
+    K = (G + G.T) / 2
+    # plain pivots with a zero diagonal now and then: a 2x2 or an interchange
+    # with a far row, then plain pivots again in the same panel
+    K[np.arange(n), np.arange(n)] += np.where(np.arange(n) % 2 == 0, 3.0, -3.0) * n
+    K[5::23, 5::23] = 0.0
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A)
+    s.factorize(A)
+    set_cluster(s, ctas)
+    s.refactorize(A)
+    stats = s.plan_stats()
+    assert stats["seq_interchange"] + stats["seq_2x2"] >= 10
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.factorize(A)
+    assert s.inertia().as_tuple() == o.inertia()
+    fs, fo = s.numericFactor().fronts[0], o.fronts()[0]
+    assert list(fs.rowIndices) == list(fo["rowIndices"])
+    assert [(b.start, b.kind) for b in fs.pivotBlocks] == fo["pivotBlocks"]
+    np.testing.assert_allclose(np.tril(fs.L, -1), np.tril(fo["L"], -1), rtol=0, atol=1e-10 * np.abs(fo["L"]).max())
+    for _ in range(3):
+        s.refactorize(A)
+        np.testing.assert_array_equal(s.numericFactor().fronts[0].L, fs.L)
