@@ -56,7 +56,7 @@ __device__ __forceinline__ double pivot_quotient(double a, double d, double inv)
 // the earlier steps (left-looking, the row's values in registers, eight
 // independent sums), then every lane factors the 8 x 8 diagonal block
 // redundantly in registers while it eliminates its own row. No shuffle, and
-// three warp barriers per step instead of two per column. Products are summed
+// one warp barrier per column instead of two. Products are summed
 // apart and subtracted from an entry once per step: subtracting them one by
 // one would round each time at the size of the entry, which on a diagonally
 // heavy matrix is far above that of the sum. Entries past np are garbage of
@@ -115,6 +115,7 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
       double next[8];  // the next column's values at the step's start
 #pragma unroll
       for (int r = c + 1; r < 8; ++r) next[r] = B.db[j0 + r][col + 1];
+      if (c < 7) __syncwarp();  // every lane has read column col + 1 before any stores its L there
       const double akk = T[c];
       double d = akk;
       if (Static) d = static_pivot(akk, sign[c], floorv, delta);

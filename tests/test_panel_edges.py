@@ -158,3 +158,30 @@ def test_restart_after_interchange(ctas):
     for _ in range(3):
         s.refactorize(A)
         np.testing.assert_array_equal(s.numericFactor().fronts[0].L, fs.L)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("last", [1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 31, 32])
+def test_diagonal_block_sizes(last):
+    """A diagonal block of every kind of size (one warp, steps of eight
+    columns): D against the oracle, and the same bits at every repetition."""
+    n = 128 + last
+    K, sign = quasi_definite(n, n // 3, 2)
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setMode(Mode.StaticRegularized)
+    s.setOrdering(OrderingType.Natural)
+    s.setExpectedSignPattern(sign)
+    s.setInitialRegularizationDelta(10.0)
+    s.analyzePattern(A)
+    s.factorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.setExpectedSignPattern(sign)
+    o.set(mode=1, initial_delta=10.0)
+    o.factorize(A)
+    f = s.numericFactor().fronts[0]
+    # quasi-definite, no growth: n eps times the condition of the leading blocks
+    np.testing.assert_allclose(f.Ddiag, o.fronts()[0]["Ddiag"], rtol=1e-10, atol=1e-10)
+    for _ in range(10):
+        s.refactorize(A)
+        np.testing.assert_array_equal(s.numericFactor().fronts[0].L, f.L)
