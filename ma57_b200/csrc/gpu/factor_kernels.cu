@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "factor_kernels.h"
+#include "panel_block.cuh"
 #include "reduce.cuh"
 
 namespace symla_gpu {
@@ -359,22 +360,11 @@ __global__ void __launch_bounds__(32 * kWarpFronts)
       const double akk = F.at(k, k);
       const int sign = sign_next;
       if (o.sign_final && k + 1 < effEnd) sign_next = o.sign_final[fi[k + 1]];
-      bool need;
-      if (sign > 0)
-        need = akk < floorv;
-      else if (sign < 0)
-        need = akk > -floorv;
-      else
-        need = fabs(akk) < floorv;
-      double d = akk;
-      if (need) {
-        const double sg = (sign != 0) ? static_cast<double>(sign) : (akk >= 0.0 ? 1.0 : -1.0);
-        d = akk + sg * delta;
-        const double applied = d - akk;
-        if (applied != 0.0) {
-          pert += fabs(applied);
-          ++nPert;
-        }
+      double applied;
+      const double d = static_pivot(akk, sign, floorv, delta, applied);
+      if (applied != 0.0) {
+        pert += fabs(applied);
+        ++nPert;
       }
       if (d > 0)
         ++n_pos;
@@ -721,22 +711,11 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
       const double akk = colk[k];
       const int sign = o.sign_final ? o.sign_final[f.fidx[k]] : 0;
       const double floorv = fmax(o.static_abs_floor, o.static_rel_floor * orig_max);
-      bool need;
-      if (sign > 0)
-        need = akk < floorv;
-      else if (sign < 0)
-        need = akk > -floorv;
-      else
-        need = fabs(akk) < floorv;
-      double d = akk;
-      if (need) {
-        const double sg = (sign != 0) ? static_cast<double>(sign) : (akk >= 0.0 ? 1.0 : -1.0);
-        d = akk + sg * S.delta;
-        const double applied = d - akk;
-        if (applied != 0.0) {
-          pert += fabs(applied);
-          ++nPert;
-        }
+      double applied;
+      const double d = static_pivot(akk, sign, floorv, S.delta, applied);
+      if (applied != 0.0) {
+        pert += fabs(applied);
+        ++nPert;
       }
       if (d > 0)
         ++n_pos;

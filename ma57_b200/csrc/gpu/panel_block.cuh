@@ -21,11 +21,16 @@ struct alignas(16) DiagBlock {
 };
 
 // Static pivoting (dense_kernel.hpp:982-1034): the pivot that replaces akk,
-// without a branch (a NaN is left alone).
-__device__ __forceinline__ double static_pivot(double akk, int sign, double floorv, double delta) {
+// without a branch, and what that adds to it. Only a pivot that fails the floor
+// test is replaced; a NaN, or an infinite one of the right sign, is left alone
+// and has nothing added (the difference of the two would be a NaN).
+__device__ __forceinline__ double static_pivot(double akk, int sign, double floorv, double delta, double& applied) {
   const double t = sign == 0 ? fabs(akk) : (sign > 0 ? akk : -akk);
   const bool up = sign > 0 || (sign == 0 && akk >= 0.0);
-  return t < floorv ? akk + (up ? delta : -delta) : akk;
+  const bool need = t < floorv;
+  const double d = need ? akk + (up ? delta : -delta) : akk;
+  applied = need ? d - akk : 0.0;
+  return d;
 }
 
 // 1 / d: two Newton steps on the hardware's approximation (under one ulp off),
@@ -117,8 +122,8 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
       for (int r = c + 1; r < 8; ++r) next[r] = B.db[j0 + r][col + 1];
       if (c < 7) __syncwarp();  // every lane has read column col + 1 before any stores its L there
       const double akk = T[c];
-      double d = akk;
-      if (Static) d = static_pivot(akk, sign[c], floorv, delta);
+      double d = akk, applied = 0.0;
+      if (Static) d = static_pivot(akk, sign[c], floorv, delta, applied);
       const double inv = pivot_reciprocal(d);
       double l[8];
 #pragma unroll
@@ -139,7 +144,7 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
       B.wv[lane][col] = v;
       B.dv[col] = d;
       B.iv[col] = inv;
-      if (Static) B.pv[col] = d - akk;
+      if (Static) B.pv[col] = applied;
     }
     __syncwarp();
   }

@@ -221,10 +221,9 @@ __global__ void __launch_bounds__(NT) panel_shared_kernel(const FrontDesc* __res
     }
     if (o.mode == 1) {
       __syncthreads();
-      const double akk = colk[k];
-      const double d = static_pivot(akk, o.sign_final ? o.sign_final[f.fidx[k]] : 0,
-                                    fmax(o.static_abs_floor, o.static_rel_floor * orig_max), S.delta);
-      const double applied = d - akk;
+      double applied;
+      const double d = static_pivot(colk[k], o.sign_final ? o.sign_final[f.fidx[k]] : 0,
+                                    fmax(o.static_abs_floor, o.static_rel_floor * orig_max), S.delta, applied);
       if (applied != 0.0) {
         S.perturb += fabs(applied);
         ++S.num_perturbed;

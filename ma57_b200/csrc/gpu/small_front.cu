@@ -223,14 +223,11 @@ __global__ void __launch_bounds__(kNT) small_front_kernel(const FrontDesc* __res
       if (mine) colk[tid] = v;
       if (is_static) {
         __syncthreads();
-        const double akk = colk[k];
-        const double d = static_pivot(akk, sgn[k], floorv, delta);
-        if (d != akk) {
-          const double applied = d - akk;
-          if (applied != 0.0) {
-            pert += fabs(applied);
-            ++nPert;
-          }
+        double applied;
+        const double d = static_pivot(colk[k], sgn[k], floorv, delta, applied);
+        if (applied != 0.0) {
+          pert += fabs(applied);
+          ++nPert;
         }
         finish_1x1(d, v);
         continue;

@@ -162,6 +162,39 @@ def test_nonfinite_values_then_clean_refactorization(bad, precision):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("ctas", [0, 1])
+@pytest.mark.parametrize("n", [16, 32, 33, 128, 129, 300, 784, 800])
+def test_nonfinite_pivots_are_not_perturbed(n, ctas, bad):
+    """Static pivoting adds delta to a pivot that fails the floor test and
+    counts that one: a NaN never fails it, nor does an infinite pivot of the
+    expected sign. One front of each kernel's range (ctas = 1: the single-CTA
+    panels), the bad entry on the last diagonal, so that every other pivot is
+    finite and well above the floor."""
+    import scipy.sparse as sp
+    G = M.Stream(n).normal(n * n).reshape(n, n)
+    K = (G + G.T) / 2 + 4 * n * np.eye(n)
+    K[n - 1, n - 1] = bad
+    A = M.lower(sp.csc_matrix(K))
+    lib = L.load()
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A)
+    _, cp, ri, vals = as_csc(A)
+    h = s._context(cp, ri).h
+    for lv in range(int(s.plan_stats()["levels"])):
+        assert lib.symla_gpu_set_level_schedule(h, lv, 0, ctas) == L.SYMLA_OK
+    o, info, signs = L.FactorOpts(), L.FactorInfo(), np.ones(n, np.int32)
+    lib.symla_factor_opts_default(C.byref(o))
+    o.mode = L.MODE_STATIC
+    o.static_delta, o.static_rel_floor, o.static_abs_floor = 1.0, 0.0, 1e-300  # (a relative floor would be infinite)
+    o.expected_sign = L.ptr_i(signs)
+    assert lib.symla_gpu_factorize(h, L.ptr_d(vals), 0, C.byref(o), C.byref(info)) == L.SYMLA_OK
+    assert info.num_perturbed == 0 and info.total_perturbation == 0.0
+    assert info.n_pos == (n if bad == np.inf else n - 1)
+
+
+@pytest.mark.gpu
 def test_size_and_order_errors_match_the_reference():
     A, b = M.config1(6)
     n = A.shape[0]

@@ -66,7 +66,7 @@ def test_static_fronts_of_different_heights():
     at every repetition."""
     sizes = [129, 801, 140, 545, 289, 1025, 130]
     blocks = [quasi_definite(n, n // 3, 2) for n in sizes]
-    K, sign = sp.block_diag([b for b, _ in blocks], format="csc"), np.concatenate([g for _, g in blocks])
+    K, sign = sp.csc_matrix(sp.block_diag([sp.coo_array(b) for b, _ in blocks])), np.concatenate([g for _, g in blocks])
     A = lower(K)
     s = SymLDLT()
     s.setMode(Mode.StaticRegularized)
