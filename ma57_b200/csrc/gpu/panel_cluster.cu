@@ -511,8 +511,11 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
         if (b0 + 32 * warp >= rend) break;  // the whole warp is past the rows
         const bool row = i < rend;
         double a[kSpecMax];
+        // a restart: the earlier pivots' products are summed apart and taken
+        // from the row's entries once (up to 30 of them, one by one, would
+        // round each time at the size of the entry; see panel_block.cuh)
 #pragma unroll
-        for (int c = 0; c < kSpecMax; ++c) a[c] = (row && c < np) ? Lr[(p0 + c) * R + li] : 0.0;
+        for (int c = 0; c < kSpecMax; ++c) a[c] = 0.0;
         for (int tt = 0; tt < p0; ++tt) {
           const double l = row ? Lr[tt * R + li] : 0.0;
           const double* w = wblk + tt * np2;
@@ -520,10 +523,12 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
           for (int c = 0; c < kSpecMax; c += 2)
             if (c < np) {
               const double2 wc = *reinterpret_cast<const double2*>(w + c);
-              a[c] = fma(-l, wc.x, a[c]);  // (a restart's few earlier pivots)
-              a[c + 1] = fma(-l, wc.y, a[c + 1]);
+              a[c] = fma(l, wc.x, a[c]);
+              a[c + 1] = fma(l, wc.y, a[c + 1]);
             }
         }
+#pragma unroll
+        for (int c = 0; c < kSpecMax; ++c) a[c] = ((row && c < np) ? Lr[(p0 + c) * R + li] : 0.0) - a[c];
         panel_row(blk, np, a);
         if (row) {
           double* out = Lr + p0 * R + li;

@@ -185,3 +185,38 @@ def test_diagonal_block_sizes(last):
     for _ in range(10):
         s.refactorize(A)
         np.testing.assert_array_equal(s.numericFactor().fronts[0].L, f.L)
+
+
+@pytest.mark.gpu
+def test_restart_sums_earlier_pivots_apart():
+    """A speculation that restarts late in a panel takes the 26 earlier pivots'
+    products from entries a thousand times their size. Summed apart, an entry of
+    [1, 2) is rounded twice (the two subtractions) and its quotient once, 0.29
+    ulp each in the root mean square, about 0.6 with the quotient's slack;
+    subtracted one by one it would be rounded 26 times, 1.5 ulp. The values
+    before scaling against 80-bit arithmetic."""
+    n, p0, d0 = 400, 26, 1024.0
+    st = Stream(n)
+    U = st.uniform(n * n, 1.0, 2.0) * np.where(st.uniform(n * n) < 0.5, -1.0, 1.0)
+    K = np.tril(U.reshape(n, n), -1)
+    K = K + K.T
+    K[np.arange(n), np.arange(n)] = d0 * np.where(np.arange(n) % 3 == 0, -1.0, 1.0)
+    K[p0 - 2, p0 - 2] = 0.0  # an interchange, then one plain pivot decided alone, then the restart
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A)
+    s.factorize(A)
+    set_cluster(s, 2)
+    s.refactorize(A)
+    f = s.numericFactor().fronts[0]
+    rows = np.asarray(f.rowIndices)
+    assert rows[p0 - 2] != p0 - 2 and all(b.kind == 0 for b in f.pivotBlocks[:32])
+    P = K[np.ix_(rows, rows)].astype(np.longdouble)[:, :32]
+    for k in range(32):
+        for j in range(k):
+            P[k:, k] -= P[k:, j] * (P[k, j] / P[j, j])
+    V = f.L[32:, :32] * f.Ddiag[:32]
+    err = (V - P[32:]).astype(np.float64) / 2.0 ** -52
+    rms = np.sqrt((err ** 2).mean(axis=0))
+    assert rms[p0:].max() < 1.0, rms[p0:]
