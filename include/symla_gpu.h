@@ -280,7 +280,10 @@ int symla_gpu_set_profiling(symla_gpu_ctx* ctx, int enable);
  * symla_gpu_set_wait_limit_ns: every device-side wait on another CTA's
  * progress -- the pipelined solves' block flags and the tensor-core Schur
  * update's copy/MMA barriers -- gives up after `ns` nanoseconds of the GPU's
- * global timer (0 restores the default of 2 s). A wait that runs out makes
+ * global timer (0 restores the default of 2 s). Under a limit below the
+ * default the solves launch each tree level by itself (slower), so that the
+ * limit bounds the waits between the blocks of one front and not that for a
+ * whole subtree. A wait that runs out makes
  * the call return SYMLA_ERR_TIMEOUT; the context stays usable (a solve can be
  * repeated, a factorization must be repeated). If a tensor-core tile that
  * gave up cannot then confirm, within the default limit, that its copies and

@@ -1643,7 +1643,12 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
   for (int c0 = 0; c0 < nrhs; c0 += kSolveChunks * chunk) {
     const int nc = std::min(kSolveChunks * chunk, nrhs - c0), groups = (nc + chunk - 1) / chunk;
     CK(cudaMemsetAsync(c->d_counters, 0, 2 * static_cast<size_t>(groups) * c->numSN * sizeof(int), st));
-    // every level in one launch, or (profiling) a launch per level
+    // Every level in one launch, or a launch per level: when profiling, and
+    // under a lowered wait limit. In one launch a front's wait for its children
+    // (or ancestors) lasts as long as all that is below (above) it; launched by
+    // level they are complete beforehand, and the limit bounds the waits between
+    // the blocks of one front, as it is documented to.
+    const bool by_level = c->profiling || c->wait_ns < kDefaultWaitNs;
     SolvePlan p = c->splan;
     p.counters = c->d_counters;
     const int ef = ++c->solve_epoch;
@@ -1665,7 +1670,7 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
                                      eb, c->d_solve_err, c->wait_ns, nrhs, c0, c->d_Xf, n, st));
       });
     };
-    if (c->profiling)
+    if (by_level)
       for (int l = 0; l < c->numLevels; ++l) {
         const auto& L = c->levels[l];
         forward(l, L.fwd_task0, L.fwd_ntasks, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs);
@@ -1675,7 +1680,7 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
     if (c0 == 0) CK(cudaEventRecord(c->ev[3], st));
     p.counters = c->d_counters + static_cast<size_t>(groups) * c->numSN;
     const int eb = ++c->solve_epoch;
-    if (c->profiling)
+    if (by_level)
       for (int l = c->numLevels - 1; l >= 0; --l) {
         const auto& L = c->levels[l];
         backward(l, eb, L.bwd_task0, L.bwd_ntasks, L.solve_bytes_fixed + nc * L.solve_bytes_per_rhs);

@@ -74,6 +74,33 @@ def test_solve_wait_timeout_is_reported_and_context_survives():
 
 
 @pytest.mark.gpu
+def test_lowered_wait_limit_does_not_count_the_tree():
+    """A band matrix in its natural order: a chain of 1500 fronts of one row
+    block each, so that no block waits for another of its front. The solve takes
+    milliseconds, far longer than the limit, which bounds the waits inside a
+    front and not a front's wait for everything below it in the tree."""
+    import scipy.sparse as sp
+    from ma57_b200.solver import SymbolicFactorOptions
+    n, band = 1500, 40
+    st = M.Stream(3)
+    A = sp.diags([st.uniform(n - d, -1.0, 1.0) for d in range(1, band + 1)], [-d for d in range(1, band + 1)])
+    A = M.lower(sp.csc_matrix(A + sp.diags(np.where(np.arange(n) % 2 == 0, 100.0, -100.0))))
+    B = np.asfortranarray(M.Stream(4).normal(2 * n).reshape(n, 2))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A, SymbolicFactorOptions(0, 0.0))
+    s.factorize(A)
+    assert s.plan_stats()["levels"] > 1000 and 32 < s.plan_stats()["max_m"] <= 64
+    X0 = s.solve(B)
+    lib = L.load()
+    assert lib.symla_gpu_set_wait_limit_ns(s._ctx.h, 20000) == L.SYMLA_OK
+    np.testing.assert_array_equal(s.solve(B), X0)
+    assert lib.symla_gpu_set_wait_limit_ns(s._ctx.h, 0) == L.SYMLA_OK
+    np.testing.assert_array_equal(s.solve(B), X0)
+    assert backward_error(A, X0, B) < 1e-12
+
+
+@pytest.mark.gpu
 def test_tensor_core_wait_timeout_is_reported_and_context_survives():
     """The mixed-precision far update waits on TMA copies and MMA groups; a
     1 ns limit makes those waits run out. The CTA abandons its tile, drains
