@@ -12,12 +12,13 @@ constexpr int kBlkStride = 34;   // even: pairs of a row are one 16-byte load
 
 // The diagonal block in shared memory. In: db's lower triangle, the block's
 // current values. Out: L below the diagonal of db (d on it); wv[i][c] = the
-// current value of row i in column c before scaling, d_c L(i, c); d, 1 / d and
-// the applied perturbation.
+// current value of row i in column c before scaling, d_c L(i, c); d, 1 / d
+// and the applied perturbation; extreme: some d is (pivot_extreme).
 struct alignas(16) DiagBlock {
   double db[kPanelMax][kBlkStride];
   double wv[kPanelMax][kBlkStride];
   double dv[kPanelMax], iv[kPanelMax], pv[kPanelMax];
+  int extreme;
 };
 
 // Static pivoting (dense_kernel.hpp:982-1034): the pivot that replaces akk,
@@ -33,27 +34,36 @@ __device__ __forceinline__ double static_pivot(double akk, int sign, double floo
   return d;
 }
 
-// 1 / d: two Newton steps on the hardware's approximation (under one ulp off),
-// or the correctly rounded reciprocal where a step could overflow or lose
-// bits to underflow.
-__device__ __forceinline__ double pivot_reciprocal(double d) {
-  const double m = fabs(d);
-  if (!(m > 1e-290 && m < 1e290)) return __drcp_rn(d);  // uniform: every lane has the same pivot
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  double e = fma(-d, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-d, r, 1.0);
-  return fma(r, e, r);
+// A pivot outside [2^-960, 2^960): there 1 / d, or a step towards it, would
+// overflow or lose bits to underflow (1 / d is infinite below 2^-1024), and what
+// follows takes the division instead. Uniform: every lane has the same pivot.
+__device__ __forceinline__ bool pivot_extreme(double d) {
+  const unsigned e = (static_cast<unsigned>(__double2hiint(d)) >> 20) & 0x7ff;
+  return e - (1023 - 960) >= 2 * 960;
 }
 
-// a / d from 1 / d with one residual step. a times the rounded 1 / d alone
-// would be off by the same relative error in the whole column, and the updates
-// (which take L D as the values before the division) would carry it into the
-// whole Schur complement.
+// 1 / d by Newton's iteration, r <- r + r (1 - d r), two steps from the
+// hardware's approximation: under one ulp off. Not for an extreme d.
+__device__ __forceinline__ double pivot_reciprocal(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  return fma(r, fma(-d, r, 1.0), r);
+}
+
+// a / d from inv = 1 / d: the product, corrected by one residual (Markstein's
+// quotient, IBM J. Res. Dev. 34(1), 1990). The product alone would be off by the
+// reciprocal's relative error in the whole column, and the updates (which take
+// L D as the values before the division) would carry it into the whole Schur
+// complement. Not for an extreme d. (An infinite quotient comes out as a NaN.)
 __device__ __forceinline__ double pivot_quotient(double a, double d, double inv) {
   const double q = a * inv;
   return fma(fma(-q, d, a), inv, q);
+}
+
+// a / d for any d, extreme = pivot_extreme(d).
+__device__ __forceinline__ double pivot_quotient(double a, double d, double inv, bool extreme) {
+  return extreme ? a / d : pivot_quotient(a, d, inv);
 }
 
 // LDL^T of the np x np block by one warp, lane = row, in steps of eight
@@ -71,9 +81,12 @@ __device__ __forceinline__ double pivot_quotient(double a, double d, double inv)
 // next pivot (one warp, 255 registers allowed). Column by column, with the
 // row in shared memory, a column took 890 cycles (14 us per block); now it
 // takes about 260 (keeping the sums apart costs the 64^3 stencil's panels 0.4
-// of 32.4 ms, the quotients' residual step 0.9).
+// of 31 ms, the quotients' residual step 0.9).
+//
+// Returns (in every lane) whether a pivot was extreme: the block is then to be
+// staged anew and given to factor_diag_block_divide.
 template <bool Static>
-__device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane, int lane_sign, double floorv,
+__device__ __forceinline__ bool factor_diag_block(DiagBlock& B, int np, int lane, int lane_sign, double floorv,
                                                   double delta) {
   double a[kPanelMax];  // the lane's row: values before scaling, by column
 #pragma unroll
@@ -148,6 +161,44 @@ __device__ __forceinline__ void factor_diag_block(DiagBlock& B, int np, int lane
     }
     __syncwarp();
   }
+  // (a NaN is none: what it comes from was found before it; nor, under threshold
+  // pivoting, a zero, which is never accepted)
+  const double own = B.dv[lane];
+  const bool extreme = lane < np && pivot_extreme(own) && own == own && (Static || own != 0.0);
+  const bool any = __any_sync(0xffffffffu, extreme);
+  if (lane == 0) B.extreme = any;
+  return any;
+}
+
+// The same with plain divisions, column by column, for a block staged anew of
+// which factor_diag_block found an extreme pivot. (Rare, so small: the fast one
+// is straight-line code that runs once per panel, and what is added to it is
+// paid in instruction fetches. The panels of the 64^3 stencil take 40 ms with an
+// extreme pivot handled where it is met, 33 with a branch per column for its
+// reciprocal alone, 31 with one check at the end.)
+template <bool Static>
+__device__ __noinline__ void factor_diag_block_divide(DiagBlock& B, int np, int lane, int lane_sign, double floorv,
+                                                      double delta) {
+  __syncwarp();
+#pragma unroll 1
+  for (int c = 0; c < np; ++c) {
+    double sum = 0.0;
+#pragma unroll 1
+    for (int t = 0; t < c; ++t) sum = fma(B.wv[lane][t], B.db[c][t], sum);
+    const double v = B.db[lane][c] - sum;  // (lanes above the diagonal: not read)
+    const double akk = __shfl_sync(0xffffffffu, v, c);
+    double d = akk, applied = 0.0;
+    if (Static) d = static_pivot(akk, __shfl_sync(0xffffffffu, lane_sign, c), floorv, delta, applied);
+    const double l = v / d;
+    __syncwarp();
+    B.db[lane][c] = lane == c ? d : l;
+    B.wv[lane][c] = v;
+    if (lane == c) {
+      B.dv[c] = d;
+      if (Static) B.pv[c] = applied;
+    }
+    __syncwarp();
+  }
 }
 
 // A row below the block: a[c] becomes the row's current value in column c,
@@ -199,7 +250,7 @@ __device__ __forceinline__ unsigned long long warp_column_max(const double (&a)[
 
 // A row's L = a / d and -(L D) = -a in the packed operands (p: pivot q0 of the
 // row), and put(c, l) for every column c < np: eight columns at a time, so
-// that the loads of d and 1 / d do not wait for the stores before them.
+// that the loads of the divisors do not wait for the stores before them.
 template <class Put>
 __device__ __forceinline__ void store_panel_row(const DiagBlock& B, int np, const double (&a)[kPanelMax], double* P,
                                                 int64_t pw, int prt, int q0, int i, Put&& put) {
@@ -227,6 +278,13 @@ __device__ __forceinline__ void store_panel_row(const DiagBlock& B, int np, cons
       if (((q0 + c0 + c + 1) & 15) == 0) p += next;
     }
   }
+  if (B.extreme)  // (the thread's own stores, read back)
+#pragma unroll 1
+    for (int c = 0; c < np; ++c) {
+      double* pk = P + packed_at(prt, q0 + c, i);
+      pk[0] = -pk[pw] / B.dv[c];
+      put(c, pk[0]);
+    }
 }
 
 }  // namespace symla_gpu

@@ -366,11 +366,12 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
       ++n_zero;
     thread_rmax = fmax(thread_rmax, fabs(d));
     const double inv = pivot_reciprocal(d);
+    const bool extreme = pivot_extreme(d);
     for (int i = max(base, k + 1) + threadIdx.x; i < rend; i += kCT) {
       const int li = i - base;
       const double a = col[li];
       thread_rmax = fmax(thread_rmax, fabs(a));
-      const double l = pivot_quotient(a, d, inv);
+      const double l = pivot_quotient(a, d, inv, extreme);
       Lr[p * R + li] = l;
       F[k * ld + i] = l;
       put_packed(k, i, l, a);
@@ -477,7 +478,17 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
         __syncthreads();
       }
       if (warp == 0) {
-        factor_diag_block<false>(blk, np, lane, 0, 0.0, 0.0);
+        if (factor_diag_block<false>(blk, np, lane, 0, 0.0, 0.0)) {
+#pragma unroll 1
+          for (int j = 0; j < np; ++j) {
+            double acc = 0.0;
+            if (lane >= j && lane < np)
+              for (int tt = 0; tt < p0; ++tt) acc += lblk[lane * p0 + tt] * wblk[tt * np2 + j];
+            blk.db[lane][j] =
+                (lane >= j && lane < np) ? F[static_cast<int64_t>(k0 + j) * ld + k0 + lane] - acc : 0.0;
+          }
+          factor_diag_block_divide<false>(blk, np, lane, 0, 0.0, 0.0);
+        }
       } else if (have_rows && !mbar_wait_bounded(&rows_bar, rows_phase)) {
         atomicCAS(&g->error, 0, kPanelErrTimeout);
         mbar_wait_bounded(&rows_bar, rows_phase);  // the copies must land before the CTA moves on

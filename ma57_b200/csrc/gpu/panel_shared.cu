@@ -190,12 +190,13 @@ __global__ void __launch_bounds__(NT) panel_shared_kernel(const FrontDesc* __res
     count(d);
     rmax = fmax(rmax, fabs(d));
     const double inv = pivot_reciprocal(d);
+    const bool extreme = pivot_extreme(d);
 #pragma unroll
     for (int n = 0; n < R; ++n) {
       const int i = tid + n * NT;
       if (i > k && i < m) {
         rmax = fmax(rmax, fabs(v[n]));
-        put(k, i, pivot_quotient(v[n], d, inv), v[n]);
+        put(k, i, pivot_quotient(v[n], d, inv, extreme), v[n]);
       }
     }
     if (tid == 0) set_d(k, d, 0.0, 0);

@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(kStaticThreads, 2) static_panel_kernel(const F
   double a[kPanelMax];
   if (warp == 0) {
     const int sign = (o.sign_final && lane < np) ? o.sign_final[f.fidx[ps + lane]] : 0;
+    const double floorv = fmax(o.static_abs_floor, o.static_rel_floor * om);
     // the loads of all columns first: they must not wait for one another's stores
     double v[kPanelMax];
 #pragma unroll
@@ -82,7 +83,12 @@ __global__ void __launch_bounds__(kStaticThreads, 2) static_panel_kernel(const F
 #pragma unroll
     for (int j = 0; j < kPanelMax; ++j) B.db[lane][j] = v[j];
     __syncwarp();
-    factor_diag_block<true>(B, np, lane, sign, fmax(o.static_abs_floor, o.static_rel_floor * om), delta);
+    if (factor_diag_block<true>(B, np, lane, sign, floorv, delta)) {
+#pragma unroll 1
+      for (int j = 0; j < np; ++j)
+        B.db[lane][j] = (lane >= j && lane < np) ? F[static_cast<int64_t>(ps + j) * ld + ps + lane] : 0.0;
+      factor_diag_block_divide<true>(B, np, lane, sign, floorv, delta);
+    }
   } else {
 #pragma unroll
     for (int c = 0; c < kPanelMax; ++c) a[c] = (row && c < np) ? F[static_cast<int64_t>(ps + c) * ld + i] : 0.0;

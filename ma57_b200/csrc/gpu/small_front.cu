@@ -204,9 +204,10 @@ __global__ void __launch_bounds__(kNT) small_front_kernel(const FrontDesc* __res
         ++n_zero;
       rmax = fmax(rmax, fabs(d));
       const double inv = pivot_reciprocal(d);
+      const bool extreme = pivot_extreme(d);
       if (tid > k && tid < m) {
         rmax = fmax(rmax, fabs(v));
-        S[k * lds + tid] = pivot_quotient(v, d, inv);
+        S[k * lds + tid] = pivot_quotient(v, d, inv, extreme);
         W[(k - ks) * kWS + tid] = v;
       } else if (tid == k) {
         S[k * lds + k] = d;
