@@ -294,7 +294,11 @@ int symla_gpu_set_profiling(symla_gpu_ctx* ctx, int enable);
  * memory that each later symla_gpu_create may allocate for a context's plan
  * (front arena, maps, solve workspaces); 0 removes it. A plan that does not
  * fit fails with SYMLA_ERR_OOM before touching the GPU further, like a
- * failing cudaMalloc does without a cap. */
+ * failing cudaMalloc does without a cap. The plan holds one buffer for the
+ * packed operands of its largest level's updates (up to 4.6 KB per row of that
+ * level's fronts of more than 128 rows). Outside the cap: fronts that delayed
+ * pivots enlarge; a context keeps their memory for its next factorization and
+ * gives it back at the one after the last that delayed any. */
 int symla_gpu_set_wait_limit_ns(symla_gpu_ctx* ctx, unsigned long long ns);
 int symla_gpu_set_memory_limit(long long bytes);
 

@@ -790,21 +790,39 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
 
 // Device memory of the re-planned fronts of the current factorization, from
 // the context's pool (a cudaMalloc for each of a front's eight arrays was most
-// of a re-planned factorization's time).
+// of a re-planned factorization's time). The pool follows what the last
+// factorization used: free_dynamic gives it back when that delayed nothing, and
+// makes one chunk of what was used out of several, or of far more.
+constexpr size_t kDynChunkMin = static_cast<size_t>(1) << 20;
+
 template <typename T>
 T* dyn_alloc(symla_gpu_ctx* c, size_t count) {
   const size_t bytes = (std::max<size_t>(1, count) * sizeof(T) + 255) & ~static_cast<size_t>(255);
   while (c->dyn_chunk < c->dyn_pool.size() && c->dyn_off + bytes > c->dyn_pool[c->dyn_chunk].second) {
-    ++c->dyn_chunk;
-    c->dyn_off = 0;
+    if (c->dyn_off == 0) {  // too small for this one, and nothing in it
+      dfree(c->dyn_pool[c->dyn_chunk].first);
+      c->dyn_pool.erase(c->dyn_pool.begin() + static_cast<std::ptrdiff_t>(c->dyn_chunk));
+    } else {
+      ++c->dyn_chunk;
+      c->dyn_off = 0;
+    }
   }
   if (c->dyn_chunk == c->dyn_pool.size()) {
-    const size_t size = std::max({bytes, c->dyn_total, static_cast<size_t>(1) << 20});
-    c->dyn_pool.push_back({dalloc<char>(size), size});
+    // the first chunk holds what the last factorization used; a further one
+    // what is missing, and an eighth of what is in use ahead
+    size_t size = std::max({bytes, c->dyn_pool.empty() ? c->dyn_last : c->dyn_used / 8, kDynChunkMin});
+    void* p = nullptr;
+    if (size > bytes && cudaMalloc(&p, size) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+      size = bytes;  // no room to spare: what is needed and no more
+    }
+    c->dyn_pool.push_back({p ? static_cast<char*>(p) : dalloc<char>(size), size});
     c->dyn_off = 0;
   }
   char* p = c->dyn_pool[c->dyn_chunk].first + c->dyn_off;
   c->dyn_off += bytes;
+  c->dyn_used += bytes;
   return reinterpret_cast<T*>(p);
 }
 
@@ -823,13 +841,11 @@ void free_dyn_pool(symla_gpu_ctx* c) {
 void free_dynamic(symla_gpu_ctx* c) {
   for (void* p : c->dyn_allocs) dfree(p);
   c->dyn_allocs.clear();
-  if (c->dyn_pool.size() > 1) {
-    // one chunk of the total from the next factorization that needs it
-    c->dyn_total = 0;
-    for (auto& b : c->dyn_pool) c->dyn_total += b.second;
-    free_dyn_pool(c);
-  }
-  c->dyn_chunk = c->dyn_off = 0;
+  size_t total = 0;
+  for (auto& b : c->dyn_pool) total += b.second;
+  if (c->dyn_used == 0 || c->dyn_pool.size() > 1 || total > 2 * std::max(c->dyn_used, kDynChunkMin)) free_dyn_pool(c);
+  c->dyn_last = c->dyn_used;
+  c->dyn_chunk = c->dyn_off = c->dyn_used = 0;
   c->dyn_front_blocks.clear();
 }
 

@@ -178,12 +178,13 @@ struct symla_gpu_ctx {
   size_t tc_guard_cap = 0;
 
   // dynamic (delayed-pivot) allocations for the current factorization: what
-  // re-planned fronts take comes from a pool that the context keeps (chunks
-  // with a bump pointer, merged into one of their total when more were
-  // needed), the rest is allocated and freed
+  // re-planned fronts take comes from a pool that the context keeps from one
+  // factorization to the next (chunks with a bump pointer, dyn_alloc), the rest
+  // is allocated and freed
   std::vector<void*> dyn_allocs;
   std::vector<std::pair<char*, size_t>> dyn_pool;
-  size_t dyn_chunk = 0, dyn_off = 0, dyn_total = 0;
+  size_t dyn_chunk = 0, dyn_off = 0;
+  size_t dyn_used = 0, dyn_last = 0;  // bytes taken by the current factorization, and by the last
   // front storage allocated by re-planning (pointer, doubles), for the
   // checked build's storage check
   std::vector<std::pair<double*, size_t>> dyn_front_blocks;

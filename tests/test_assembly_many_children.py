@@ -51,3 +51,37 @@ def test_many_children(m, leaves, zero_leaves):
     # backward stable: a modest multiple of n eps, pivot growth included
     bw = np.abs(R).max() / (abs(F).sum(axis=1).max() * np.abs(X).max() + np.abs(B).max())
     assert bw < 100 * A.shape[0] * 2.0 ** -53
+
+
+@pytest.mark.gpu
+def test_memory_of_replanned_fronts_follows_their_use():
+    """Factorizations that delay one pivot more each time: what the context
+    holds beyond its plan stays near what the largest of them needs (a dense
+    front of about 1540 rows), and goes back when nothing is delayed any more."""
+    import torch
+    m, leaves = 1500, 40
+    base = leaves_on_a_dense_root(m, leaves, 0)
+    lead = [base.indptr[i] for i in range(leaves)]  # the leaves' diagonal entries
+    assert all(base.indices[p] == i and base.data[p] == 3.0 for i, p in enumerate(lead))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(base, SymbolicFactorOptions(0, 0.0))
+
+    def held(zeros):
+        A = base.copy()
+        for i, p in enumerate(lead):
+            A.data[p] = 0.0 if i < zeros else 3.0
+        s.factorize(A)
+        assert s.last_info.num_delayed == zeros
+        torch.cuda.synchronize()
+        return -torch.cuda.mem_get_info()[0]
+
+    plan = held(0)
+    front = 8 * (m + leaves) ** 2
+    used = [held(z) - plan for z in range(2, leaves, 3)]
+    # an eighth ahead, the packed operands of the enlarged front (17 chunks of 16
+    # pivots), the driver's 2 MB pages of the few arrays beside them
+    packed = 2 * 17 * ((m + leaves) // 64 + 1) * 16 * 68 * 8
+    assert max(used) < 1.25 * front + packed + 6 * 2 ** 20, (used, front, packed)
+    held(0)
+    assert held(0) - plan < 0.25 * front
