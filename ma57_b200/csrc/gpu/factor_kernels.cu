@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(32 * kWarpFronts)
       if (lambda <= o.zero_tol) {
         const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
         dec = (fabs(akk) <= isolatedFloor) ? 3 : 0;
-      } else if (fabs(akk) >= kAlpha * lambda) {
+      } else if (r < 0 || fabs(akk) >= kAlpha * lambda) {  // (r < 0: no candidate, under a negative zero_tol)
         dec = 0;
       } else {
         double sm = 0.0;
@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(const FrontDesc* _
     if (lambda <= o.zero_tol) {
       const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
       dec = (fabs(akk) <= isolatedFloor) ? 3 : 0;
-    } else if (fabs(akk) >= kAlpha * lambda) {
+    } else if (r < 0 || fabs(akk) >= kAlpha * lambda) {  // (r < 0: no candidate, under a negative zero_tol)
       dec = 0;
     } else if (r >= S.ob_end && ps > S.ob) {
       dec = 4;  // partner beyond the outer block: apply the deferred update first

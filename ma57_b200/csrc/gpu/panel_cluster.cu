@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kCT) cluster_panel_kernel(const FrontDesc* __r
     if (lambda <= o.zero_tol) {
       const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
       dec = (fabs(akk) <= isolatedFloor) ? 3 : 0;
-    } else if (fabs(akk) >= kAlphaBK * lambda) {
+    } else if (r < 0 || fabs(akk) >= kAlphaBK * lambda) {  // (r < 0: no candidate, under a negative zero_tol)
       dec = 0;
     } else if (r >= S.ob_end && ps > S.ob) {
       // the partner lies beyond the outer block while earlier panels of the

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(NT) panel_shared_kernel(const FrontDesc* __res
     if (lambda <= o.zero_tol) {
       const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
       dec = (fabs(akk) <= isolatedFloor) ? 3 : 0;
-    } else if (fabs(akk) >= kAlphaBK * lambda) {
+    } else if (r < 0 || fabs(akk) >= kAlphaBK * lambda) {  // (r < 0: no candidate, under a negative zero_tol)
       dec = 0;
     } else if (r >= S.ob_end && ps > S.ob) {
       dec = 4;  // partner beyond the outer block: apply the deferred update first

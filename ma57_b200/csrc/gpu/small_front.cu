@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kNT) small_front_kernel(const FrontDesc* __res
       if (lambda <= o.zero_tol) {
         const double isolatedFloor = fmax(o.zero_tol, o.rel_floor * orig_max);
         dec = (fabs(akk) <= isolatedFloor) ? 3 : 0;
-      } else if (fabs(akk) >= kAlphaBK * lambda) {
+      } else if (r < 0 || fabs(akk) >= kAlphaBK * lambda) {  // (r < 0: no candidate, under a negative zero_tol)
         dec = 0;
       } else {
         u = mine ? column(r, tid >= r ? S[r * lds + tid] : S[tid * lds + r]) : 0.0;

@@ -222,6 +222,32 @@ def test_nonfinite_pivots_are_not_perturbed(n, ctas, bad):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,ctas", [(16, 0), (100, 0), (300, 1), (300, 2), (800, 1), (800, 16)])
+def test_no_candidate_under_a_negative_zero_tolerance(n, ctas):
+    """The last pivot has no other candidate; a negative zero tolerance does not
+    take it for isolated, and a NaN fails every test against it: it is a 1x1
+    pivot (in every kernel's range), not a search at row -1."""
+    import scipy.sparse as sp
+    G = M.Stream(n).normal(n * n).reshape(n, n)
+    K = (G + G.T) / 2 + 4 * n * np.eye(n)
+    K[n - 1, n - 1] = np.nan
+    A = M.lower(sp.csc_matrix(K))
+    lib = L.load()
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A)
+    _, cp, ri, vals = as_csc(A)
+    h = s._context(cp, ri).h
+    for lv in range(int(s.plan_stats()["levels"])):
+        assert lib.symla_gpu_set_level_schedule(h, lv, 0, ctas) == L.SYMLA_OK
+    o, info = L.FactorOpts(), L.FactorInfo()
+    lib.symla_factor_opts_default(C.byref(o))
+    o.zero_tolerance = -1.0
+    assert lib.symla_gpu_factorize(h, L.ptr_d(vals), 0, C.byref(o), C.byref(info)) == L.SYMLA_OK
+    assert (info.n_pos, info.n_neg, info.n_zero, info.singular) == (n - 1, 0, 1, 0)
+
+
+@pytest.mark.gpu
 def test_size_and_order_errors_match_the_reference():
     A, b = M.config1(6)
     n = A.shape[0]
