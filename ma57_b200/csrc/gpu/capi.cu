@@ -515,7 +515,9 @@ size_t packed_level_doubles(const symla_gpu_ctx* c, const LevelLists& L) {
   for (int s : L.large) t += packed_doubles(c->hdesc[s]);
   return t;
 }
-void assign_packed_level(symla_gpu_ctx* c, const LevelLists& L, double* base) {
+void assign_packed_level(symla_gpu_ctx* c, LevelLists& L, double* base) {
+  L.packed = base;
+  L.packed_doubles = packed_level_doubles(c, L);
   for (int s : L.large) {
     FrontDesc& d = c->hdesc[s];
     const size_t len = packed_doubles(d);
@@ -742,7 +744,7 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
     c->packed_doubles = std::max(c->packed_doubles, packed_level_doubles(c, c->levels[l]));
   }
   c->d_packed = dalloc<double>(c->packed_doubles);
-  for (const auto& L : c->levels) assign_packed_level(c, L, c->d_packed);
+  for (auto& L : c->levels) assign_packed_level(c, L, c->d_packed);
   c->hdesc_static = c->hdesc;
   c->d_desc = dupload(c->hdesc, c->stream);
 
@@ -918,6 +920,10 @@ const char* check_code_name(int code) {
     case kChkPermute: return "solve permutation entry";
     case kChkSolveRow: return "level-solve row index";
     case kChkWorkspace: return "solve workspace slice";
+    case kChkTask: return "assembly task or level list";
+    case kChkPacked: return "packed update operands";
+    case kChkSolveTask: return "solve task";
+    case kChkSolveTable: return "per-front table of the solves";
     default: return "unknown check";
   }
 }
@@ -936,9 +942,12 @@ void check_status_word(symla_gpu_ctx* c, const char* when) {
   }
 }
 
-// Validate every front's tables (phase as launch_validate_fronts), then, with
-// sync, read the status word: a failure marks the context unusable.
-void validate_tables(symla_gpu_ctx* c, int phase, const KernelOpts& ko, const char* when) {
+// Validate every front's tables (phase as launch_validate_fronts), before the
+// launches of the factorization also those of its levels (or of the re-planned
+// one), then, with sync, read the status word: a failure marks the context
+// unusable.
+void validate_tables(symla_gpu_ctx* c, int phase, const KernelOpts& ko, const char* when,
+                     const LevelLists* replanned = nullptr) {
   if constexpr (!kCheckedBuild) return;
   cudaStream_t st = c->stream;
   c->h_ranges.clear();
@@ -960,6 +969,15 @@ void validate_tables(symla_gpu_ctx* c, int phase, const KernelOpts& ko, const ch
   launch_validate_fronts(c->d_desc, c->d_links, c->d_state, nullptr, c->numSN, c->numSN, c->n, c->d_a_colptr, ko,
                          c->d_ranges, static_cast<int>(c->h_ranges.size() / 2), c->d_W, c->d_W + wtotal, c->w_nrhs,
                          phase, st);
+  auto level = [&](const LevelLists& L) {
+    launch_validate_level(c->d_desc, L.d_small, static_cast<int>(L.small.size()), L.d_large,
+                          static_cast<int>(L.large.size()), L.d_tasks, static_cast<int>(L.tasks.size()), L.d_touch,
+                          static_cast<int>(L.touch.size()), c->d_a_colptr, c->numSN, L.packed,
+                          L.packed + L.packed_doubles, ko, st);
+  };
+  if (phase == 0 && replanned) level(*replanned);
+  if (phase == 0 && !replanned)
+    for (const auto& L : c->levels) level(L);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(st));
   check_status_word(c, when);
@@ -1377,7 +1395,7 @@ void run_factorization(symla_gpu_ctx* c, const symla_factor_opts* o, symla_facto
           c->tc_guard_cap = L.large.size();
         }
       }
-      validate_tables(c, 0, ko, "after re-planning delayed pivots");
+      validate_tables(c, 0, ko, "after re-planning delayed pivots", &L);
       launch_level(c, L, l, ko, 1, L.d_small, L.d_large);
       read_states(c);
       free_level_device(L);
@@ -1608,6 +1626,7 @@ void ensure_solve_tasks(symla_gpu_ctx* c, int nchunks) {
     p.nflags = total;
     p.nfronts = c->numSN;
     p.nslots = slots;
+    p.ntiny = static_cast<int>(tiny.size());
     c->solve_np = np;
     c->solve_chunks = 0;  // the per-group state is sized anew
   }
@@ -1651,6 +1670,7 @@ void device_solve(symla_gpu_ctx* c, const double* dB, int ldb, int nrhs, double*
     ko.a_idx = c->d_a_idx;
     ko.nnz = c->nnz;
     ko.chk = c->d_check;
+    launch_validate_solve(c->d_desc, c->d_state, c->splan, c->fwd_ntasks, c->bwd_ntasks, c->d_check, st);
     validate_tables(c, 2, ko, "before the solve");
   }
   const int n = c->n;

@@ -6,7 +6,10 @@
 // bound is checked before it is made: the front descriptors and their storage,
 // the extend-add maps, the scatter map of A's values, the row indices the
 // solves gather and scatter through, and the contribution-block positions the
-// assembly reads. A failed check skips the access and records the first
+// assembly reads. The tables that the host makes and nothing on the device
+// changes (assembly tasks with their lists of children, packed operands, the
+// solves' task lists and per-front tables, the extend-add maps) are checked as
+// a whole before the launches that go through them. A failed check skips the access and records the first
 // failure (a code and where it happened) in a status word in device memory;
 // nothing traps or asserts. The host reads the word after every factorization
 // and solve and turns a failure into SYMLA_ERR_INTERNAL; the context is then
@@ -35,6 +38,10 @@ enum CheckCode : int {
   kChkPermute = 10,      // solve permutation entry outside [0, n)
   kChkSolveRow = 11,     // level-solve row index or child workspace row out of range
   kChkWorkspace = 12,    // a front's solve workspace outside the workspace allocation
+  kChkTask = 13,         // an assembly task, its list of children or its A entries out of range
+  kChkPacked = 14,       // a front's packed update operands outside their buffer, or too small
+  kChkSolveTask = 15,    // a solve task, its fronts, flags or helper slots out of range
+  kChkSolveTable = 16,   // a per-front table of the solves: flags, or the front waited for
 };
 
 // First failure wins; count keeps counting.
@@ -84,6 +91,43 @@ __host__ __device__ inline bool a_entry_ok(int j, int pos, long long idx, int nc
   if (!in_range(j, 0, ncols) || pos < 0) return false;
   const int i = pos < ncols ? pos : pos + nextra;
   return i >= j && i < m && in_range(idx, 0, nnz);
+}
+
+// An assembly task: rows [i0, i1) of the 32 columns from j0 of a front of m rows,
+// at most max_rows of them; entries [ch0, ch0 + nch) of the ntouch children's
+// offsets, A's entries [a0, a1) among the front's own [e0, e1).
+__host__ __device__ inline bool asm_task_ok(int j0, int i0, int i1, int m, int max_rows, int ch0, int nch, int ntouch,
+                                            int a0, int a1, int e0, int e1) {
+  if (j0 < 0 || j0 % 32 != 0 || j0 >= m || i0 < j0 || i1 <= i0 || i1 > m || i1 - i0 > max_rows) return false;
+  if (ch0 < 0 || nch < 0 || nch > ntouch - ch0) return false;
+  return a0 == a1 || (a0 >= e0 && a0 < a1 && a1 <= e1);
+}
+
+// The packed operands of a front of m rows: prt row tiles, two blocks of pw
+// doubles (chunks pivot chunks of tile doubles a row tile) in [lo, hi).
+__host__ __device__ inline bool packed_ok(const double* P, long long pw, int prt, int m, int chunks, int tile,
+                                          const double* lo, const double* hi) {
+  if (prt != (m + 63) / 64 || pw < static_cast<long long>(chunks) * prt * tile) return false;
+  return P != nullptr && P >= lo && P <= hi && 2 * pw <= static_cast<long long>(hi - P);
+}
+
+// A list of count tiny fronts from first of ntiny, at most eight.
+__host__ __device__ inline bool tiny_task_ok(int first, int count, int ntiny) {
+  return first >= 0 && count >= 1 && count <= 8 && count <= ntiny - first;
+}
+
+// Block b of a front of rows rows (forward) or pivots (backward) in blocks of rb,
+// its flag among nflags.
+__host__ __device__ inline bool block_task_ok(int b, int rows, int rb, int flag_base, int nflags) {
+  return b >= 0 && static_cast<long long>(b) * rb < rows && flag_base >= 0 && b < nflags - flag_base;
+}
+
+// Part p of P of a backward block, its helpers' slots from h0 among nslots (the
+// main part, 0: all P - 1 of them; a helper: its own).
+__host__ __device__ inline bool part_task_ok(int p, int P, int h0, int nslots) {
+  if (P < 1 || P > 8 || p < 0 || p >= P) return false;
+  const int slots = p > 0 ? 1 : P - 1;
+  return h0 >= 0 && slots <= nslots - h0;
 }
 
 }  // namespace symla_gpu

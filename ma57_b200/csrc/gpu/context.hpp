@@ -45,6 +45,8 @@ struct LevelLists {
   int panel_width = 32;        // pivots per panel (narrower for fronts too tall for a full-width cluster panel)
   double* d_panel_cols = nullptr;  // single-CTA panel kernel, fronts too tall for shared memory: 2 m per front
   int trailing_grid = 0;
+  double* packed = nullptr;    // the large fronts' packed update operands, not owned
+  size_t packed_doubles = 0;
   std::vector<AsmTask> tasks;  // assembly tasks of the large fronts
   std::vector<int> touch;      // and their children (AsmTask::ch0)
   std::vector<int> all;        // every front of the level (solve)

@@ -1428,6 +1428,46 @@ void launch_validate_fronts(const FrontDesc* fronts, const ChildLink* links, con
                                                      nranges, wlo, whi, wcols, phase);
 }
 
+// Tables of one level that the host makes with the plan (or a re-planned level).
+__global__ void validate_level_kernel(const FrontDesc* __restrict__ fronts, const int* __restrict__ small, int nsmall,
+                                      const int* __restrict__ large, int nlarge, const AsmTask* __restrict__ tasks,
+                                      int ntasks, const int* __restrict__ touch, int ntouch,
+                                      const int* __restrict__ a_colptr, int num_fronts, const double* plo,
+                                      const double* phi, KernelOpts o) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int t = t0; t < nsmall; t += step) {
+    const int s = small[t];
+    if (check(in_range(s, 0, num_fronts), o.chk, kChkTask, s))
+      check(fronts[s].m <= kSmallFrontMax, o.chk, kChkFrontShape, s);
+  }
+  for (int t = t0; t < nlarge; t += step) {
+    const int s = large[t];
+    if (!check(in_range(s, 0, num_fronts), o.chk, kChkTask, s)) continue;
+    const FrontDesc& f = fronts[s];
+    check(packed_ok(f.P, f.pw, f.prt, f.m, packed_chunks(f.nelig), kPkTile, plo, phi), o.chk, kChkPacked, s);
+  }
+  for (int t = t0; t < ntasks; t += step) {
+    const AsmTask k = tasks[t];
+    if (!check(in_range(k.front, 0, num_fronts), o.chk, kChkTask, t)) continue;
+    const FrontDesc& f = fronts[k.front];
+    if (!check(asm_task_ok(k.j0, k.i0, k.i1, f.m, kAsmRows, k.ch0, k.nch, ntouch, k.a0, k.a1, a_colptr[f.a_begin],
+                           a_colptr[f.a_begin + f.ncols]),
+               o.chk, kChkTask, t))
+      continue;
+    for (int c = 0; c < k.nch; ++c) check(in_range(touch[k.ch0 + c], 0, f.ch_end - f.ch_begin), o.chk, kChkTask, t);
+  }
+}
+
+void launch_validate_level(const FrontDesc* fronts, const int* small, int nsmall, const int* large, int nlarge,
+                           const AsmTask* tasks, int ntasks, const int* touch, int ntouch, const int* a_colptr,
+                           int num_fronts, const double* plo, const double* phi, const KernelOpts& o,
+                           cudaStream_t stream) {
+  const int work = std::max({nsmall, nlarge, ntasks});
+  if (work <= 0) return;
+  validate_level_kernel<<<std::min((work + 255) / 256, 1184), 256, 0, stream>>>(
+      fronts, small, nsmall, large, nlarge, tasks, ntasks, touch, ntouch, a_colptr, num_fronts, plo, phi, o);
+}
+
 cudaError_t configure_factor_kernels() {
   cudaError_t e;
   e = cudaFuncSetAttribute(factor_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -93,6 +93,12 @@ void launch_validate_fronts(const FrontDesc* fronts, const ChildLink* links, con
                             int count, int num_fronts, int n, const int* a_colptr, const KernelOpts& o,
                             const double* const* ranges, int nranges, const double* wlo, const double* whi,
                             int wcols, int phase, cudaStream_t stream);
+// Of one level: the lists of small and large fronts, the assembly tasks with the
+// children's offsets, the large fronts' packed operands inside [plo, phi).
+void launch_validate_level(const FrontDesc* fronts, const int* small, int nsmall, const int* large, int nlarge,
+                           const AsmTask* tasks, int ntasks, const int* touch, int ntouch, const int* a_colptr,
+                           int num_fronts, const double* plo, const double* phi, const KernelOpts& o,
+                           cudaStream_t stream);
 
 // graph launches: atomicMin(g->unfinished_level, level) if a front of the
 // list is not finished
@@ -135,8 +141,11 @@ struct SolvePlan {
   int* counters;
   int* hflags;
   double* hscratch;
-  int nflags, nfronts, nslots;
+  int nflags, nfronts, nslots, ntiny;
 };
+// Checked build: the task lists and the per-front tables of the solves.
+void launch_validate_solve(const FrontDesc* fronts, const FrontState* st, const SolvePlan& p, int nfwd, int nbwd,
+                           CheckWord* chk, cudaStream_t stream);
 int solve_block_rows();
 int solve_rhs_chunk();
 int solve_tiny_rows();

@@ -957,6 +957,47 @@ cudaError_t launch_backward_pipelined(const FrontDesc* fronts, const FrontState*
                                      args, kSolveSmem, stream);
 }
 
+__global__ void validate_solve_kernel(const FrontDesc* __restrict__ fronts, const FrontState* __restrict__ st,
+                                      SolvePlan pl, int nfwd, int nbwd, CheckWord* chk) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  const auto tiny_ok = [&](int4 tk, int t) {
+    if (!check(tiny_task_ok(tk.x, tk.z, pl.ntiny), chk, kChkSolveTask, t)) return;
+    for (int k = 0; k < tk.z; ++k) {
+      const int s = pl.tiny[tk.x + k];
+      if (check(in_range(s, 0, pl.nfronts), chk, kChkSolveTask, t)) check(fronts[s].m <= kTinyRows, chk, kChkSolveTask, t);
+    }
+  };
+  for (int s = t0; s < pl.nfronts; s += step) {
+    check(in_range(pl.bwd_wait[s], -1, pl.nfronts) && pl.fwd_need[s] >= 0 && pl.bwd_need[s] >= 0 &&
+              in_range(fronts[s].parent, -1, pl.nfronts) && pl.flag_base[s] >= 0 &&
+              (fronts[s].m + kRB - 1) / kRB <= pl.nflags - pl.flag_base[s],
+          chk, kChkSolveTable, s);
+  }
+  for (int t = t0; t < nfwd; t += step) {
+    const int4 tk = pl.fwd_tasks[t];
+    if (tk.y == -2)
+      tiny_ok(tk, t);
+    else if (check(in_range(tk.x, 0, pl.nfronts), chk, kChkSolveTask, t))
+      check(block_task_ok(tk.y, fronts[tk.x].m, kRB, pl.flag_base[tk.x], pl.nflags), chk, kChkSolveTask, t);
+  }
+  for (int t = t0; t < nbwd; t += step) {
+    const int4 tk = pl.bwd_tasks[t];
+    if (tk.y == -2)
+      tiny_ok(tk, t);
+    else if (check(in_range(tk.x, 0, pl.nfronts), chk, kChkSolveTask, t) && tk.y != -1)
+      check(block_task_ok(tk.y, st[tk.x].npiv, kRB, pl.flag_base[tk.x], pl.nflags) &&
+                part_task_ok(tk.z, tk.w >> 20, tk.w & ((1 << 20) - 1), pl.nslots),
+            chk, kChkSolveTask, t);
+  }
+}
+
+void launch_validate_solve(const FrontDesc* fronts, const FrontState* st, const SolvePlan& p, int nfwd, int nbwd,
+                           CheckWord* chk, cudaStream_t stream) {
+  const int work = std::max({p.nfronts, nfwd, nbwd});
+  if (work <= 0) return;
+  validate_solve_kernel<<<std::min((work + 255) / 256, 1184), 256, 0, stream>>>(fronts, st, p, nfwd, nbwd, chk);
+}
+
 void launch_permute_in(int n, int nrhs, const int* perm, const double* B, int ldb, double* Bp, cudaStream_t stream,
                        CheckWord* chk) {
   permute_in_kernel<<<grid_for(static_cast<long long>(n) * nrhs, 256), 256, 0, stream>>>(n, nrhs, perm, B, ldb, Bp,

@@ -61,6 +61,49 @@ int main() {
   for (int v : bad_inv) EXPECT(!in_range(v, -1, 4));
   for (int v : bad_rel) EXPECT(!in_range(v, 0, 6));
 
+  // assembly tasks of a 100-row front, at most 64 rows each: j0, i0, i1, m, rows,
+  // then its children (of 10 offsets), then its A entries (of [20, 30))
+  EXPECT(asm_task_ok(32, 32, 96, 100, 64, 0, 10, 10, 20, 30, 20, 30));
+  EXPECT(asm_task_ok(96, 96, 100, 100, 64, 10, 0, 10, 0, 0, 20, 30));     // no children, no entries
+  EXPECT(!asm_task_ok(33, 40, 96, 100, 64, 0, 10, 10, 20, 30, 20, 30));   // not a 32-column block
+  EXPECT(!asm_task_ok(128, 128, 130, 100, 64, 0, 0, 10, 0, 0, 20, 30));   // past the front
+  EXPECT(!asm_task_ok(32, 0, 64, 100, 64, 0, 10, 10, 20, 30, 20, 30));    // rows above the diagonal block
+  EXPECT(!asm_task_ok(32, 64, 101, 100, 64, 0, 10, 10, 20, 30, 20, 30));  // a row past the front
+  EXPECT(!asm_task_ok(0, 0, 65, 100, 64, 0, 10, 10, 20, 30, 20, 30));     // too many rows
+  EXPECT(!asm_task_ok(0, 0, 64, 100, 64, 5, 6, 10, 20, 30, 20, 30));      // a child past the list
+  EXPECT(!asm_task_ok(0, 0, 64, 100, 64, -1, 2, 10, 20, 30, 20, 30));
+  EXPECT(!asm_task_ok(0, 0, 64, 100, 64, 0, 10, 10, 19, 30, 20, 30));     // another front's entry
+  EXPECT(!asm_task_ok(0, 0, 64, 100, 64, 0, 10, 10, 20, 31, 20, 30));
+  EXPECT(!asm_task_ok(0, 0, 64, 100, 64, 0, 10, 10, 25, 24, 20, 30));
+
+  // packed operands of a 100-row front: 2 row tiles, 3 chunks of 8 doubles a tile
+  EXPECT(packed_ok(arena.data(), 48, 2, 100, 3, 8, lo, hi));
+  EXPECT(packed_ok(arena.data() + 4, 48, 2, 100, 3, 8, lo, hi));          // ends exactly at the end
+  EXPECT(!packed_ok(arena.data() + 5, 48, 2, 100, 3, 8, lo, hi));
+  EXPECT(!packed_ok(arena.data(), 47, 2, 100, 3, 8, lo, hi));             // too small
+  EXPECT(!packed_ok(arena.data(), 48, 1, 100, 3, 8, lo, hi));             // a row tile missing
+  EXPECT(!packed_ok(nullptr, 48, 2, 100, 3, 8, lo, hi));
+
+  // solve tasks: tiny fronts, blocks with their flags, parts with their slots
+  EXPECT(tiny_task_ok(0, 8, 8));
+  EXPECT(tiny_task_ok(7, 1, 8));
+  EXPECT(!tiny_task_ok(7, 2, 8));
+  EXPECT(!tiny_task_ok(0, 9, 20));  // more than warps
+  EXPECT(!tiny_task_ok(-1, 1, 8));
+  EXPECT(!tiny_task_ok(0, 0, 8));
+  EXPECT(block_task_ok(1, 65, 64, 5, 7));
+  EXPECT(!block_task_ok(1, 64, 64, 5, 7));  // no such block
+  EXPECT(!block_task_ok(1, 65, 64, 6, 7));  // its flag past the flags
+  EXPECT(!block_task_ok(-1, 65, 64, 5, 7));
+  EXPECT(!block_task_ok(0, 65, 64, -1, 7));
+  EXPECT(part_task_ok(0, 1, 4, 4));   // no helpers
+  EXPECT(part_task_ok(0, 4, 1, 4));
+  EXPECT(part_task_ok(3, 4, 3, 4));
+  EXPECT(!part_task_ok(0, 4, 2, 4));  // a helper's slot past the slots
+  EXPECT(!part_task_ok(3, 4, 4, 4));
+  EXPECT(!part_task_ok(4, 4, 0, 4));
+  EXPECT(!part_task_ok(0, 0, 0, 4));
+
   if (failures) return 1;
   std::printf("check_predicates OK\n");
   return 0;
