@@ -8,6 +8,7 @@ import sys
 import numpy as np
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 
 from ma57_b200 import Mode, OrderingType, Precision, RefinementOptions, SymbolicFactorOptions, SymLDLT  # noqa: E402
 from ma57_b200 import _lib as L  # noqa: E402
@@ -45,6 +46,18 @@ def main(out):
     res["arrow_x"] = s.solve(B)
     res["arrow_dynamic"] = np.array(s.last_info.used_dynamic_path)
     res["arrow_status"] = np.array(status(s))
+    # a re-planned front of more than 128 rows (its own assembly tasks and packed
+    # operands), warp-sized leaves, and three groups of right-hand sides
+    from test_assembly_many_children import leaves_on_a_dense_root
+    A = leaves_on_a_dense_root(300, 80, 5)
+    B = np.asfortranarray(M.Stream(1).normal(40 * A.shape[0]).reshape(A.shape[0], 40))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A, SymbolicFactorOptions(max_relax_size=1, max_relax_fill_fraction=0.0))
+    s.factorize(A)
+    res["tree_x"] = s.solve(B)
+    res["tree_dynamic"] = np.array(s.last_info.used_dynamic_path)
+    res["tree_status"] = np.array(status(s))
     cases = [("c1", *M.config1(12), Precision.FP64, Mode.ThresholdPivot),
              ("c3", *M.config3(24, nrhs=4), Precision.FP64, Mode.ThresholdPivot),
              ("c3m", *M.config3(24, nrhs=4), Precision.Mixed, Mode.ThresholdPivot)]

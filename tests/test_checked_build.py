@@ -7,7 +7,7 @@ CPU: the library is built, exports every declared entry point and reports
 itself as checked; the predicates the checks use (ma57_b200/csrc/gpu/
 checked.cuh) are compiled for the host and run against planted bad tables.
 GPU: the same factorizations and solves (the delayed-pivot arrow, which
-re-plans a front; config 1; the 27-point stencil in FP64 and mixed precision;
+re-plans a front; leaves that delay pivots to a large one; config 1; the 27-point stencil in FP64 and mixed precision;
 a KKT system in threshold and StaticRegularized mode) run through both
 builds: no check fails, and the results are bit-identical."""
 import ctypes as C
@@ -76,6 +76,7 @@ def test_checked_build_passes_and_matches_the_ordinary_build(tmp_path):
     chk = _run_worker("checked", tmp_path)
     prod = _run_worker("", tmp_path)
     assert int(chk["checked_build"]) == 1 and int(prod["checked_build"]) == 0
+    assert int(chk["tree_dynamic"]) == 1
     assert int(chk["arrow_dynamic"]) == 1  # the re-planned (delayed-pivot) path ran under the checks
     assert chk["arrow_npiv"].tolist() == [0, 0, 5]
     for key in chk:

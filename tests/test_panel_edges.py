@@ -220,3 +220,59 @@ def test_restart_sums_earlier_pivots_apart():
     err = (V - P[32:]).astype(np.float64) / 2.0 ** -52
     rms = np.sqrt((err ** 2).mean(axis=0))
     assert rms[p0:].max() < 1.0, rms[p0:]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [160, 285, 600, 784, 785, 1100])
+@pytest.mark.parametrize("ctas", [1, 2, 4])
+def test_panel_kernels_take_the_oracles_pivots(n, ctas):
+    """The single-CTA panels (with L in shared memory up to 784 rows, reading it
+    back above) and clusters on the same fronts, several outer blocks of 256
+    pivots with interchanges and 2x2 pivots throughout: the oracle's pivot
+    order, kinds and factor."""
+    G = Stream(n).normal(n * n).reshape(n, n)
+    K = (G + G.T) / 2
+    K[np.arange(0, n, 3), np.arange(0, n, 3)] += 3 * np.sqrt(n)
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setOrdering(OrderingType.Natural)
+    s.analyzePattern(A)
+    s.factorize(A)
+    set_cluster(s, ctas)
+    s.refactorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.factorize(A)
+    fs, fo = s.numericFactor().fronts[0], o.fronts()[0]
+    assert s.inertia().as_tuple() == o.inertia()
+    assert list(fs.rowIndices) == list(fo["rowIndices"])
+    assert [(b.start, b.kind) for b in fs.pivotBlocks] == fo["pivotBlocks"]
+    assert sum(b.kind for b in fs.pivotBlocks) > n // 20 and list(fs.rowIndices) != sorted(fs.rowIndices)
+    # growth times the rounding of n sums
+    scale = np.abs(fo["L"]).max() * n * 2.0 ** -53 * 1e4
+    np.testing.assert_allclose(np.tril(fs.L, -2), np.tril(fo["L"], -2), rtol=0, atol=scale)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [129, 256, 300, 784, 785, 900])
+def test_static_single_cta(n):
+    """The static branches of the single-CTA panels, against the oracle."""
+    K, sign = quasi_definite(n, n // 3, 3)
+    A = lower(sp.csc_matrix(K))
+    s = SymLDLT()
+    s.setMode(Mode.StaticRegularized)
+    s.setOrdering(OrderingType.Natural)
+    s.setExpectedSignPattern(sign)
+    s.setInitialRegularizationDelta(10.0)
+    s.analyzePattern(A)
+    s.factorize(A)
+    set_cluster(s, 1)
+    s.refactorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.setExpectedSignPattern(sign)
+    o.set(mode=1, initial_delta=10.0)
+    o.factorize(A)
+    assert s.inertia().as_tuple() == o.inertia()
+    assert s.numPerturbedPivots() == o.info()["num_perturbed"] >= 3
+    fs, fo = s.numericFactor().fronts[0], o.fronts()[0]
+    np.testing.assert_allclose(fs.Ddiag, fo["Ddiag"], rtol=1e-10, atol=1e-10)
+    np.testing.assert_allclose(np.tril(fs.L, -1), np.tril(fo["L"], -1), rtol=0, atol=1e-10)

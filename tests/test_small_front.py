@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
-from ma57_b200 import Mode, OrderingType, SymLDLT
+from ma57_b200 import Mode, OrderingType, SymLDLT, autotune
 from ma57_b200 import matrices as M
 from ma57_b200.solver import SymbolicFactorOptions
 from oracle.pyoracle import OracleSymLDLT
@@ -85,4 +85,53 @@ def test_children(m, leaves, zero_leaves):
     o = OracleSymLDLT(s.symbolicFactor())
     o.factorize(A)
     assert s.last_info.num_delayed == zero_leaves
+    compare(s, o, 1e-9)
+
+
+def factor_both(A, ordering, options=None):
+    s = SymLDLT()
+    s.setOrdering(ordering)
+    s.analyzePattern(A, options or SymbolicFactorOptions())
+    s.factorize(A)
+    o = OracleSymLDLT(s.symbolicFactor())
+    o.factorize(A)
+    return s, o
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("every", [0, 15])
+def test_warp_per_front(every):
+    """Levels whose small fronts all have at most 32 rows: a warp each, with
+    children, 2x2 pivots and interchanges; a zero on every 15th diagonal delays
+    pivots too. (Random values: no ties for rounding to decide.)"""
+    blocks = []
+    for i in (0, 2, 3, 6):  # (regular with the zeros too)
+        n = 120 + 10 * i
+        S = M.random_sparse_spd(n, 4, 50 + i) - sp.identity(n) * 2.0
+        S = sp.coo_matrix(sp.tril(S))
+        if every:
+            S.data[(S.row == S.col) & (S.row % every == 0)] = 0.0
+        blocks.append(sp.coo_array(S))
+    A = sp.csc_matrix(sp.block_diag(blocks))
+    s, o = factor_both(A, OrderingType.AMD)
+    assert any(i["small"] and i["small_max_m"] <= 32 for i in autotune.level_info(s))
+    assert (s.last_info.num_delayed > 0) == (every > 0)
+    assert any(b.kind for f in s.numericFactor().fronts for b in f.pivotBlocks)
+    compare(s, o, 1e-9 * max(np.abs(f["L"]).max() for f in o.fronts() if f["L"].size))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("leaves", [1000, 1023, 1024, 1100])
+def test_level_of_warp_and_cta_fronts(leaves):
+    """On either side of the number of warp-sized fronts (1024) from which those
+    of a level take a launch of their own beside the larger ones; four of them
+    delay their pivot to a front that is assembled from all of them."""
+    from test_assembly_many_children import leaves_on_a_dense_root
+    tree = leaves_on_a_dense_root(100, leaves, 4)
+    blocks = [tree] + [M.lower(sp.csc_matrix(dense(n, "random"))) for n in (33, 40, 64, 127, 128)]
+    A = sp.csc_matrix(sp.block_diag([sp.coo_array(b) for b in blocks]))
+    s, o = factor_both(A, OrderingType.Natural, SymbolicFactorOptions(0, 0.0))
+    info = autotune.level_info(s)[0]
+    assert info["small"] == leaves + 5 and info["small_max_m"] == 128
+    assert s.last_info.num_delayed == 4
     compare(s, o, 1e-9)
