@@ -254,9 +254,13 @@ void build_maps(const std::vector<int>& cbRows, const std::unordered_map<int, in
 
 // Fewest warp-sized fronts that get a launch of their own in a level with
 // larger small fronts: below that a CTA each is at most a few waves and done
-// sooner (a level of 141 fronts of up to 57 rows takes 0.16 ms with the two
-// launches, about 0.1 with one; of 8866 of up to 86 rows 0.38, and 0.5 as CTAs).
-constexpr int kWarpFrontsMin = 1024;
+// sooner, and the two launches follow one another. Measured with N warp-sized
+// fronts of r rows and five of 60, microseconds with one launch / with two:
+//   r =  6:  N = 300  56 /  67,  1500  70 /  68,  3000   90 /  71,  9000  158 /  92
+//   r = 20:  N = 300  57 /  94,  1500  96 /  98,  3000  152 / 108,  9000  350 / 191
+//   r = 31:  N = 300  57 / 131,  1500 117 / 144,  3000  201 / 172,  9000  516 / 368
+// They cross at 1300, 1550 and 2000 fronts.
+constexpr int kWarpFrontsMin = 1536;
 
 // The children (offsets) of a front with a row in each 32-column block, from
 // their extend-add maps: rel(t) points at child t's map to the front's rows,

@@ -121,9 +121,9 @@ def test_warp_per_front(every):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("leaves", [1000, 1023, 1024, 1100])
+@pytest.mark.parametrize("leaves", [1000, 1535, 1536, 1700])
 def test_level_of_warp_and_cta_fronts(leaves):
-    """On either side of the number of warp-sized fronts (1024) from which those
+    """On either side of the number of warp-sized fronts (1536) from which those
     of a level take a launch of their own beside the larger ones; four of them
     delay their pivot to a front that is assembled from all of them."""
     from test_assembly_many_children import leaves_on_a_dense_root
