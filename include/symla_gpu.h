@@ -320,7 +320,9 @@ int symla_gpu_set_graph(symla_gpu_ctx* ctx, int enable);
  * a warp or a CTA by its size), and panel cluster size in {2, 4, 8, 16}, or 1
  * for the single-CTA panel kernel (no cluster barriers: faster for levels
  * whose panels decide many pivots one at a time), 0 = chosen by front size; a
- * cluster size too small for the level's fronts falls back to the default. */
+ * cluster size too small for the level's fronts falls back to the default.
+ * Static pivoting has one panel kernel without clusters: 0 and 2 to 16 all take
+ * it, 1 the single-CTA kernel. */
 int symla_gpu_level_info(symla_gpu_ctx* ctx, int level, int* out6);
 int symla_gpu_set_level_schedule(symla_gpu_ctx* ctx, int level, int small_threads, int cluster_ctas);
 /* Rows per tile of the level's Schur-complement update (the tile shape

@@ -4,15 +4,14 @@ Two launch shapes depend on front size and have no single best value: the
 number of CTAs in the panel cluster of the large fronts (2, 4, 8 or 16; more
 CTAs hold fewer rows each but occupy more SMs; or 1, the single-CTA panel
 kernel, whose pivot-by-pivot decisions need no cluster barriers) and the
-tile shape of their
-Schur-complement update (128 x 64 or 64 x 64: the smaller tile wastes less
-of small fronts' trailing blocks, the larger reuses operands more). The tree
-levels are bucketed by
-the largest front they hold, and a coordinate search times the actual
+tile shape of their Schur-complement update (128 x 64 or 64 x 64: the smaller
+tile wastes less of small fronts' trailing blocks, the larger reuses operands
+more). Under static pivoting, whose panels use no clusters, only 1 differs from
+the default. The tree levels are bucketed by the largest front they hold, and a coordinate search times the actual
 factorization (CUDA events around the numeric factorization) for each
 candidate shape of one bucket at a time, keeping the fastest. The result is
 installed per level through symla_gpu_set_level_schedule; it changes launch
-shapes only, never results.
+shapes only, and results by no more than rounding.
 """
 from __future__ import annotations
 
@@ -20,6 +19,7 @@ import ctypes as C
 import math
 
 from . import _lib as L
+from .solver import Mode
 
 LARGE_BUCKETS = (512, 2048, 8192, 1 << 30)  # panel cluster, by the level's largest large front
 
@@ -80,7 +80,8 @@ def tune(solver, A, reps: int = 2):
     apply(solver, schedule)
     base = _factor_ms(solver, A, reps)
     best = base
-    for kind, buckets, cands in (("large", large_b, (1, 2, 4, 8, 16)), ("update", large_b, (64, 128))):
+    panels = (1,) if solver.mode_ == Mode.StaticRegularized else (1, 2, 4, 8, 16)
+    for kind, buckets, cands in (("large", large_b, panels), ("update", large_b, (64, 128))):
         for b in buckets:
             for cand in cands:
                 trial = {k: dict(v) for k, v in schedule.items()}

@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(32 * kWarpFronts)
 // candidate columns up to date from the front (which holds the panel-start
 // state for every non-pivoted column) and the panel's L and D
 // (dense_kernel.hpp:516-559). The trailing update follows in
-// trailing_update_kernel.
+// update_mma_kernel.
 namespace {
 
 constexpr int kPanelThreads = 512;
@@ -966,7 +966,7 @@ __device__ __forceinline__ int update_tiles(int m, int c0, int c1, int tm) {
 // pivot column and a block barrier per chunk, kept the pipe half idle: the
 // updates of the 64^3 27-point stencil took 38.4 ms (11.7 TF/s, most launches
 // being near updates of at most 32 pivots) and take 29.7 ms (15.2 TF/s), those
-// of a KKT system with a 15568-row front 84.8 ms (15.5) and 68.0 ms (19.3).
+// of a KKT system with a 15568-row front 84.8 ms (15.5) and 59.8 ms (21.9).
 namespace {
 constexpr int kTJ = 64;   // column tile width
 constexpr int kKM = 16;   // K chunk

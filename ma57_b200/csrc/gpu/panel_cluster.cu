@@ -16,25 +16,27 @@
 // The front in global memory holds the panel-start ("raw") values of every
 // non-pivoted column; row/column interchanges are applied to it and to the
 // shared-memory copies. The near and far updates of the panel follow in
-// update_kernel / the tensor-core far update.
+// update_mma_kernel / the tensor-core far update.
 //
 // Speculative panel. Most pivots of most fronts are 1x1 pivots at k (the
 // Bunch-Kaufman test |a_kk| >= alpha * lambda passes), and the test can be
 // checked after the fact: factor the panel without pivoting, then compare
 // each pivot with lambda = max over the eligible rows of its column's
-// current values, which the unpivoted factorization produces exactly (the
-// same left-looking sums as the sequential path). Every CTA factors the
+// current values, which the unpivoted factorization produces (the same sums as
+// the sequential path's, grouped differently: equal up to rounding, which can
+// decide a tie otherwise). Every CTA factors the
 // panel's diagonal block redundantly in shared memory (no exchange needed
 // for D and the L rows of the block), then its own rows below the block in
 // one pass with no per-pivot synchronisation; the per-pivot partial lambdas
 // cross the cluster once. The pivots before the first one that fails are
-// accepted (identical values and decisions to the sequential path), and
-// the same launch finishes the panel on the sequential path from the first
+// accepted, and the same launch finishes the panel on the sequential path from the first
 // failing pivot (measured: cheaper than a new panel + update launch pair).
-// A 32-pivot panel of 4096 rows accepted whole takes 24 us (33 us when the
+// A 32-pivot panel of 4096 rows accepted whole took 24 us (33 us when the
 // block was factored column by column and the rows went through shared memory
-// once more for the maxima and for L), of which the block's chain is about 4, the
-// row pass 5.6, the exchange of the maxima 1.7, the stores of L 2.3 us.
+// once more for the maxima and for L), of which the block's chain was about 4,
+// the row pass 5.6, the exchange of the maxima 1.7, the stores of L 2.3 us. On
+// the 64^3 stencil, where one panel in ten stops and restarts, a launch takes
+// 68 us on average (31.1 ms for 460).
 #include <cooperative_groups.h>
 
 #include <cmath>
@@ -918,11 +920,14 @@ int panel_width_for(int max_m, int count) {
 }
 
 int cluster_size_for(int max_m, int count, int nb) {
-  // The panel is latency-bound: a CTA costs a fixed ~8 us (the diagonal
-  // block's pivot chain, the exchanges) plus ~10 ns per row it holds, and
-  // one CTA runs per SM (200 registers x 256 threads). More CTAs per front
-  // shorten each CTA; fewer let more fronts run in one wave. Pick the
-  // cluster size with the smallest modelled time (waves x CTA time).
+  // The panel is latency-bound, and one CTA runs per SM (its 240 to 254
+  // registers x 256 threads). More CTAs per front shorten each CTA; fewer let
+  // more fronts run in one wave. Pick the cluster size with the smallest
+  // modelled time (waves x CTA time). The model's 8 us and 10 ns a row were
+  // fitted to an earlier form of the kernel. Now a panel of one dense front
+  // takes 23 to 26 us at 1024 rows, 23 to 26 at 2048 and 26 to 28 at 4096, with
+  // no order among 2, 4, 8 and 16 CTAs, so that an additional wave costs about
+  // three times the model's 8 us.
   int best = 0;
   double best_t = 0.0;
   for (int cs : {2, 4, 8, 16}) {

@@ -15,8 +15,9 @@
 // threshold pivoting uses kept the rows in the shared memory of at most 16
 // CTAs, exchanged per-pivot maxima it did not need here, and had to narrow
 // its panels on fronts of more than 10,000 rows: 33 us for 16 pivots of a
-// 15568-row front, against 24 us for 32 here (all panels of that KKT step:
-// 33.0 and 12.2 ms; an interior-point step's: 2.4 and 1.4 ms).
+// 15568-row front, against 24 us for 32 here when this kernel was new (all
+// panels of that KKT step: 33.0 and 12.2 ms, 10.9 now; an interior-point
+// step's: 2.4 and 1.4 ms, 1.2 now).
 #include <algorithm>
 
 #include "common.cuh"
