@@ -61,9 +61,11 @@ __device__ __forceinline__ double pivot_quotient(double a, double d, double inv)
   return fma(fma(-q, d, a), inv, q);
 }
 
-// a / d for any d, extreme = pivot_extreme(d).
+// a / d for any d, extreme = pivot_extreme(d) (a call, so that the division
+// stays out of the loops over pivots).
+static __device__ __noinline__ double pivot_divide(double a, double d) { return a / d; }
 __device__ __forceinline__ double pivot_quotient(double a, double d, double inv, bool extreme) {
-  return extreme ? a / d : pivot_quotient(a, d, inv);
+  return extreme ? pivot_divide(a, d) : pivot_quotient(a, d, inv);
 }
 
 // LDL^T of the np x np block by one warp, lane = row, in steps of eight
